@@ -202,22 +202,7 @@ __device__ __forceinline__ Vq<Q> dzq(const float* s, int off, const float* c) {
 //    scaled-numerator route selected per lane instead of branched to;
 //  * otherwise (a huge value, or the correction unverified) each value
 //    takes its own route through div_c.
-// The group test, the same predicate as mk_ok on every lane, in three
-// instructions per value: the smallest of 2*bits - 2 (unsigned; a zero of
-// either sign maps to 0xfffffffe, a magnitude below 2^-100 below
-// 2*0x0d800000 - 2) and the largest |x| (NaN is ignored by fmaxf; it stays
-// NaN on every path).
-struct RangeAcc {
-  unsigned lo = 0xffffffffu;
-  float hi = 0.f;
-  __device__ __forceinline__ void add(float x) {
-    lo = min(lo, __float_as_uint(x) * 2u - 2u);
-    hi = fmaxf(hi, fabsf(x));
-  }
-  __device__ __forceinline__ bool ok() const { return lo >= 2u * 0x0D800000u - 2u && hi < 0x1p100f; }
-  __device__ __forceinline__ bool below_huge() const { return hi < 0x1p100f; }
-};
-
+// The group test is RangeAcc (sw_device.cuh).
 template <int K, int Q>
 __device__ __forceinline__ void div_group(Vq<Q> (&v)[K], const float (&d)[K], const float (&r)[K], int fast) {
   RangeAcc acc;

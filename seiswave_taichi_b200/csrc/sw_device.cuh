@@ -227,17 +227,24 @@ __device__ __forceinline__ float mk_div_tiny(float x, float d, float r) {
   return tiny_finish(xs, mk_core(xs, d, r), d);
 }
 
-// tiny_finish without branches (both outcomes computed, one selected), for
-// groups whose lanes take different routes
+// tiny_finish without branches, for groups whose lanes take different routes:
+// both outcomes computed, one selected.  Adding and taking away 2^23 with t's
+// sign rounds |t| <= 2^23 to the nearest integer (ties to even) on the FMA
+// pipe; floorf, truncf and rintf run at an eighth of its rate.  Where t is a
+// midpoint (diff = +-1/2) the residual's sign says on which side of it x/d
+// lies; a quotient on the other side than n moves n by one.
 __device__ __forceinline__ float tiny_finish_sel(float xs, float ys, float d) {
   const float t = __fmul_rn(ys, 0x1p85f);
-  const float fl = floorf(t);
-  const bool mid = fabsf(__fadd_rn(t, -truncf(t))) == 0.5f;
+  const unsigned sg = __float_as_uint(t) & 0x80000000u;
+  const float m = __uint_as_float(sg | 0x4b000000u);  // 2^23 with t's sign
+  const float n0 = __fadd_rn(__fadd_rn(t, m), -m);
+  const float diff = __fadd_rn(t, -n0);
   const float res = __fmaf_rn(-ys, d, xs);
-  float n = rintf(t);
-  n = mid && res > 0.f ? __fadd_rn(fl, 1.f) : n;
-  n = mid && res < 0.f ? fl : n;
-  return fabsf(ys) >= 0x1p-62f ? __fmul_rn(ys, 0x1p-64f) : __fmul_rn(n, 0x1p-149f);
+  const bool cross = fabsf(diff) == 0.5f && __fmul_rn(diff, res) > 0.f;
+  const float n = cross ? __fmaf_rn(2.f, diff, n0) : n0;
+  // n = +0 where a negative t rounds to zero: the quotient is -0 there
+  const float sub = __uint_as_float(__float_as_uint(__fmul_rn(n, 0x1p-149f)) | sg);
+  return fabsf(ys) >= 0x1p-62f ? __fmul_rn(ys, 0x1p-64f) : sub;
 }
 
 // div_c's result with a verified correction (fast != 0) for any |x| < 2^100
@@ -279,6 +286,59 @@ __device__ __forceinline__ float div_c(float x, float d, float r, int fast) {
   return div_rare(x, d);
 }
 __device__ __forceinline__ double div_c(double x, double d, double, int) { return div_v(x, d); }
+
+// x / d for a divisor that is not verified exhaustively, y = RN(1/d): Markstein's
+// correction twice.  The first makes the quotient faithful (its error before
+// rounding is below 2^-40 of the quotient), and from a faithful quotient q and
+// |y - 1/d| < 2^-p/d the correction q + y*RN(x - q*d) rounds x/d correctly
+// (P. Markstein, IBM J. Res. Dev. 34(1), 1990, theorem on division), where
+// nothing underflows: a float numerator in [2^-100, 2^100), a double one in
+// [2^-900, 2^900), and a divisor in [2^-20, 2^20].  A zero numerator gives
+// +0 (callers that can meet -0 restore its sign).
+__device__ __forceinline__ float mk2_core(float x, float d, float y) {
+  float q = __fmul_rn(x, y);
+  q = __fmaf_rn(__fmaf_rn(-q, d, x), y, q);
+  return __fmaf_rn(__fmaf_rn(-q, d, x), y, q);
+}
+__device__ __forceinline__ double mk2_core(double x, double d, double y) {
+  double q = __dmul_rn(x, y);
+  q = __fma_rn(__fma_rn(-q, d, x), y, q);
+  return __fma_rn(__fma_rn(-q, d, x), y, q);
+}
+template <typename T>
+__device__ __forceinline__ bool mk2_divisor(T d) { return d >= (T)0x1p-20 && d <= (T)0x1p20; }
+
+// Range test of a group of numerators (the tiers below).  Float, in three
+// instructions per value, the same predicate as mk_ok on every lane: the
+// smallest of 2*bits - 2 (unsigned; a zero of either sign maps to 0xfffffffe,
+// a magnitude below 2^-100 below 2*0x0d800000 - 2) and the largest |x| (NaN
+// is ignored by fmaxf; it stays NaN on every path).
+template <typename T>
+struct RangeAccT;
+template <>
+struct RangeAccT<float> {
+  unsigned lo = 0xffffffffu;
+  float hi = 0.f;
+  __device__ __forceinline__ void add(float x) {
+    lo = min(lo, __float_as_uint(x) * 2u - 2u);
+    hi = fmaxf(hi, fabsf(x));
+  }
+  __device__ __forceinline__ bool ok() const { return lo >= 2u * 0x0D800000u - 2u && hi < 0x1p100f; }
+  __device__ __forceinline__ bool below_huge() const { return hi < 0x1p100f; }
+};
+using RangeAcc = RangeAccT<float>;
+// Double: every value zero or of magnitude in [2^-900, 2^900); NaN and
+// infinities fail
+template <>
+struct RangeAccT<double> {
+  bool good = true;
+  __device__ __forceinline__ void add(double x) {
+    const unsigned h = (unsigned)__double2hiint(x) & 0x7fffffffu;
+    const unsigned z = h | (unsigned)__double2loint(x);
+    good = good & ((h - (123u << 20) < (1800u << 20)) | (z == 0u));
+  }
+  __device__ __forceinline__ bool ok() const { return good; }
+};
 
 // ---- groups of exact quotients without a per-lane range branch -------------
 // mk_ok: x is zero or of magnitude in [2^-100, 2^100), where div_c's
