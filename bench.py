@@ -795,10 +795,11 @@ def main(argv=None):
     # per run: velocity + stress kernel per time step, plus the first step's
     # moment-tensor injection (receivers and next-step sources ride inside the
     # stress kernel); w.reset() zeroes the state with torch fills
-    launches_per_run = 2 * nt + 1
-    info = w._plan.info() if three_d else {"path": "two_pass"}
+    # (2D: the whole run is one on-chip launch)
+    launches_per_run = 2 * nt + 1 if three_d else 1
+    info = w._plan.info() if three_d else {"path": "two_pass", "run": "on-chip loop"}
     kname = {"staged": "k3s_velocity + k3s_stress", "two_pass": "k3_velocity + k3_stress",
-             "fused": "k3_fused"}.get(info["path"], info["path"]) if three_d else "k2_velocity + k2_stress"
+             "fused": "k3_fused"}.get(info["path"], info["path"]) if three_d else "k2r_run"
     if rank == 0:
         line = {
             "metric": "Gcell-updates/s", "value": value, "unit": "Gcell-updates/s", "n_gpus": world,

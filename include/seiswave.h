@@ -188,18 +188,21 @@ SW_API int sw_check_division(float divisor, int32_t mode, uint64_t* mismatches, 
 
 /* Block until the stream is idle and report a device-side failure recorded
  * by the plan's kernels since the previous status read (SW_ERR_TIMEOUT: a
- * bounded wait for TMA data, or a grid barrier of the 2D persistent run, gave
- * up); a failure is reported once and then cleared, so a caller may retry.  No reference counterpart (the reference has no error
+ * bounded wait for TMA data, for a tile's rims in the 2D on-chip run or for a
+ * grid barrier of the 2D persistent run gave up); a failure is reported once and then cleared, so a caller may retry.  No reference counterpart (the reference has no error
  * path); it is the status read the drivers' loops can add after run(). */
 SW_API int sw_plan_status(sw_plan* plan, void* stream);
 
 /* Describe the plan's execution path: info[0] current path of sw_step/sw_run
- * (0 register-queue two-pass kernels, 2D: two launches per step, 1 TMA-staged
+ * (0 register-queue two-pass kernels; 2D: sw_step and sw_run without a graph
+ * make two launches per step, sw_run with one keeps runs of at least 4 steps of
+ * orders up to 4 that record a velocity on the chip where their tiles fit --
+ * one cooperative launch, neighbouring tiles exchange their rims -- and
+ * replays the launches otherwise; 1 TMA-staged
  * two-pass kernels, 2 fused single-pass kernel, 3 2D persistent: sw_run is
  * one cooperative launch for all its steps, the phases separated by a
- * bounded grid barrier; opt-in, as the two launches per step replayed from
- * a CUDA graph are faster on B200 at every grid size measured; sw_step
- * keeps the two launches), [1] constant-divisor fast path verified, [2] staged
+ * bounded grid barrier; opt-in, as path 0 is faster on B200 at every grid
+ * size measured; sw_step keeps the two launches), [1] constant-divisor fast path verified, [2] staged
  * path available, [3] its grid, [4] its x-chunk length, [5] fused path set
  * up, [6] its grid, [7] its x-chunk length, [8] exact numerics (see
  * sw_plan_set_exact).  info must hold 9 int32. */

@@ -17,6 +17,7 @@
 #include <type_traits>
 
 #include "sw_fused.cuh"
+#include "sw_resident2d.cuh"
 #include "sw_staged.cuh"
 
 namespace sw {
@@ -154,6 +155,10 @@ struct sw_plan {
   int path = 0;
   unsigned int* d_bar = nullptr;  // 2D persistent path: grid-barrier arrival and generation words
   bool aea = false;               // free-surface hook before every step (sw_plan_set_free_surface)
+  // 2D on-chip loop (sw_run of path 0): tiles (0: not available) and the rim inbox
+  int res_tx = 0, res_tz = 0, res_words = 0, res_width = 0;
+  size_t res_smem = 0;
+  uint64_t* d_inbox = nullptr;
 };
 
 namespace {
@@ -627,6 +632,93 @@ cudaError_t persistent_run2(sw_plan* pl, int it0, int nsteps, cudaStream_t st) {
                                     pl->gather_in_stress, pl->d_bar, pl->d_err, st);
 }
 
+// ---------------------------------------------------------------------------
+// 2D loops that stay on the chip (elastic2d_resident.cu)
+// ---------------------------------------------------------------------------
+
+// SMs and shared memory per block of the current device; blocks = 0 where a
+// cooperative launch is not possible
+void resident_limits(int* blocks, size_t* smem) {
+  int dev = 0, sms = 0, coop = 0, lim = 0;
+  *blocks = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&lim, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess) {
+    cudaGetLastError();
+    return;
+  }
+  if (coop) *blocks = sms;
+  *smem = lim > 64 ? (size_t)lim - 64 : 0;  // 64: the kernel's static shared memory
+}
+
+// The on-chip loop covers the SSG schemes of orders up to SW_RES_ORDER whose
+// receivers record a velocity and whose tiles fit the device.
+bool resident_covers(const sw_plan* pl) {
+  return pl->dim == 2 && (pl->scheme == SW2D_SSG_VS || pl->scheme == SW2D_SSG_SV) && pl->order <= SW_RES_ORDER &&
+         pl->gather_in_stress;
+}
+
+void setup_resident(sw_plan* pl) {
+  pl->res_tx = 0;
+  if (!resident_covers(pl)) return;
+  int blocks;
+  size_t smem;
+  resident_limits(&blocks, &smem);
+  int tx, tz, words, width;
+  size_t bytes;
+  const bool ok = pl->dtype == SW_F32 ? sw::sw2r_tiles<float>(pl->p2f, pl->order, blocks, smem, 0, &tx, &tz, &words, &bytes, &width)
+                                      : sw::sw2r_tiles<double>(pl->p2d, pl->order, blocks, smem, 0, &tx, &tz, &words, &bytes, &width);
+  if (!ok) return;
+  pl->res_tx = tx;
+  pl->res_tz = tz;
+  pl->res_words = words;
+  pl->res_width = width;
+  pl->res_smem = bytes;
+}
+
+template <typename T>
+cudaError_t resident_run_t(sw_plan* pl, const sw::P2<T>& p, int it0, int nsteps, cudaStream_t st) {
+  sw::Res2<T> r{};
+  r.shots[0] = p;
+  r.n = 1;
+  r.tx[0] = pl->res_tx;
+  r.tz[0] = pl->res_tz;
+  r.stride[0] = pl->res_words;
+  r.blocks = pl->res_tx * pl->res_tz;
+  r.width = pl->res_width;
+  r.smem = pl->res_smem;
+  r.inbox = pl->d_inbox;
+  r.err = pl->d_err;
+  return sw::sw2r_run<T>(r, pl->scheme, pl->order, it0, nsteps, pl->aea ? 1 : 0, st);
+}
+
+// *done = false when the launches of the other path have to run instead: the
+// scratch could not be allocated, or not yet and the stream is being captured
+cudaError_t resident_run(sw_plan* pl, int it0, int nsteps, cudaStream_t st, bool* done) {
+  *done = false;
+  if (!pl->d_inbox || !pl->d_err) {
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) {
+      cudaGetLastError();
+      return cudaSuccess;
+    }
+    if (!pl->d_err) {
+      if (cudaMalloc(&pl->d_err, sizeof(int)) != cudaSuccess) { cudaGetLastError(); return cudaSuccess; }
+      cudaError_t e = cudaMemset(pl->d_err, 0, sizeof(int));
+      if (e != cudaSuccess) return e;
+    }
+    const size_t words = 2 * (size_t)pl->res_tx * pl->res_tz * pl->res_words;
+    if (!pl->d_inbox && cudaMalloc(&pl->d_inbox, words * sizeof(uint64_t)) != cudaSuccess) {
+      cudaGetLastError();
+      return cudaSuccess;
+    }
+  }
+  *done = true;
+  return pl->dtype == SW_F32 ? resident_run_t<float>(pl, pl->p2f, it0, nsteps, st)
+                             : resident_run_t<double>(pl, pl->p2d, it0, nsteps, st);
+}
+
 cudaError_t enqueue_sequence(sw_plan* pl, int it0, int nsteps, cudaStream_t st) {
   if (pl->fused && pl->path == 2 && nsteps >= 2 && !pl->aea) return enqueue_fused_run(pl, it0, nsteps, st);
   for (int s = 0; s < nsteps; ++s) {
@@ -697,6 +789,7 @@ int sw2d_plan_create(const sw2d_desc* d, sw_plan** out) {
   for (int q = 0; q < 5; ++q) pl->fields[q] = d->field[q];
   if (d->dtype == SW_F32) make_p2<float>(d, pl->p2f);
   else make_p2<double>(d, pl->p2d);
+  setup_resident(pl);
   *out = pl;
   return SW_OK;
 }
@@ -802,6 +895,7 @@ int sw_plan_status(sw_plan* pl, void* stream) {
     }
     if (h & 1) return fail(SW_ERR_TIMEOUT, "a bounded device wait gave up (TMA data never arrived)");
     if (h & 2) return fail(SW_ERR_TIMEOUT, "a bounded device wait gave up (grid barrier of the persistent run)");
+    if (h & 4) return fail(SW_ERR_TIMEOUT, "a bounded device wait gave up (tile rims of the on-chip 2D run)");
   }
   return SW_OK;
 }
@@ -880,6 +974,7 @@ int sw_plan_destroy(sw_plan* pl) {
   if (pl->fused_buf) cudaFree(pl->fused_buf);
   if (pl->d_err) cudaFree(pl->d_err);
   if (pl->d_bar) cudaFree(pl->d_bar);
+  if (pl->d_inbox) cudaFree(pl->d_inbox);
   delete pl;
   return SW_OK;
 }
@@ -919,6 +1014,12 @@ int sw_run(sw_plan* pl, int32_t it0, int32_t nsteps, int32_t use_graph, void* st
     e = enqueue_sequence(pl, it0, nsteps, st);
     if (e != cudaSuccess) return cuda_fail(e, "sw_run");
     return SW_OK;
+  }
+  if (pl->path == 0 && pl->res_tx > 0 && nsteps >= SW_RES_STEPS) {
+    bool done;
+    e = resident_run(pl, it0, nsteps, st, &done);
+    if (e != cudaSuccess) return cuda_fail(e, "sw_run: on-chip loop");
+    if (done) return SW_OK;
   }
   if (!(pl->gexec && pl->g_it0 == it0 && pl->g_n == nsteps)) {
     if (pl->gexec) { cudaGraphExecDestroy(pl->gexec); pl->gexec = nullptr; }

@@ -305,6 +305,16 @@ __device__ __forceinline__ double mk2_core(double x, double d, double y) {
   q = __fma_rn(__fma_rn(-q, d, x), y, q);
   return __fma_rn(__fma_rn(-q, d, x), y, q);
 }
+// mk2_core's quotient for any |x| < 2^100 (zero, below 2^-100 or above),
+// without a branch: the scaled route of mk_div_any
+__device__ __forceinline__ float tiny_finish_sel(float xs, float ys, float d);
+__device__ __forceinline__ float mk2_div_any(float x, float d, float y) {
+  const bool tiny = fabsf(x) < 0x1p-100f;
+  const float xs = tiny ? __fmul_rn(x, 0x1p64f) : x;
+  const float q = mk2_core(xs, d, y);
+  const float z = tiny ? tiny_finish_sel(xs, q, d) : q;
+  return __uint_as_float(__float_as_uint(z) | (__float_as_uint(x) & 0x80000000u));  // the sign of a zero
+}
 template <typename T>
 __device__ __forceinline__ bool mk2_divisor(T d) { return d >= (T)0x1p-20 && d <= (T)0x1p20; }
 
