@@ -143,8 +143,7 @@ __device__ __forceinline__ void cell_quotients(float (&x)[K], const float (&d)[K
   for (int k = 0; k < K; ++k) acc.add(x[k]);
   if (fast && acc.ok()) {
 #pragma unroll
-    for (int k = 0; k < K; ++k)  // a quotient by d > 0 has its numerator's sign, zeros included
-      x[k] = __uint_as_float(__float_as_uint(mk2_core(x[k], d[k], y[k])) | (__float_as_uint(x[k]) & 0x80000000u));
+    for (int k = 0; k < K; ++k) x[k] = mk2_signed(x[k], d[k], y[k]);
   } else if (fast && acc.below_huge()) {
 #pragma unroll
     for (int k = 0; k < K; ++k) x[k] = mk2_div_any(x[k], d[k], y[k]);

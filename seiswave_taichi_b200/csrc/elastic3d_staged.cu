@@ -416,176 +416,322 @@ __device__ __forceinline__ void fill_tables(const P3<float>& p, float* tyt, floa
 // ---------------------------------------------------------------------------
 enum { SCH_CPML = 0, SCH_SPML = 1 };
 
-__device__ __forceinline__ float spml_part(float psi, float term, float damp, float hdt) {
-  return div_v((1.f - hdt * damp) * psi + term, 1.f + hdt * damp);
+// One axis of a cell's split update at an integer or half point: w = 1 - dt/2 d,
+// the divisor 1 + dt/2 d and its reciprocal
+struct SplitCoef {
+  float w, den, y;
+};
+
+// A pair of cells whose split parts lie side by side in the shell, at an even
+// position (and an even component stride), moves them in 8-byte accesses
+template <int Q>
+struct SplitAt {
+  float* s;          // part 0 of the pair's first cell in the shell
+  long long off[Q];  // cell e's offset from s
+  bool pair;
+};
+
+// The NP split parts (components c0 .. c0+NP-1) of one field in a thread's Q
+// cells: psi_p = (w psi_p + term_p) / den, field = sum of the parts, for the
+// cells with on[e].  The divisors depend on one index each, so their
+// reciprocals come from tables and mk2_core gives the quotients (mk: all
+// divisors in its range); numerators below 2^-100 take its scaled form, the
+// rest div_v.  Every tier gives div_v's bits.  What bounded the split passes
+// was the chain of one branching IEEE division after another and 4-byte
+// accesses to the parts: at 200^3 the groups and pairs took the velocity pass
+// from 478 to 335 us and the stress pass from 747 to 530 us.
+template <int NP, int Q>
+__device__ __forceinline__ void split_update(const SplitAt<Q>& at, long long G, int c0, const bool (&on)[Q],
+                                             const float (&term)[NP][Q], const SplitCoef (&co)[NP][Q], bool mk,
+                                             Vq<Q>& f) {
+  static_assert(Q == 2, "pairs");
+  float* s = at.s + c0 * G;
+  float psi[NP][Q], x[NP][Q];
+#pragma unroll
+  for (int p = 0; p < NP; ++p) {
+    if (at.pair) {
+      const float2 v = *reinterpret_cast<const float2*>(s + p * G);
+      psi[p][0] = v.x;
+      psi[p][1] = v.y;
+    } else {
+#pragma unroll
+      for (int e = 0; e < Q; ++e) psi[p][e] = on[e] ? s[p * G + at.off[e]] : 0.f;
+    }
+  }
+  RangeAcc acc;
+#pragma unroll
+  for (int p = 0; p < NP; ++p)
+#pragma unroll
+    for (int e = 0; e < Q; ++e) {
+      x[p][e] = on[e] ? co[p][e].w * psi[p][e] + term[p][e] : 0.f;
+      acc.add(x[p][e]);
+    }
+  if (mk && acc.ok()) {
+#pragma unroll
+    for (int p = 0; p < NP; ++p)
+#pragma unroll
+      for (int e = 0; e < Q; ++e) x[p][e] = mk2_signed(x[p][e], co[p][e].den, co[p][e].y);
+  } else if (mk && acc.below_huge()) {
+#pragma unroll
+    for (int p = 0; p < NP; ++p)
+#pragma unroll
+      for (int e = 0; e < Q; ++e) x[p][e] = mk2_div_any(x[p][e], co[p][e].den, co[p][e].y);
+  } else {
+#pragma unroll
+    for (int p = 0; p < NP; ++p)
+#pragma unroll
+      for (int e = 0; e < Q; ++e) x[p][e] = div_v(x[p][e], co[p][e].den);
+  }
+#pragma unroll
+  for (int p = 0; p < NP; ++p) {
+    if (at.pair) {
+      *reinterpret_cast<float2*>(s + p * G) = make_float2(on[0] ? x[p][0] : psi[p][0], on[1] ? x[p][1] : psi[p][1]);
+    } else {
+#pragma unroll
+      for (int e = 0; e < Q; ++e)
+        if (on[e]) s[p * G + at.off[e]] = x[p][e];
+    }
+  }
+#pragma unroll
+  for (int e = 0; e < Q; ++e)
+    if (on[e]) {
+      float v = x[0][e] + x[1][e];
+      if constexpr (NP == 3) v = v + x[2][e];
+      s4(f, e, v);
+    }
 }
 
+// per-plane, per-row and per-cell split coefficients of a thread: [0] at the
+// integer, [1] at the half point
 template <int Q>
-__device__ __forceinline__ void spml_velocity(const P3<float>& p, int i, int j, int k, uint8_t fy,
-                                              const uint8_t (&fz)[Q], float dt, const bool (&mx)[Q],
-                                              const bool (&my)[Q], const bool (&mz)[Q], const Vq<Q>& a1,
-                                              const Vq<Q>& a2, const Vq<Q>& a3, const Vq<Q>& b1, const Vq<Q>& b2,
-                                              const Vq<Q>& b3, const Vq<Q>& c1, const Vq<Q>& c2, const Vq<Q>& c3,
-                                              const Vq<Q>& rc, const Vq<Q>& rn, const Vq<Q>& r1c, const Vq<Q>& r1n,
-                                              Vq<Q>& vx, Vq<Q>& vy, Vq<Q>& vz) {
-  const int nx = p.nx, ny = p.ny, nz = p.nz;
-  const uint8_t fx = p.fl[0][i];
-  const float hdt = 0.5f * dt;
-  const float *dpx = p.dmp[0], *dpy = p.dmp[1], *dpz = p.dmp[2];
-  float* sp = p.split;
-  const long long G = p.scomp;
+struct SplitTab {
+  SplitCoef x[2], y[2], z[2][Q];
+  bool mk;  // every divisor is in mk2_core's range
+};
+
+__device__ __forceinline__ SplitCoef split_coef(float damp, float hdt) {
+  SplitCoef c;
+  c.w = 1.f - hdt * damp;
+  c.den = 1.f + hdt * damp;
+  c.y = __frcp_rn(c.den);
+  return c;
+}
+
+// the row's and the z cells' coefficients (true when in mk2_core's range),
+// then the plane's
+template <int Q>
+__device__ __forceinline__ bool split_tab_yz(const P3<float>& p, int j, int k, bool jin, float hdt, SplitTab<Q>& t) {
+  bool ok = true;
 #pragma unroll
-  for (int e = 0; e < Q; ++e) {
-    const int kk = k + e;
-    const uint8_t fze = fz[e];
-    const long long sh = (fx | fy | fze) ? shell_index(p, i, j, kk) : 0;
-    const float rce = g4(rc, e), rne = g4(rn, e);
-    // vx (:182-205): x half, y and z integer; rho unaveraged
-    if (mx[e]) {
-      const float ro = __fdiv_rn(1.f, rce);
-      const float d1 = g4(a1, e), d2 = g4(a2, e), d3 = g4(a3, e);
-      if ((fx & 2) || (fy & 1) || (fze & 1)) {
-        float* s = sp + PVX_X * G + sh;
-        const float A = spml_part(s[0], d1 * dt * ro, __ldg(dpx + nx + i), hdt);
-        const float B = spml_part(s[G], d2 * dt * ro, __ldg(dpy + j), hdt);
-        const float C = spml_part(s[2 * G], d3 * dt * ro, __ldg(dpz + kk), hdt);
-        s[0] = A;
-        s[G] = B;
-        s[2 * G] = C;
-        s4(vx, e, A + B + C);
-      } else {
-        s4(vx, e, g4(vx, e) + (d1 + d2 + d3) * dt * ro);
-      }
+  for (int h = 0; h < 2; ++h) {
+    t.y[h] = split_coef(jin ? __ldg(p.dmp[1] + h * p.ny + j) : 0.f, hdt);
+    ok = ok && mk2_divisor(t.y[h].den);
+#pragma unroll
+    for (int e = 0; e < Q; ++e) {
+      t.z[h][e] = split_coef(k + e < p.nz ? __ldg(p.dmp[2] + h * p.nz + k + e) : 0.f, hdt);
+      ok = ok && mk2_divisor(t.z[h][e].den);
     }
-    // vy (:209-233): y half; rho averaged over j, j+1
-    if (my[e]) {
-      const float ro = __fdiv_rn(1.f, 0.5f * (rce + rne));
-      const float d1 = g4(b1, e), d2 = g4(b2, e), d3 = g4(b3, e);
-      if ((fx & 1) || (fy & 2) || (fze & 1)) {
-        float* s = sp + PVY_X * G + sh;
-        const float A = spml_part(s[0], dt * d1 * ro, __ldg(dpx + i), hdt);
-        const float B = spml_part(s[G], dt * d2 * ro, __ldg(dpy + ny + j), hdt);
-        const float C = spml_part(s[2 * G], dt * d3 * ro, __ldg(dpz + kk), hdt);
-        s[0] = A;
-        s[G] = B;
-        s[2 * G] = C;
-        s4(vy, e, A + B + C);
-      } else {
-        s4(vy, e, g4(vy, e) + (d1 + d2 + d3) * dt * ro);
-      }
-    }
-    // vz (:235-259): z half; rho averaged over the x-y quad
-    if (mz[e]) {
-      const float ro = __fdiv_rn(1.f, 0.25f * (rce + rne + g4(r1n, e) + g4(r1c, e)));
-      const float d1 = g4(c1, e), d2 = g4(c2, e), d3 = g4(c3, e);
-      if ((fx & 1) || (fy & 1) || (fze & 2)) {
-        float* s = sp + PVZ_X * G + sh;
-        const float A = spml_part(s[0], dt * d1 * ro, __ldg(dpx + i), hdt);
-        const float B = spml_part(s[G], dt * d2 * ro, __ldg(dpy + j), hdt);
-        const float C = spml_part(s[2 * G], dt * d3 * ro, __ldg(dpz + nz + kk), hdt);
-        s[0] = A;
-        s[G] = B;
-        s[2 * G] = C;
-        s4(vz, e, A + B + C);
-      } else {
-        s4(vz, e, g4(vz, e) + (d1 + d2 + d3) * dt * ro);
-      }
-    }
+  }
+  return ok;
+}
+template <int Q>
+__device__ __forceinline__ void split_tab_x(const P3<float>& p, int i, float hdt, bool yz, SplitTab<Q>& t) {
+  t.mk = yz;
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    t.x[h] = split_coef(__ldg(p.dmp[0] + h * p.nx + i), hdt);
+    t.mk = t.mk && mk2_divisor(t.x[h].den);
   }
 }
 
 template <int Q>
-__device__ __forceinline__ void spml_stress(const P3<float>& p, int i, int j, int k, uint8_t fy,
-                                            const uint8_t (&fz)[Q], float dt, const bool (&mn)[Q],
-                                            const bool (&mxy)[Q], const bool (&mxz)[Q], const bool (&myz)[Q],
-                                            const Vq<Q>& e1, const Vq<Q>& e2, const Vq<Q>& e3, const Vq<Q>& f1,
-                                            const Vq<Q>& f2, const Vq<Q>& h1, const Vq<Q>& h2, const Vq<Q>& q1,
-                                            const Vq<Q>& q2, const Vq<Q>& l0, const Vq<Q>& u0, const Vq<Q>& u1,
-                                            const Vq<Q>& unj, const float (&unk)[Q], Vq<Q>& sxx, Vq<Q>& syy,
-                                            Vq<Q>& szz, Vq<Q>& sxy, Vq<Q>& sxz, Vq<Q>& syz) {
-  const int nx = p.nx, ny = p.ny, nz = p.nz;
-  const uint8_t fx = p.fl[0][i];
-  const float hdt = 0.5f * dt;
-  const float *dpx = p.dmp[0], *dpy = p.dmp[1], *dpz = p.dmp[2];
-  float* sp = p.split;
+__device__ __forceinline__ SplitAt<Q> split_at(const P3<float>& p, int i, int j, int k, uint8_t fxy,
+                                               const uint8_t (&fz)[Q]) {
+  SplitAt<Q> at;
+  const bool in0 = fxy | fz[0], in1 = fxy | fz[Q - 1];
+  const long long s0 = in0 ? shell_index(p, i, j, k) : 0;
+  const long long s1 = in1 ? shell_index(p, i, j, k + Q - 1) : 0;
+  const long long base = in0 ? s0 : s1;
+  at.s = p.split + base;
+  at.off[0] = 0;
+  at.off[Q - 1] = s1 - base;
+  at.pair = in0 && in1 && s1 == s0 + 1 && ((s0 | p.scomp) & 1) == 0 && ((uintptr_t)p.split & 7) == 0;
+  return at;
+}
+
+template <int Q>
+__device__ __forceinline__ void spml_velocity(const P3<float>& p, int i, int j, int k, uint8_t fx, uint8_t fy,
+                                              const uint8_t (&fz)[Q], float dt, const SplitTab<Q>& t,
+                                              const bool (&mx)[Q], const bool (&my)[Q], const bool (&mz)[Q],
+                                              const Vq<Q>& a1, const Vq<Q>& a2, const Vq<Q>& a3, const Vq<Q>& b1,
+                                              const Vq<Q>& b2, const Vq<Q>& b3, const Vq<Q>& c1, const Vq<Q>& c2,
+                                              const Vq<Q>& c3, const Vq<Q>& rc, const Vq<Q>& rn, const Vq<Q>& r1c,
+                                              const Vq<Q>& r1n, Vq<Q>& vx, Vq<Q>& vy, Vq<Q>& vz) {
   const long long G = p.scomp;
+  const SplitAt<Q> at = split_at<Q>(p, i, j, k, fx | fy, fz);
+  // vx (:182-205): x half, y and z integer; rho unaveraged
+  float ro[Q];
+  bool on[Q];
 #pragma unroll
   for (int e = 0; e < Q; ++e) {
-    const int kk = k + e;
-    const uint8_t fze = fz[e];
-    const long long sh = (fx | fy | fze) ? shell_index(p, i, j, kk) : 0;
-    const float u = g4(u0, e);
-    // normal stresses (:296-333): unaveraged lambda and mu
-    if (mn[e]) {
-      const float lm = g4(l0, e);
-      const float l2m = lm + 2.f * u;
+    ro[e] = __fdiv_rn(1.f, g4(rc, e));
+    on[e] = mx[e] && ((fx & 2) || (fy & 1) || (fz[e] & 1));
+    if (mx[e] && !on[e]) s4(vx, e, g4(vx, e) + (g4(a1, e) + g4(a2, e) + g4(a3, e)) * dt * ro[e]);
+  }
+  if (on[0] | on[Q - 1]) {
+    float term[3][Q];
+    SplitCoef co[3][Q];
+#pragma unroll
+    for (int e = 0; e < Q; ++e) {
+      term[0][e] = g4(a1, e) * dt * ro[e];
+      term[1][e] = g4(a2, e) * dt * ro[e];
+      term[2][e] = g4(a3, e) * dt * ro[e];
+      co[0][e] = t.x[1]; co[1][e] = t.y[0]; co[2][e] = t.z[0][e];
+    }
+    split_update<3, Q>(at, G, PVX_X, on, term, co, t.mk, vx);
+  }
+  // vy (:209-233): y half; rho averaged over j, j+1
+#pragma unroll
+  for (int e = 0; e < Q; ++e) {
+    ro[e] = __fdiv_rn(1.f, 0.5f * (g4(rc, e) + g4(rn, e)));
+    on[e] = my[e] && ((fx & 1) || (fy & 2) || (fz[e] & 1));
+    if (my[e] && !on[e]) s4(vy, e, g4(vy, e) + (g4(b1, e) + g4(b2, e) + g4(b3, e)) * dt * ro[e]);
+  }
+  if (on[0] | on[Q - 1]) {
+    float term[3][Q];
+    SplitCoef co[3][Q];
+#pragma unroll
+    for (int e = 0; e < Q; ++e) {
+      term[0][e] = dt * g4(b1, e) * ro[e];
+      term[1][e] = dt * g4(b2, e) * ro[e];
+      term[2][e] = dt * g4(b3, e) * ro[e];
+      co[0][e] = t.x[0]; co[1][e] = t.y[1]; co[2][e] = t.z[0][e];
+    }
+    split_update<3, Q>(at, G, PVY_X, on, term, co, t.mk, vy);
+  }
+  // vz (:235-259): z half; rho averaged over the x-y quad
+#pragma unroll
+  for (int e = 0; e < Q; ++e) {
+    ro[e] = __fdiv_rn(1.f, 0.25f * (g4(rc, e) + g4(rn, e) + g4(r1n, e) + g4(r1c, e)));
+    on[e] = mz[e] && ((fx & 1) || (fy & 1) || (fz[e] & 2));
+    if (mz[e] && !on[e]) s4(vz, e, g4(vz, e) + (g4(c1, e) + g4(c2, e) + g4(c3, e)) * dt * ro[e]);
+  }
+  if (on[0] | on[Q - 1]) {
+    float term[3][Q];
+    SplitCoef co[3][Q];
+#pragma unroll
+    for (int e = 0; e < Q; ++e) {
+      term[0][e] = dt * g4(c1, e) * ro[e];
+      term[1][e] = dt * g4(c2, e) * ro[e];
+      term[2][e] = dt * g4(c3, e) * ro[e];
+      co[0][e] = t.x[0]; co[1][e] = t.y[0]; co[2][e] = t.z[1][e];
+    }
+    split_update<3, Q>(at, G, PVZ_X, on, term, co, t.mk, vz);
+  }
+}
+
+template <int Q>
+__device__ __forceinline__ void spml_stress(const P3<float>& p, int i, int j, int k, uint8_t fx, uint8_t fy,
+                                            const uint8_t (&fz)[Q], float dt, const SplitTab<Q>& t,
+                                            const bool (&mn)[Q], const bool (&mxy)[Q], const bool (&mxz)[Q],
+                                            const bool (&myz)[Q], const Vq<Q>& e1, const Vq<Q>& e2, const Vq<Q>& e3,
+                                            const Vq<Q>& f1, const Vq<Q>& f2, const Vq<Q>& h1, const Vq<Q>& h2,
+                                            const Vq<Q>& q1, const Vq<Q>& q2, const Vq<Q>& l0, const Vq<Q>& u0,
+                                            const Vq<Q>& u1, const Vq<Q>& unj, const float (&unk)[Q], Vq<Q>& sxx,
+                                            Vq<Q>& syy, Vq<Q>& szz, Vq<Q>& sxy, Vq<Q>& sxz, Vq<Q>& syz) {
+  const long long G = p.scomp;
+  const SplitAt<Q> at = split_at<Q>(p, i, j, k, fx | fy, fz);
+  bool on[Q];
+  // normal stresses (:296-333): unaveraged lambda and mu
+#pragma unroll
+  for (int e = 0; e < Q; ++e) {
+    on[e] = mn[e] && ((fx | fy | fz[e]) & 1);
+    if (mn[e] && !on[e]) {
+      const float lm = g4(l0, e), l2m = lm + 2.f * g4(u0, e);
       const float A = g4(e1, e), B = g4(e2, e), Cc = g4(e3, e);
-      if ((fx | fy | fze) & 1) {
-        const float dX = __ldg(dpx + i), dY = __ldg(dpy + j), dZ = __ldg(dpz + kk);
-        float* s = sp + sh;
-        const float xx = spml_part(s[PSXX_X * G], dt * l2m * A, dX, hdt);
-        const float xy = spml_part(s[PSXX_Y * G], dt * lm * B, dY, hdt);
-        const float xz = spml_part(s[PSXX_Z * G], dt * lm * Cc, dZ, hdt);
-        const float yx = spml_part(s[PSYY_X * G], dt * lm * A, dX, hdt);
-        const float yy = spml_part(s[PSYY_Y * G], dt * l2m * B, dY, hdt);
-        const float yz = spml_part(s[PSYY_Z * G], dt * lm * Cc, dZ, hdt);
-        const float zx = spml_part(s[PSZZ_X * G], dt * lm * A, dX, hdt);
-        const float zy = spml_part(s[PSZZ_Y * G], dt * lm * B, dY, hdt);
-        const float zz = spml_part(s[PSZZ_Z * G], dt * l2m * Cc, dZ, hdt);
-        s[PSXX_X * G] = xx; s[PSXX_Y * G] = xy; s[PSXX_Z * G] = xz;
-        s[PSYY_X * G] = yx; s[PSYY_Y * G] = yy; s[PSYY_Z * G] = yz;
-        s[PSZZ_X * G] = zx; s[PSZZ_Y * G] = zy; s[PSZZ_Z * G] = zz;
-        s4(sxx, e, xx + xy + xz);
-        s4(syy, e, yx + yy + yz);
-        s4(szz, e, zx + zy + zz);
-      } else {
-        s4(sxx, e, g4(sxx, e) + (l2m * A + lm * (Cc + B)) * dt);
-        s4(syy, e, g4(syy, e) + (l2m * B + lm * (A + Cc)) * dt);
-        s4(szz, e, g4(szz, e) + (l2m * Cc + lm * (A + B)) * dt);
-      }
+      s4(sxx, e, g4(sxx, e) + (l2m * A + lm * (Cc + B)) * dt);
+      s4(syy, e, g4(syy, e) + (l2m * B + lm * (A + Cc)) * dt);
+      s4(szz, e, g4(szz, e) + (l2m * Cc + lm * (A + B)) * dt);
     }
-    // sxy (:334-350): x half, y half
-    if (mxy[e]) {
-      const float m4 = 0.25f * (g4(unj, e) + u + u + g4(u1, e));
-      if ((fx & 2) || (fy & 2) || (fze & 1)) {
-        float* s = sp + PSXY_X * G + sh;
-        const float a = spml_part(s[0], dt * m4 * g4(f1, e), __ldg(dpx + nx + i), hdt);
-        const float b = spml_part(s[G], dt * m4 * g4(f2, e), __ldg(dpy + ny + j), hdt);
-        s[0] = a;
-        s[G] = b;
-        s4(sxy, e, a + b);
-      } else {
-        s4(sxy, e, g4(sxy, e) + m4 * (g4(f2, e) + g4(f1, e)) * dt);
-      }
+  }
+  if (on[0] | on[Q - 1]) {
+    SplitCoef co[3][Q];
+#pragma unroll
+    for (int e = 0; e < Q; ++e) {
+      co[0][e] = t.x[0]; co[1][e] = t.y[0]; co[2][e] = t.z[0][e];
     }
-    // sxz (:352-371): x half, z half
-    if (mxz[e]) {
-      const float m4 = 0.25f * (u + g4(u1, e) + u + g4(unj, e));
-      if ((fx & 2) || (fy & 1) || (fze & 2)) {
-        float* s = sp + PSXZ_X * G + sh;
-        const float a = spml_part(s[0], dt * m4 * g4(h1, e), __ldg(dpx + nx + i), hdt);
-        const float b = spml_part(s[G], dt * m4 * g4(h2, e), __ldg(dpz + nz + kk), hdt);
-        s[0] = a;
-        s[G] = b;
-        s4(sxz, e, a + b);
-      } else {
-        s4(sxz, e, g4(sxz, e) + m4 * (g4(h2, e) + g4(h1, e)) * dt);
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {  // sxx syy szz: lambda + 2 mu on the component's own axis
+      float term[3][Q];
+#pragma unroll
+      for (int e = 0; e < Q; ++e) {
+        const float lm = g4(l0, e), l2m = lm + 2.f * g4(u0, e);
+        term[0][e] = dt * (q == 0 ? l2m : lm) * g4(e1, e);
+        term[1][e] = dt * (q == 1 ? l2m : lm) * g4(e2, e);
+        term[2][e] = dt * (q == 2 ? l2m : lm) * g4(e3, e);
       }
+      if (q == 0) split_update<3, Q>(at, G, PSXX_X, on, term, co, t.mk, sxx);
+      else if (q == 1) split_update<3, Q>(at, G, PSYY_X, on, term, co, t.mk, syy);
+      else split_update<3, Q>(at, G, PSZZ_X, on, term, co, t.mk, szz);
     }
-    // syz (:373-391): y half, z half; its plain update adds dvy/dz + dvz/dy
-    if (myz[e]) {
-      const float m4 = 0.25f * (g4(unj, e) + u + unk[e] + u);
-      if ((fx & 1) || (fy & 2) || (fze & 2)) {
-        float* s = sp + PSYZ_Y * G + sh;
-        const float a = spml_part(s[0], dt * m4 * g4(q1, e), __ldg(dpy + ny + j), hdt);
-        const float b = spml_part(s[G], dt * m4 * g4(q2, e), __ldg(dpz + nz + kk), hdt);
-        s[0] = a;
-        s[G] = b;
-        s4(syz, e, a + b);
-      } else {
-        s4(syz, e, g4(syz, e) + m4 * (g4(q2, e) + g4(q1, e)) * dt);
-      }
+  }
+  // sxy (:334-350): x half, y half
+  float m4[Q];
+#pragma unroll
+  for (int e = 0; e < Q; ++e) {
+    const float u = g4(u0, e);
+    m4[e] = 0.25f * (g4(unj, e) + u + u + g4(u1, e));
+    on[e] = mxy[e] && ((fx & 2) || (fy & 2) || (fz[e] & 1));
+    if (mxy[e] && !on[e]) s4(sxy, e, g4(sxy, e) + m4[e] * (g4(f2, e) + g4(f1, e)) * dt);
+  }
+  if (on[0] | on[Q - 1]) {
+    float term[2][Q];
+    SplitCoef co[2][Q];
+#pragma unroll
+    for (int e = 0; e < Q; ++e) {
+      term[0][e] = dt * m4[e] * g4(f1, e);
+      term[1][e] = dt * m4[e] * g4(f2, e);
+      co[0][e] = t.x[1]; co[1][e] = t.y[1];
     }
+    split_update<2, Q>(at, G, PSXY_X, on, term, co, t.mk, sxy);
+  }
+  // sxz (:352-371): x half, z half
+#pragma unroll
+  for (int e = 0; e < Q; ++e) {
+    const float u = g4(u0, e);
+    m4[e] = 0.25f * (u + g4(u1, e) + u + g4(unj, e));
+    on[e] = mxz[e] && ((fx & 2) || (fy & 1) || (fz[e] & 2));
+    if (mxz[e] && !on[e]) s4(sxz, e, g4(sxz, e) + m4[e] * (g4(h2, e) + g4(h1, e)) * dt);
+  }
+  if (on[0] | on[Q - 1]) {
+    float term[2][Q];
+    SplitCoef co[2][Q];
+#pragma unroll
+    for (int e = 0; e < Q; ++e) {
+      term[0][e] = dt * m4[e] * g4(h1, e);
+      term[1][e] = dt * m4[e] * g4(h2, e);
+      co[0][e] = t.x[1]; co[1][e] = t.z[1][e];
+    }
+    split_update<2, Q>(at, G, PSXZ_X, on, term, co, t.mk, sxz);
+  }
+  // syz (:373-391): y half, z half; its plain update adds dvy/dz + dvz/dy
+#pragma unroll
+  for (int e = 0; e < Q; ++e) {
+    const float u = g4(u0, e);
+    m4[e] = 0.25f * (g4(unj, e) + u + unk[e] + u);
+    on[e] = myz[e] && ((fx & 1) || (fy & 2) || (fz[e] & 2));
+    if (myz[e] && !on[e]) s4(syz, e, g4(syz, e) + m4[e] * (g4(q2, e) + g4(q1, e)) * dt);
+  }
+  if (on[0] | on[Q - 1]) {
+    float term[2][Q];
+    SplitCoef co[2][Q];
+#pragma unroll
+    for (int e = 0; e < Q; ++e) {
+      term[0][e] = dt * m4[e] * g4(q1, e);
+      term[1][e] = dt * m4[e] * g4(q2, e);
+      co[0][e] = t.y[1]; co[1][e] = t.z[1][e];
+    }
+    split_update<2, Q>(at, G, PSYZ_Y, on, term, co, t.mk, syz);
   }
 }
 
@@ -668,6 +814,9 @@ k3s_velocity(const __grid_constant__ P3<float> p, const __grid_constant__ Staged
     uint8_t fz[Q];
 #pragma unroll
     for (int e = 0; e < Q; ++e) fz[e] = SCH == SCH_SPML && k + e < nz ? p.fl[2][k + e] : 0;
+    SplitTab<Q> st;  // split PML: the coefficients of the row and of the z cells
+    bool st_yz = false;
+    if constexpr (SCH == SCH_SPML) st_yz = split_tab_yz<Q>(p, j, k, jin, 0.5f * dt, st);
     bool kxy[Q], kz[Q];
 #pragma unroll
     for (int e = 0; e < Q; ++e) {
@@ -764,7 +913,8 @@ k3s_velocity(const __grid_constant__ P3<float> p, const __grid_constant__ Staged
         const Vq<Q> rc = ldq<Q>(r0 + o_xx), rn = ldq<Q>(r0 + o_xx + G::TZ);
         const Vq<Q> r1c = ldq<Q>(r1 + o_xx), r1n = ldq<Q>(r1 + o_xx + G::TZ);
         if constexpr (SCH == SCH_SPML) {
-          spml_velocity<Q>(p, i, j, k, fy, fz, dt, mx, my, mz, a1, a2, a3, b1, b2, b3, c1, c2, c3, rc, rn, r1c, r1n,
+          split_tab_x<Q>(p, i, 0.5f * dt, st_yz, st);
+          spml_velocity<Q>(p, i, j, k, p.fl[0][i], fy, fz, dt, st, mx, my, mz, a1, a2, a3, b1, b2, b3, c1, c2, c3, rc, rn, r1c, r1n,
                            vx, vy, vz);
         } else {
           // CPML: components 0 (vx), 1 (vy), 2 (vz) of each axis; vx is at
@@ -930,6 +1080,9 @@ k3s_stress(const __grid_constant__ P3<float> p, const __grid_constant__ StagedMa
     uint8_t fz[Q];
 #pragma unroll
     for (int e = 0; e < Q; ++e) fz[e] = SCH == SCH_SPML && k + e < nz ? p.fl[2][k + e] : 0;
+    SplitTab<Q> st;  // split PML: the coefficients of the row and of the z cells
+    bool st_yz = false;
+    if constexpr (SCH == SCH_SPML) st_yz = split_tab_yz<Q>(p, j, k, jin, 0.5f * dt, st);
     bool kn[Q], kxy[Q], kh[Q];
 #pragma unroll
     for (int e = 0; e < Q; ++e) {
@@ -1038,7 +1191,8 @@ k3s_stress(const __grid_constant__ P3<float> p, const __grid_constant__ StagedMa
         for (int e = 0; e + 1 < Q; ++e) unk[e] = g4(u0, e + 1);
         unk[Q - 1] = m0p[o_m + Q];
         if constexpr (SCH == SCH_SPML) {
-          spml_stress<Q>(p, i, j, k, fy, fz, dt, mn, mxy, mxz, myz, e1, e2, e3, f1, f2, h1, h2, q1, q2, l0, u0, u1,
+          split_tab_x<Q>(p, i, 0.5f * dt, st_yz, st);
+          spml_stress<Q>(p, i, j, k, p.fl[0][i], fy, fz, dt, st, mn, mxy, mxz, myz, e1, e2, e3, f1, f2, h1, h2, q1, q2, l0, u0, u1,
                          unj, unk, sxx, syy, szz, sxy, sxz, syz);
         } else {
           // CPML: components 3 (normal), 4, 5 of each axis

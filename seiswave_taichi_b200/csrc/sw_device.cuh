@@ -315,6 +315,11 @@ __device__ __forceinline__ float mk2_div_any(float x, float d, float y) {
   const float z = tiny ? tiny_finish_sel(xs, q, d) : q;
   return __uint_as_float(__float_as_uint(z) | (__float_as_uint(x) & 0x80000000u));  // the sign of a zero
 }
+// with the sign of a zero numerator (a quotient by d > 0 has its numerator's
+// sign, zeros included)
+__device__ __forceinline__ float mk2_signed(float x, float d, float y) {
+  return __uint_as_float(__float_as_uint(mk2_core(x, d, y)) | (__float_as_uint(x) & 0x80000000u));
+}
 template <typename T>
 __device__ __forceinline__ bool mk2_divisor(T d) { return d >= (T)0x1p-20 && d <= (T)0x1p20; }
 
