@@ -227,47 +227,46 @@ __device__ __forceinline__ float mk_div_tiny(float x, float d, float r) {
   return tiny_finish(xs, mk_core(xs, d, r), d);
 }
 
-// tiny_finish without branches, for groups whose lanes take different routes:
-// both outcomes computed, one selected.  Adding and taking away 2^23 with t's
-// sign rounds |t| <= 2^23 to the nearest integer (ties to even) on the FMA
-// pipe; floorf, truncf and rintf run at an eighth of its rate.  Where t is a
-// midpoint (diff = +-1/2) the residual's sign says on which side of it x/d
-// lies; a quotient on the other side than n moves n by one.
-__device__ __forceinline__ float tiny_finish_sel(float xs, float ys, float d) {
-  const float t = __fmul_rn(ys, 0x1p85f);
-  const unsigned sg = __float_as_uint(t) & 0x80000000u;
-  const float m = __uint_as_float(sg | 0x4b000000u);  // 2^23 with t's sign
-  const float n0 = __fadd_rn(__fadd_rn(t, m), -m);
-  const float diff = __fadd_rn(t, -n0);
+// Branch-free forms for groups whose lanes take different routes.  Numerators
+// below 2^-100 are scaled by up = 2^64, the others by up = 1, down = 1/up;
+// scaled_finish takes the correctly rounded quotient ys = RN(xs/d) back to
+// the caller's scale.  ys*down rounds again only in the subnormal range, and
+// that can only differ from rounding x/d directly when ys is a midpoint of the
+// subnormal grid (diff, what the rounding took away, is half a unit: 2^-150
+// scaled back up) while the quotient is not; then the exact residual's sign
+// says on which side of ys the quotient lies, and r moves by one unit when it
+// went to the other side.  16 operations for a quotient by a spacing; the form
+// before it, which rounded on an integer grid, took 28.
+__device__ __forceinline__ float scaled_finish(float xs, float ys, float d, float up, float down) {
+  const float r = __fmul_rn(ys, down);
+  const float diff = __fmaf_rn(-r, up, ys);
   const float res = __fmaf_rn(-ys, d, xs);
-  const bool cross = fabsf(diff) == 0.5f && __fmul_rn(diff, res) > 0.f;
-  const float n = cross ? __fmaf_rn(2.f, diff, n0) : n0;
-  // n = +0 where a negative t rounds to zero: the quotient is -0 there
-  const float sub = __uint_as_float(__float_as_uint(__fmul_rn(n, 0x1p-149f)) | sg);
-  return fabsf(ys) >= 0x1p-62f ? __fmul_rn(ys, 0x1p-64f) : sub;
+  const bool cross = fabsf(diff) == 0x1p-86f && (__float_as_int(diff) ^ __float_as_int(res)) >= 0 && res != 0.f;
+  return cross ? __fmaf_rn(diff, 0x1p-63f, r) : r;
+}
+// the sign of a zero numerator (a quotient by d > 0 has its numerator's sign)
+__device__ __forceinline__ float with_sign(float y, float x) {
+  return __uint_as_float(__float_as_uint(y) | (__float_as_uint(x) & 0x80000000u));
 }
 
 // div_c's result with a verified correction (fast != 0) for any |x| < 2^100
 // -- zero, below 2^-100 or in [2^-100, 2^100) -- without a branch
 __device__ __forceinline__ float mk_div_any(float x, float d, float r) {
-  const unsigned u = __float_as_uint(x) & 0x7fffffffu;
-  const bool tiny = u < 0x0D800000u;  // |x| < 2^-100, zero included
-  const float xs = tiny ? __fmul_rn(x, 0x1p64f) : x;
-  const float q = mk_core(xs, d, r);
-  const float y = tiny ? tiny_finish_sel(xs, q, d) : q;
-  return u == 0u ? x : y;
+  const bool tiny = fabsf(x) < 0x1p-100f;
+  const float up = tiny ? 0x1p64f : 1.f, down = tiny ? 0x1p-64f : 1.f;
+  const float xs = __fmul_rn(x, up);
+  return with_sign(scaled_finish(xs, mk_core(xs, d, r), d, up, down), x);
 }
 
 // div_v's result for |x| < 2^100 and d in [2^-60, 2^60] without a branch (a
 // zero numerator divides 1 instead, so the division stays on its fast path,
 // and passes through)
 __device__ __forceinline__ float dv_div_any(float x, float d) {
-  const unsigned u = __float_as_uint(x) & 0x7fffffffu;
-  const bool tiny = u < 0x0D800000u;
-  const float xs = u == 0u ? 1.f : (tiny ? __fmul_rn(x, 0x1p64f) : x);
-  const float q = __fdiv_rn(xs, d);
-  const float y = tiny ? tiny_finish_sel(xs, q, d) : q;
-  return u == 0u ? x : y;
+  const bool tiny = fabsf(x) < 0x1p-100f;
+  const float up = tiny ? 0x1p64f : 1.f, down = tiny ? 0x1p-64f : 1.f;
+  const float xs = x == 0.f ? 1.f : __fmul_rn(x, up);
+  const float y = scaled_finish(xs, __fdiv_rn(xs, d), d, up, down);
+  return x == 0.f ? x : y;
 }
 
 // x / d for a divisor fixed for the run (dx, dy, dz), r = RN(1/d).  With
@@ -306,22 +305,16 @@ __device__ __forceinline__ double mk2_core(double x, double d, double y) {
   return __fma_rn(__fma_rn(-q, d, x), y, q);
 }
 // mk2_core's quotient for any |x| < 2^100 (zero, below 2^-100 or above),
-// without a branch: the scaled route of mk_div_any
-__device__ __forceinline__ float tiny_finish_sel(float xs, float ys, float d);
+// without a branch
 __device__ __forceinline__ float mk2_div_any(float x, float d, float y) {
   const bool tiny = fabsf(x) < 0x1p-100f;
-  const float xs = tiny ? __fmul_rn(x, 0x1p64f) : x;
-  const float q = mk2_core(xs, d, y);
-  const float z = tiny ? tiny_finish_sel(xs, q, d) : q;
-  return __uint_as_float(__float_as_uint(z) | (__float_as_uint(x) & 0x80000000u));  // the sign of a zero
-}
-// with the sign of a zero numerator (a quotient by d > 0 has its numerator's
-// sign, zeros included)
-__device__ __forceinline__ float mk2_signed(float x, float d, float y) {
-  return __uint_as_float(__float_as_uint(mk2_core(x, d, y)) | (__float_as_uint(x) & 0x80000000u));
+  const float up = tiny ? 0x1p64f : 1.f, down = tiny ? 0x1p-64f : 1.f;
+  const float xs = __fmul_rn(x, up);
+  return with_sign(scaled_finish(xs, mk2_core(xs, d, y), d, up, down), x);
 }
 template <typename T>
 __device__ __forceinline__ bool mk2_divisor(T d) { return d >= (T)0x1p-20 && d <= (T)0x1p20; }
+__device__ __forceinline__ float mk2_signed(float x, float d, float y) { return with_sign(mk2_core(x, d, y), x); }
 
 // Range test of a group of numerators (the tiers below).  Float, in three
 // instructions per value, the same predicate as mk_ok on every lane: the
