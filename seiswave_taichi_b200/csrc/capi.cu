@@ -693,16 +693,12 @@ cudaError_t resident_run_t(sw_plan* pl, const sw::P2<T>& p, int it0, int nsteps,
   return sw::sw2r_run<T>(r, pl->scheme, pl->order, it0, nsteps, pl->aea ? 1 : 0, st);
 }
 
-// *done = false when the launches of the other path have to run instead: the
-// scratch could not be allocated, or not yet and the stream is being captured
+// *done = false when the graph of the other path has to run instead: the
+// scratch could not be allocated, or the stream is being captured (a run that
+// replays a graph is refused there, and stays refused)
 cudaError_t resident_run(sw_plan* pl, int it0, int nsteps, cudaStream_t st, bool* done) {
   *done = false;
   if (!pl->d_inbox || !pl->d_err) {
-    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) {
-      cudaGetLastError();
-      return cudaSuccess;
-    }
     if (!pl->d_err) {
       if (cudaMalloc(&pl->d_err, sizeof(int)) != cudaSuccess) { cudaGetLastError(); return cudaSuccess; }
       cudaError_t e = cudaMemset(pl->d_err, 0, sizeof(int));
@@ -825,6 +821,11 @@ int sw3d_plan_create(const sw3d_desc* d, sw_plan** out) {
   bool in_kernel = true;
   if (s.kind != SW_SRC_NONE) {
     if (s.i < 0 || s.i >= d->nx || s.j < 0 || s.j >= d->ny || s.k < 0 || s.k >= d->nz)
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) {
+    cudaGetLastError();
+    return cudaSuccess;
+  }
       return fail(SW_ERR_ARG, "source cell outside the grid");
     if (!s.wavelet) return fail(SW_ERR_ARG, "source wavelet missing");
     if (d->scheme == SW3D_CPML_TENSOR && s.kind != SW_SRC_MOMENT)

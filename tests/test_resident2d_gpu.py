@@ -5,8 +5,8 @@ trace, bit for bit.  The cases sit at the edges of its tiling: the smallest
 grids, one tile and many, widths around 32 and 64 columns, short and long
 sides, slabs wider than a tile and no slabs, sources and receivers in corners
 and rims, more receivers in a tile than its table holds, densities outside the
-corrected quotient's range, the free-surface hook, runs in pieces and runs
-captured in a graph."""
+corrected quotient's range, the free-surface hook, runs in pieces, and a run
+without its own graph captured by the caller."""
 import numpy as np
 import pytest
 import torch
@@ -100,12 +100,12 @@ def test_captured_run(cuda):
     c = case2d(shape=(100, 90), nt=30, nrec=5, MT="explosive", src_scale=1e5)
     ref = _both(c, "VS", 30)
     w = product2d(c)
-    w.run(30)  # the first run allocates the plan's scratch
+    w.run(30)
     torch.cuda.synchronize()
     g = torch.cuda.CUDAGraph()
     with torch.cuda.graph(g):
         w.reset()
-        w.run(30)
+        w.run(30, use_graph=False)
     for _ in range(2):
         g.replay()
     torch.cuda.synchronize()
