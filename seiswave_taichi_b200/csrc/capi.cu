@@ -143,7 +143,7 @@ struct sw_plan {
   sw::FusedMaps fmaps{};
   sw::FusedExtra fx{};
   void* fused_buf = nullptr;
-  int* d_err = nullptr;
+  int* d_err = nullptr;  // error word, then the staged passes' two unit counters
   // TMA-staged two-pass path (3D float CPML schemes)
   bool staged = false;
   sw::StagedMaps svm{}, ssm{};
@@ -502,8 +502,8 @@ void setup_fused(sw_plan* pl) {
   float* buf = nullptr;
   if (cudaMalloc(&buf, total * sizeof(float)) != cudaSuccess) { cudaGetLastError(); return; }
   if (!pl->d_err) {
-    if (cudaMalloc(&pl->d_err, sizeof(int)) != cudaSuccess) { cudaFree(buf); cudaGetLastError(); return; }
-    cudaMemset(pl->d_err, 0, sizeof(int));
+    if (cudaMalloc(&pl->d_err, 3 * sizeof(int)) != cudaSuccess) { cudaFree(buf); cudaGetLastError(); return; }
+    cudaMemset(pl->d_err, 0, 3 * sizeof(int));
   }
   cudaMemset(buf, 0, total * sizeof(float));
   auto& x = pl->fx;
@@ -531,6 +531,36 @@ int units_grid(int units, int per_sm) {
   return units < cap ? units : cap;
 }
 
+// Planes per work unit of the staged passes.  A unit costs its planes plus
+// about N/4 planes of pipeline fill; CTAs take units from a counter, so a pass
+// ends about one slab unit (1.7 times a plain one) after the average CTA --
+// or, when every CTA has at most one unit, with the slowest unit.  Measured
+// with order 2 (us per step, planes per unit): 60 x 60 x 64 34 with 2, 53
+// with 4, 74 with 6 (the rule's earlier minimum); 100^3 114, 134, 176, and 145
+// with 8; 200^3 436, 413, 411, 421, 443 with 12; 400 x 400 x 200 1560, 1433,
+// 1409, 1396, 1402, and 1547 with 34 (1802 with 34 planes dealt out in turn).
+int staged_chunk_rule(const sw_plan* pl, int tiles) {
+  const auto& p = pl->p3f;
+  int gv = 0, gs = 0;
+  if (sw::sw3_staged_grid(pl->staged_N, pl->staged_tz, pl->scheme == SW3D_SPML, pl->scheme == SW3D_CPML_TENSOR,
+                          pl->sa.exact != 0, 1 << 30, &gv, &gs) != cudaSuccess) {
+    cudaGetLastError();
+    return 8;
+  }
+  const double slots = std::min(gv, gs);
+  int best = 8;
+  double cost = 1e300;
+  for (int len = 2; len <= 64; ++len) {
+    const double w = (double)tiles * ((p.nx + len - 1) / len) / slots, unit = len + 0.25 * pl->staged_N;
+    const double c = (w <= 1 ? 0 : w * unit) + 1.7 * unit;
+    if (c < cost) {
+      cost = c;
+      best = len;
+    }
+  }
+  return best;
+}
+
 void staged_chunks(sw_plan* pl, int len) {
   const auto& p = pl->p3f;
   sw::StagedConfig sc;
@@ -538,15 +568,8 @@ void staged_chunks(sw_plan* pl, int len) {
   auto& a = pl->sa;
   a.tiles_y = (p.ny + sc.TY - 1) / sc.TY;
   a.tiles_z = (p.nz + sc.TZ - 1) / sc.TZ;
-  if (len <= 0) {
-    // about five work units per resident CTA
-    int dev = 0, sms = 148;
-    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const int tiles = a.tiles_y * a.tiles_z;
-    int chunks = (10 * sms + tiles - 1) / tiles;
-    len = (p.nx + chunks - 1) / chunks;
-  }
-  if (len < 2 * pl->staged_N + 2) len = 2 * pl->staged_N + 2;
+  if (len <= 0) len = staged_chunk_rule(pl, a.tiles_y * a.tiles_z);
+  if (len < 2) len = 2;
   a.chunk_len = len;
   a.chunks = (p.nx + len - 1) / len;
 }
@@ -574,13 +597,14 @@ void setup_staged(sw_plan* pl) {
   cudaDeviceGetAttribute(&maxsm, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
   if ((size_t)maxsm < sc.vel_smem || (size_t)maxsm < sc.str_smem) return;
   if (!pl->d_err) {
-    if (cudaMalloc(&pl->d_err, sizeof(int)) != cudaSuccess) { cudaGetLastError(); return; }
-    cudaMemset(pl->d_err, 0, sizeof(int));
+    if (cudaMalloc(&pl->d_err, 3 * sizeof(int)) != cudaSuccess) { cudaGetLastError(); return; }
+    cudaMemset(pl->d_err, 0, 3 * sizeof(int));
   }
   if (!sw::sw3_staged_maps(pl->order, tz, p, &pl->svm, &pl->ssm)) return;
   pl->staged_N = pl->order;
   pl->staged_tz = tz;
   pl->sa.err = pl->d_err;
+  pl->sa.next = pl->d_err + 1;
   pl->sa.exact = 1;
   staged_chunks(pl, 0);
   pl->staged = true;
@@ -620,9 +644,9 @@ cudaError_t persistent_run2(sw_plan* pl, int it0, int nsteps, cudaStream_t st) {
     if (e != cudaSuccess) return e;
   }
   if (!pl->d_err) {
-    cudaError_t e = cudaMalloc(&pl->d_err, sizeof(int));
+    cudaError_t e = cudaMalloc(&pl->d_err, 3 * sizeof(int));
     if (e != cudaSuccess) return e;
-    e = cudaMemset(pl->d_err, 0, sizeof(int));
+    e = cudaMemset(pl->d_err, 0, 3 * sizeof(int));
     if (e != cudaSuccess) return e;
   }
   if (pl->dtype == SW_F32)
@@ -698,10 +722,15 @@ cudaError_t resident_run_t(sw_plan* pl, const sw::P2<T>& p, int it0, int nsteps,
 // replays a graph is refused there, and stays refused)
 cudaError_t resident_run(sw_plan* pl, int it0, int nsteps, cudaStream_t st, bool* done) {
   *done = false;
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) {
+    cudaGetLastError();
+    return cudaSuccess;
+  }
   if (!pl->d_inbox || !pl->d_err) {
     if (!pl->d_err) {
-      if (cudaMalloc(&pl->d_err, sizeof(int)) != cudaSuccess) { cudaGetLastError(); return cudaSuccess; }
-      cudaError_t e = cudaMemset(pl->d_err, 0, sizeof(int));
+      if (cudaMalloc(&pl->d_err, 3 * sizeof(int)) != cudaSuccess) { cudaGetLastError(); return cudaSuccess; }
+      cudaError_t e = cudaMemset(pl->d_err, 0, 3 * sizeof(int));
       if (e != cudaSuccess) return e;
     }
     const size_t words = 2 * (size_t)pl->res_tx * pl->res_tz * pl->res_words;
@@ -821,11 +850,6 @@ int sw3d_plan_create(const sw3d_desc* d, sw_plan** out) {
   bool in_kernel = true;
   if (s.kind != SW_SRC_NONE) {
     if (s.i < 0 || s.i >= d->nx || s.j < 0 || s.j >= d->ny || s.k < 0 || s.k >= d->nz)
-  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) {
-    cudaGetLastError();
-    return cudaSuccess;
-  }
       return fail(SW_ERR_ARG, "source cell outside the grid");
     if (!s.wavelet) return fail(SW_ERR_ARG, "source wavelet missing");
     if (d->scheme == SW3D_CPML_TENSOR && s.kind != SW_SRC_MOMENT)

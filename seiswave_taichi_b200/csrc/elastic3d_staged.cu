@@ -735,6 +735,20 @@ __device__ __forceinline__ void spml_stress(const P3<float>& p, int i, int j, in
   }
 }
 
+// Work unit number u: x chunks of a tile first, then the tiles along z and y,
+// so that units in flight together share their halos in L2 (slab tiles first
+// measured 5% slower).  A CTA takes its next unit from the pass's counter
+// (thread 0, at the start of the current unit): with units dealt out in turn
+// the CTAs that drew slab tiles finished last while the others idled (400 x
+// 400 x 200: 1454-1802 us per step over the chunk lengths, 1394-1434 with the
+// counter; 200^3 425-541, 411-446).
+__device__ __forceinline__ void unit_at(const StagedArgs& a, int u, int* tyi, int* tzi, int* ch) {
+  const int t = u / a.chunks;
+  *ch = u - t * a.chunks;
+  *tyi = t / a.tiles_z;
+  *tzi = t - *tyi * a.tiles_z;
+}
+
 // ---------------------------------------------------------------------------
 // velocity pass
 // ---------------------------------------------------------------------------
@@ -785,15 +799,20 @@ k3s_velocity(const __grid_constant__ P3<float> p, const __grid_constant__ Staged
   const int o_yz = (r + N) * G::WZ + G::H4 + Q * cq;   // syz box
 
   const int units = a.tiles_y * a.tiles_z * a.chunks;
+  __shared__ int next_u[2];
+  if (blockIdx.x == 0 && tid == 0) a.next[1] = 0;  // the other pass's counter
   uint32_t g = 0;
   bool ok = true;
-  for (int u = blockIdx.x; u < units && ok; u += gridDim.x) {
-    const int ch = u % a.chunks;
-    const int tzi = (u / a.chunks) % a.tiles_z;
-    const int tyi = u / (a.chunks * a.tiles_z);
+  for (int u = blockIdx.x, turn = 0; u < units && ok; u = next_u[turn], turn ^= 1) {
+    if (tid == 0) next_u[turn] = gridDim.x + atomicAdd(a.next + 0, 1);
+    int tyi, tzi, ch;
+    unit_at(a, u, &tyi, &tzi, &ch);
     const int j0 = tyi * TY, k0 = tzi * G::TZ;
     const int x0 = max(ch * a.chunk_len, N), x1 = min(min((ch + 1) * a.chunk_len, nx - N), nx);
-    if (x0 >= x1) continue;
+    if (x0 >= x1) {
+      __syncthreads();
+      continue;
+    }
     if (SCH == SCH_CPML) fill_tables<TY, G::TZ, G::NT>(p, tyt, tzt, j0, k0, tid);
     const int j = j0 + r, k = k0 + Q * cq;
     const bool jin = j < ny, kin = k < nz;
@@ -1052,15 +1071,20 @@ k3s_stress(const __grid_constant__ P3<float> p, const __grid_constant__ StagedMa
   const int o_m = r * G::WM + Q * cq;
 
   const int units = a.tiles_y * a.tiles_z * a.chunks;
+  __shared__ int next_u[2];
+  if (blockIdx.x == 0 && tid == 0) a.next[0] = 0;  // the other pass's counter
   uint32_t g = 0;
   bool ok = true;
-  for (int u = blockIdx.x; u < units && ok; u += gridDim.x) {
-    const int ch = u % a.chunks;
-    const int tzi = (u / a.chunks) % a.tiles_z;
-    const int tyi = u / (a.chunks * a.tiles_z);
+  for (int u = blockIdx.x, turn = 0; u < units && ok; u = next_u[turn], turn ^= 1) {
+    if (tid == 0) next_u[turn] = gridDim.x + atomicAdd(a.next + 1, 1);
+    int tyi, tzi, ch;
+    unit_at(a, u, &tyi, &tzi, &ch);
     const int j0 = tyi * TY, k0 = tzi * G::TZ;
     const int x0 = max(ch * a.chunk_len, N), x1 = min((ch + 1) * a.chunk_len, nx - N);
-    if (x0 >= x1) continue;
+    if (x0 >= x1) {
+      __syncthreads();
+      continue;
+    }
     if (SCH == SCH_CPML) fill_tables<TY, G::TZ, G::NT>(p, tyt, tzt, j0, k0, tid);
     const int j = j0 + r, k = k0 + Q * cq;
     const bool jin = j < ny, kin = k < nz;

@@ -15,7 +15,8 @@ struct StagedMaps {
 };
 
 struct StagedArgs {
-  int* err;  // error word: bit0 = a TMA wait gave up
+  int* err;   // error word: bit0 = a TMA wait gave up
+  int* next;  // unit counters of the velocity and the stress pass; each pass zeroes the other's
   int tiles_y, tiles_z, chunks, chunk_len;
   int exact;  // 1: IEEE-exact reference order (bit-identical to the CPU oracle)
 };
