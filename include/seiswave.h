@@ -198,7 +198,9 @@ SW_API int sw_plan_status(sw_plan* plan, void* stream);
  * make two launches per step, sw_run with one keeps runs of at least 4 steps of
  * orders up to 4 that record a velocity on the chip where their tiles fit --
  * one cooperative launch, neighbouring tiles exchange their rims -- and
- * replays the launches otherwise; 1 TMA-staged
+ * replays the launches otherwise; 3D float: a run of at least 6 steps whose
+ * rows are no multiple of 16 bytes steps pitched copies of the state with the
+ * kernels of path 1 and copies them back; 1 TMA-staged
  * two-pass kernels, 2 fused single-pass kernel, 3 2D persistent: sw_run is
  * one cooperative launch for all its steps, the phases separated by a
  * bounded grid barrier; opt-in, as path 0 is faster on B200 at every grid

@@ -121,6 +121,10 @@ __global__ void k_count_nonfinite(const T* a, long long n, unsigned long long* o
 
 }  // namespace
 
+// fewest steps of a run that pay for the pitched copies' way in and out
+// (about as much traffic as 1.2 steps)
+#define SW_PITCH_STEPS 6
+
 struct sw_plan {
   int dim = 0, scheme = 0, dtype = 0, order = 0, nt_max = 0;
   sw::P2<float> p2f{};
@@ -136,6 +140,7 @@ struct sw_plan {
   cudaStream_t cap_stream = nullptr;
   cudaGraphExec_t gexec = nullptr;
   int g_it0 = -1, g_n = -1;
+  bool g_pitched = false;
   unsigned long long* d_count = nullptr;
   // fused single-pass path (3D float CPML schemes)
   bool fused = false;
@@ -149,6 +154,13 @@ struct sw_plan {
   sw::StagedMaps svm{}, ssm{};
   sw::StagedArgs sa{};
   int staged_N = 0, staged_tz = 32;
+  // staged runs of grids whose rows are no multiple of 16 bytes: pitched
+  // copies of the state (allocated by the first run), stepped by the staged
+  // kernels and copied back
+  bool pitch_ok = false;
+  float* pitch_buf = nullptr;
+  sw::P3<float> pp{};
+  sw::StagedMaps pvm{}, psm{};
   // 0: register-queue two-pass kernels (2D: two launches per step), 1: staged
   // two-pass, 2: fused single pass, 3: 2D persistent (one cooperative launch
   // per run)
@@ -285,7 +297,7 @@ void set_divisors(T* rd, int* fast, const double* h, int n) {
 
 template <typename T>
 int make_p3(sw_plan* pl, const sw3d_desc* d, sw::P3<T>& p) {
-  p.nx = d->nx; p.ny = d->ny; p.nz = d->nz;
+  p.nx = d->nx; p.ny = d->ny; p.nz = p.pz = d->nz;
   p.dx = (T)d->dx; p.dy = (T)d->dy; p.dz = (T)d->dz; p.dt = (T)d->dt;
   for (int m = 0; m < SW_MAX_ORDER; ++m) p.c[m] = (T)d->coef[m];
   for (int q = 0; q < 9; ++q) p.f[q] = (T*)d->field[q];
@@ -584,31 +596,123 @@ void setup_staged(sw_plan* pl) {
   // needs the per-cell split-PML kernels
   if (pl->scheme == SW3D_SPML && pl->src_kind != SW_SRC_NONE && (p.si < pl->order || p.si >= p.nx - pl->order))
     return;
-  if (p.nz % 4 != 0) return;
   // z tile width: the one leaving fewer idle cells in the last tile (32 on ties)
   const int tz = (p.nz + 39) / 40 * 40 < (p.nz + 31) / 32 * 32 ? 40 : 32;
   sw::StagedConfig sc;
   if (!sw::sw3_staged_config(pl->order, tz, &sc)) return;
-  for (int q = 0; q < 9; ++q)
-    if (!aligned(p.f[q], 16)) return;
-  if (!aligned(p.rho, 16) || !aligned(p.lam, 16) || !aligned(p.mu, 16)) return;
   int dev = 0, maxsm = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&maxsm, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
   if ((size_t)maxsm < sc.vel_smem || (size_t)maxsm < sc.str_smem) return;
+  bool direct = p.nz % 4 == 0;
+  for (int q = 0; q < 9; ++q) direct = direct && aligned(p.f[q], 16);
+  direct = direct && aligned(p.rho, 16) && aligned(p.lam, 16) && aligned(p.mu, 16);
+  // Split PML of orders 3 and 4 on small grids: their staged tiles leave one CTA
+  // per SM, and the per-cell kernels are faster below about two million cells
+  // (us per step, staged / per cell: order 3 100^3 242 / 216, 140^3 354 / 533;
+  // order 4 60 x 60 x 64 68 / 41, 100^3 247 / 169, 140^3 491 / 502, 200^3
+  // 1229 / 1342)
+  const bool worth = pl->scheme != SW3D_SPML || pl->order <= 2 || (long long)p.nx * p.ny * p.nz >= 2000000LL;
+  // Rows that are no multiple of 16 bytes: a run steps pitched copies (us per
+  // step, the caller's rows with the two-pass kernels -> pitched: 60 x 61 x 62
+  // 68 -> 35, 153 x 131 x 117 order 3 462 -> 302, 200 x 190 x 201 1320 -> 422)
+  pl->pitch_ok = p.nz % 4 != 0 && pl->gather_in_stress && worth;
+  if (!direct && !pl->pitch_ok) return;
   if (!pl->d_err) {
-    if (cudaMalloc(&pl->d_err, 3 * sizeof(int)) != cudaSuccess) { cudaGetLastError(); return; }
+    if (cudaMalloc(&pl->d_err, 3 * sizeof(int)) != cudaSuccess) {
+      cudaGetLastError();
+      pl->pitch_ok = false;
+      return;
+    }
     cudaMemset(pl->d_err, 0, 3 * sizeof(int));
   }
-  if (!sw::sw3_staged_maps(pl->order, tz, p, &pl->svm, &pl->ssm)) return;
+  if (direct && !sw::sw3_staged_maps(pl->order, tz, p, &pl->svm, &pl->ssm)) return;
   pl->staged_N = pl->order;
   pl->staged_tz = tz;
   pl->sa.err = pl->d_err;
   pl->sa.next = pl->d_err + 1;
   pl->sa.exact = 1;
   staged_chunks(pl, 0);
+  if (!direct) return;
   pl->staged = true;
-  pl->path = 1;
+  if (worth) pl->path = 1;
+}
+
+// The pitched copies of a plan: true when they exist.  They are allocated by
+// the first run that wants them; without memory, or while the stream is being
+// captured, the two-pass kernels run instead.
+bool pitch_ready(sw_plan* pl, int nsteps, cudaStream_t st) {
+  if (pl->dim != 3 || !pl->pitch_ok || pl->path != 0 || pl->aea || nsteps < SW_PITCH_STEPS) return false;
+  if (pl->pitch_buf) return true;
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) {
+    cudaGetLastError();
+    return false;
+  }
+  const auto& p = pl->p3f;
+  const int pz = (p.nz + 3) / 4 * 4;
+  const size_t cells = (size_t)p.nx * p.ny * pz;
+  const size_t m0 = (size_t)p.sn[0] * p.ny * pz, m1 = (size_t)p.nx * p.sn[1] * pz;
+  const bool mem = pl->scheme != SW3D_SPML;
+  const size_t total = 12 * cells + (mem ? 6 * (m0 + m1) : 0);
+  float* b = nullptr;
+  if (cudaMalloc(&b, total * sizeof(float)) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  sw::P3<float> q = p;
+  q.pz = pz;
+  float* cur = b;
+  for (int f = 0; f < 9; ++f, cur += cells) q.f[f] = cur;
+  q.rho = cur, cur += cells;
+  q.lam = cur, cur += cells;
+  q.mu = cur, cur += cells;
+  if (mem) {
+    q.mem[0] = cur, cur += 6 * m0;
+    q.mem[1] = cur;
+    q.mcomp[0] = (long long)m0;
+    q.mcomp[1] = (long long)m1;
+  }
+  if (!sw::sw3_staged_maps(pl->staged_N, pl->staged_tz, q, &pl->pvm, &pl->psm)) {
+    cudaFree(b);
+    pl->pitch_ok = false;
+    return false;
+  }
+  pl->pp = q;
+  pl->pitch_buf = b;
+  return true;
+}
+
+cudaError_t enqueue_pitched_run(sw_plan* pl, int it0, int nsteps, cudaStream_t st) {
+  const auto& p = pl->p3f;
+  const auto& q = pl->pp;
+  const bool spml = pl->scheme == SW3D_SPML, tensor = pl->scheme == SW3D_CPML_TENSOR;
+  const bool moment = pl->src_kind == SW_SRC_MOMENT, force = pl->src_kind == SW_SRC_FORCE;
+  cudaError_t e = cudaSuccess;
+  if (moment) e = sw::sw3_moment_inject<float>(p, it0, st);
+  const long long rows = (long long)p.nx * p.ny;
+  auto in = [&](const float* a, const float* b, long long n) {
+    if (e == cudaSuccess) e = sw::sw3_pitch_rows(a, const_cast<float*>(b), n, p.nz, p.nz, q.pz, st);
+  };
+  auto out = [&](const float* a, float* b, long long n) {
+    if (e == cudaSuccess) e = sw::sw3_pitch_rows(a, b, n, p.nz, q.pz, p.nz, st);
+  };
+  for (int f = 0; f < 9; ++f) in(p.f[f], q.f[f], rows);
+  in(p.rho, q.rho, rows);
+  in(p.lam, q.lam, rows);
+  in(p.mu, q.mu, rows);
+  const long long r0 = spml ? 0 : 6LL * p.sn[0] * p.ny, r1 = spml ? 0 : 6LL * p.nx * p.sn[1];
+  in(p.mem[0], q.mem[0], r0);
+  in(p.mem[1], q.mem[1], r1);
+  sw::StagedArgs a = pl->sa;
+  a.exact = 1;  // path 0 is always exact
+  for (int s = 0; s < nsteps && e == cudaSuccess; ++s)
+    e = sw::sw3_staged_step(pl->staged_N, pl->staged_tz, spml, tensor, q, pl->pvm, pl->psm, a, it0 + s, force,
+                            moment && s != nsteps - 1, true, st);
+  for (int f = 0; f < 9; ++f) out(q.f[f], p.f[f], rows);
+  out(q.mem[0], p.mem[0], r0);
+  out(q.mem[1], p.mem[1], r1);
+  return e;
 }
 
 // nsteps >= 2 steps through the fused kernel (the last one two-pass when odd)
@@ -746,6 +850,8 @@ cudaError_t resident_run(sw_plan* pl, int it0, int nsteps, cudaStream_t st, bool
 
 cudaError_t enqueue_sequence(sw_plan* pl, int it0, int nsteps, cudaStream_t st) {
   if (pl->fused && pl->path == 2 && nsteps >= 2 && !pl->aea) return enqueue_fused_run(pl, it0, nsteps, st);
+  if (pl->pitch_buf && pl->path == 0 && !pl->aea && nsteps >= SW_PITCH_STEPS)
+    return enqueue_pitched_run(pl, it0, nsteps, st);
   for (int s = 0; s < nsteps; ++s) {
     cudaError_t e = enqueue_step(pl, it0 + s, s == 0, s == nsteps - 1, false, 0.0, st);
     if (e != cudaSuccess) return e;
@@ -1000,6 +1106,7 @@ int sw_plan_destroy(sw_plan* pl) {
   if (pl->d_err) cudaFree(pl->d_err);
   if (pl->d_bar) cudaFree(pl->d_bar);
   if (pl->d_inbox) cudaFree(pl->d_inbox);
+  if (pl->pitch_buf) cudaFree(pl->pitch_buf);
   delete pl;
   return SW_OK;
 }
@@ -1035,6 +1142,7 @@ int sw_run(sw_plan* pl, int32_t it0, int32_t nsteps, int32_t use_graph, void* st
     if (e != cudaSuccess) return cuda_fail(e, "sw_run: persistent launch");
     return SW_OK;
   }
+  const bool pitched = pitch_ready(pl, nsteps, st);
   if (!use_graph) {
     e = enqueue_sequence(pl, it0, nsteps, st);
     if (e != cudaSuccess) return cuda_fail(e, "sw_run");
@@ -1046,7 +1154,7 @@ int sw_run(sw_plan* pl, int32_t it0, int32_t nsteps, int32_t use_graph, void* st
     if (e != cudaSuccess) return cuda_fail(e, "sw_run: on-chip loop");
     if (done) return SW_OK;
   }
-  if (!(pl->gexec && pl->g_it0 == it0 && pl->g_n == nsteps)) {
+  if (!(pl->gexec && pl->g_it0 == it0 && pl->g_n == nsteps && pl->g_pitched == pitched)) {
     if (pl->gexec) { cudaGraphExecDestroy(pl->gexec); pl->gexec = nullptr; }
     if (!pl->cap_stream) {
       e = cudaStreamCreateWithFlags(&pl->cap_stream, cudaStreamNonBlocking);
@@ -1064,6 +1172,7 @@ int sw_run(sw_plan* pl, int32_t it0, int32_t nsteps, int32_t use_graph, void* st
     if (e != cudaSuccess) { pl->gexec = nullptr; return cuda_fail(e, "sw_run: instantiate"); }
     pl->g_it0 = it0;
     pl->g_n = nsteps;
+    pl->g_pitched = pitched;
   }
   e = cudaGraphLaunch(pl->gexec, st);
   if (e != cudaSuccess) return cuda_fail(e, "sw_run: graph launch");

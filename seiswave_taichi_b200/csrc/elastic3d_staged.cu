@@ -356,11 +356,11 @@ __device__ __forceinline__ void prefetch_memvars(const P3<float>& p, int i, int 
                                                  const int (&zk)[Q], bool zany) {
   const int xn = slab_index(i, p.nx, p.lo[0], p.hi[0]);
   if (xn >= 0) {
-    const float* b = p.mem[0] + c0 * p.mcomp[0] + ((size_t)xn * p.ny + j) * p.nz + k;
+    const float* b = p.mem[0] + c0 * p.mcomp[0] + ((size_t)xn * p.ny + j) * p.pz + k;
     for (int c = 0; c < 3; ++c) prefetch_l2(b + c * p.mcomp[0]);
   }
   if (yj >= 0) {
-    const float* b = p.mem[1] + c0 * p.mcomp[1] + ((size_t)i * p.sn[1] + yj) * p.nz + k;
+    const float* b = p.mem[1] + c0 * p.mcomp[1] + ((size_t)i * p.sn[1] + yj) * p.pz + k;
     for (int c = 0; c < 3; ++c) prefetch_l2(b + c * p.mcomp[1]);
   }
   if (zany) {
@@ -384,6 +384,11 @@ __device__ __forceinline__ void prefetch_split(const P3<float>& p, int i, int j,
     const float* b = p.split + c0 * p.scomp + shell_index(p, i, j, k + e);
     for (int c = 0; c < nc; ++c) prefetch_l1(b + c * p.scomp);
   }
+}
+
+// a receiver's linear cell index in the pitched fields
+__device__ __forceinline__ long long pitched(const P3<float>& p, long long g) {
+  return p.pz == p.nz ? g : g / p.nz * p.pz + g % p.nz;
 }
 
 // per-unit CPML table of the tile's rows (y) or z cells: row q of the axis
@@ -548,7 +553,7 @@ template <int Q>
 __device__ __forceinline__ SplitAt<Q> split_at(const P3<float>& p, int i, int j, int k, uint8_t fxy,
                                                const uint8_t (&fz)[Q]) {
   SplitAt<Q> at;
-  const bool in0 = fxy | fz[0], in1 = fxy | fz[Q - 1];
+  const bool in0 = fxy | fz[0], in1 = k + Q - 1 < p.nz && (fxy | fz[Q - 1]);
   const long long s0 = in0 ? shell_index(p, i, j, k) : 0;
   const long long s1 = in1 ? shell_index(p, i, j, k + Q - 1) : 0;
   const long long base = in0 ? s0 : s1;
@@ -763,7 +768,7 @@ k3s_velocity(const __grid_constant__ P3<float> p, const __grid_constant__ Staged
   float* tzt = tyt + 6 * TY;    // [6][TZ]
   const int tid = threadIdx.x;
   const int nx = p.nx, ny = p.ny, nz = p.nz;
-  const size_t nyz = (size_t)ny * nz;
+  const size_t pz = p.pz, nyz = (size_t)ny * pz;  // pz: the fields' row pitch
   if (tid == 0) {
     for (int b = 0; b <= D; ++b) mbar_init(&bars[b], 1);
     mbar_fence_init();
@@ -896,7 +901,7 @@ k3s_velocity(const __grid_constant__ P3<float> p, const __grid_constant__ Staged
         }
         const float* r0 = rho_p(i);
         const float* r1 = rho_p(i + 1);
-        const size_t gi = (size_t)i * nyz + (size_t)j * nz + k;
+        const size_t gi = (size_t)i * nyz + (size_t)j * pz + k;
         // derivatives of the three components (Dx3fm/Dy3bm/Dz3bm etc.)
         Vq<Q> dv[9] = {dxq<N, EX, Q>(pxx, o_xx, cx),
                         dyq<N, false, EX, Q>(sxy_p(i), o_y, G::TZ, cy),
@@ -943,7 +948,7 @@ k3s_velocity(const __grid_constant__ P3<float> p, const __grid_constant__ Staged
             const float bi = __ldg(cf + CB * nx + i), ai = __ldg(cf + CA * nx + i), ki = __ldg(cf + CK * nx + i);
             const float bh = __ldg(cf + CBH * nx + i), ah = __ldg(cf + CAH * nx + i),
                         kh = __ldg(cf + CKH * nx + i);
-            float* m0 = p.mem[0] + ((size_t)xi * ny + j) * nz + k;
+            float* m0 = p.mem[0] + ((size_t)xi * ny + j) * pz + k;
             const long long mc = p.mcomp[0];
             Vq<Q> s0 = ldq<Q>(m0), s1 = ldq<Q>(m0 + mc), s2 = ldq<Q>(m0 + 2 * mc);
             cpml_pair<EX, Q>(a1, s0, mx, bh, ah, kh);
@@ -956,7 +961,7 @@ k3s_velocity(const __grid_constant__ P3<float> p, const __grid_constant__ Staged
           if (yj >= 0) {
             const float bi = tab(tyt, CB, TY, r), ai = tab(tyt, CA, TY, r), ki = tab(tyt, CK, TY, r);
             const float bh = tab(tyt, CBH, TY, r), ah = tab(tyt, CAH, TY, r), kh = tab(tyt, CKH, TY, r);
-            float* m1 = p.mem[1] + ((size_t)i * p.sn[1] + yj) * nz + k;
+            float* m1 = p.mem[1] + ((size_t)i * p.sn[1] + yj) * pz + k;
             const long long mc = p.mcomp[1];
             Vq<Q> s0 = ldq<Q>(m1), s1 = ldq<Q>(m1 + mc), s2 = ldq<Q>(m1 + 2 * mc);
             cpml_pair<EX, Q>(a2, s0, mx, bi, ai, ki);
@@ -1035,11 +1040,11 @@ k3s_stress(const __grid_constant__ P3<float> p, const __grid_constant__ StagedMa
   float* tzt = tyt + 6 * TY;    // [6][TZ]
   const int tid = threadIdx.x;
   const int nx = p.nx, ny = p.ny, nz = p.nz;
-  const size_t nyz = (size_t)ny * nz;
+  const size_t pz = p.pz, nyz = (size_t)ny * pz;  // pz: the fields' row pitch
   // receivers: the velocities are final for this step and not written here
   if (gather && p.nrec > 0)
     for (int rr = blockIdx.x * G::NT + tid; rr < p.nrec; rr += gridDim.x * G::NT)
-      store_rec(p.rec_data, p.rec_f64, (long long)it * p.nrec + rr, p.f[p.rec_field][p.rec_idx[rr]]);
+      store_rec(p.rec_data, p.rec_f64, (long long)it * p.nrec + rr, p.f[p.rec_field][pitched(p, p.rec_idx[rr])]);
   if (tid == 0) {
     for (int b = 0; b <= D; ++b) mbar_init(&bars[b], 1);
     mbar_fence_init();
@@ -1170,7 +1175,7 @@ k3s_stress(const __grid_constant__ P3<float> p, const __grid_constant__ StagedMa
         const float* vxi = vx_p(i);
         const float* vyi = vy_p(i);
         const float* vzi = vz_p(i);
-        const size_t gi = (size_t)i * nyz + (size_t)j * nz + k;
+        const size_t gi = (size_t)i * nyz + (size_t)j * pz + k;
         // derivatives: dvx/dx dvy/dy dvz/dz dvy/dx dvx/dy dvz/dx dvx/dz dvz/dy dvy/dz
         Vq<Q> dv[9] = {dxq<N, EX, Q>(pvx, o_v, cx),
                         dyq<N, false, EX, Q>(vyi, o_v, G::WZ, cy),
@@ -1226,7 +1231,7 @@ k3s_stress(const __grid_constant__ P3<float> p, const __grid_constant__ StagedMa
             const float bh = __ldg(cf + CBH * nx + i), ah = __ldg(cf + CAH * nx + i),
                         khx = __ldg(cf + CKH * nx + i);
             const long long mc = p.mcomp[0];
-            float* m0 = p.mem[0] + 3 * mc + ((size_t)xi * ny + j) * nz + k;
+            float* m0 = p.mem[0] + 3 * mc + ((size_t)xi * ny + j) * pz + k;
             Vq<Q> s0 = ldq<Q>(m0), s1 = ldq<Q>(m0 + mc), s2 = ldq<Q>(m0 + 2 * mc);
             cpml_pair<EX, Q>(e1, s0, mn, bi, ai, ki);    // dvx_dx
             cpml_pair<EX, Q>(f1, s1, mxy, bh, ah, khx);  // dvy_dx
@@ -1239,7 +1244,7 @@ k3s_stress(const __grid_constant__ P3<float> p, const __grid_constant__ StagedMa
             const float bi = tab(tyt, CB, TY, r), ai = tab(tyt, CA, TY, r), ki = tab(tyt, CK, TY, r);
             const float bh = tab(tyt, CBH, TY, r), ah = tab(tyt, CAH, TY, r), khy = tab(tyt, CKH, TY, r);
             const long long mc = p.mcomp[1];
-            float* m1 = p.mem[1] + 3 * mc + ((size_t)i * p.sn[1] + yj) * nz + k;
+            float* m1 = p.mem[1] + 3 * mc + ((size_t)i * p.sn[1] + yj) * pz + k;
             Vq<Q> s0 = ldq<Q>(m1), s1 = ldq<Q>(m1 + mc), s2 = ldq<Q>(m1 + 2 * mc);
             cpml_pair<EX, Q>(e2, s0, mn, bi, ai, ki);    // dvy_dy
             cpml_pair<EX, Q>(f2, s1, mxy, bh, ah, khy);  // dvx_dy
@@ -1322,11 +1327,11 @@ static PFN_cuTensorMapEncodeTiled_v12000 staged_encoder() {
   return fn;
 }
 
-static bool map3(CUtensorMap* m, const void* base, int nx, int ny, int nz, int bz, int by) {
+static bool map3(CUtensorMap* m, const void* base, int nx, int ny, int nz, int pz, int bz, int by) {
   auto enc = staged_encoder();
   if (!enc) return false;
   cuuint64_t dims[3] = {(cuuint64_t)nz, (cuuint64_t)ny, (cuuint64_t)nx};
-  cuuint64_t strides[2] = {(cuuint64_t)nz * 4, (cuuint64_t)ny * nz * 4};
+  cuuint64_t strides[2] = {(cuuint64_t)pz * 4, (cuuint64_t)ny * pz * 4};
   cuuint32_t box[3] = {(cuuint32_t)bz, (cuuint32_t)by, 1};
   cuuint32_t es[3] = {1, 1, 1};
   return enc(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<void*>(base), dims, strides, box, es,
@@ -1340,21 +1345,21 @@ static bool staged_maps_t(const P3<float>& p, StagedMaps* vm, StagedMaps* sm_) {
   const int nx = p.nx, ny = p.ny, nz = p.nz;
   bool ok = true;
   // velocity pass: sxx sxy sxz syy syz szz rho
-  ok = ok && map3(&vm->m[0], p.f[3], nx, ny, nz, G::TZ, TY);
-  ok = ok && map3(&vm->m[1], p.f[6], nx, ny, nz, G::TZ, G::HY);
-  ok = ok && map3(&vm->m[2], p.f[7], nx, ny, nz, G::WZ, TY);
-  ok = ok && map3(&vm->m[3], p.f[4], nx, ny, nz, G::TZ, G::HY);
-  ok = ok && map3(&vm->m[4], p.f[8], nx, ny, nz, G::WZ, G::HY);
-  ok = ok && map3(&vm->m[5], p.f[5], nx, ny, nz, G::WZ, TY);
-  ok = ok && map3(&vm->m[6], p.rho, nx, ny, nz, G::TZ, TY + 1);
-  for (int c = 0; c < 3; ++c) ok = ok && map3(&vm->m[7 + c], p.f[c], nx, ny, nz, G::TZ, TY);
+  ok = ok && map3(&vm->m[0], p.f[3], nx, ny, nz, p.pz, G::TZ, TY);
+  ok = ok && map3(&vm->m[1], p.f[6], nx, ny, nz, p.pz, G::TZ, G::HY);
+  ok = ok && map3(&vm->m[2], p.f[7], nx, ny, nz, p.pz, G::WZ, TY);
+  ok = ok && map3(&vm->m[3], p.f[4], nx, ny, nz, p.pz, G::TZ, G::HY);
+  ok = ok && map3(&vm->m[4], p.f[8], nx, ny, nz, p.pz, G::WZ, G::HY);
+  ok = ok && map3(&vm->m[5], p.f[5], nx, ny, nz, p.pz, G::WZ, TY);
+  ok = ok && map3(&vm->m[6], p.rho, nx, ny, nz, p.pz, G::TZ, TY + 1);
+  for (int c = 0; c < 3; ++c) ok = ok && map3(&vm->m[7 + c], p.f[c], nx, ny, nz, p.pz, G::TZ, TY);
   // stress pass: vx vy vz lam mu, then the six stresses
-  ok = ok && map3(&sm_->m[0], p.f[0], nx, ny, nz, G::WZ, G::HY);
-  ok = ok && map3(&sm_->m[1], p.f[1], nx, ny, nz, G::WZ, G::HY);
-  ok = ok && map3(&sm_->m[2], p.f[2], nx, ny, nz, G::WZ, G::HY);
-  ok = ok && map3(&sm_->m[3], p.lam, nx, ny, nz, G::TZ, TY);
-  ok = ok && map3(&sm_->m[4], p.mu, nx, ny, nz, G::WM, TY + 1);
-  for (int c = 0; c < 6; ++c) ok = ok && map3(&sm_->m[5 + c], p.f[3 + c], nx, ny, nz, G::TZ, TY);
+  ok = ok && map3(&sm_->m[0], p.f[0], nx, ny, nz, p.pz, G::WZ, G::HY);
+  ok = ok && map3(&sm_->m[1], p.f[1], nx, ny, nz, p.pz, G::WZ, G::HY);
+  ok = ok && map3(&sm_->m[2], p.f[2], nx, ny, nz, p.pz, G::WZ, G::HY);
+  ok = ok && map3(&sm_->m[3], p.lam, nx, ny, nz, p.pz, G::TZ, TY);
+  ok = ok && map3(&sm_->m[4], p.mu, nx, ny, nz, p.pz, G::WM, TY + 1);
+  for (int c = 0; c < 6; ++c) ok = ok && map3(&sm_->m[5 + c], p.f[3 + c], nx, ny, nz, p.pz, G::TZ, TY);
   return ok;
 }
 
@@ -1397,6 +1402,25 @@ bool sw3_staged_maps(int N, int tz, const P3<float>& p, StagedMaps* vm, StagedMa
   SW_STAGED_SWITCH(N, tz, SW_MAPS)
 #undef SW_MAPS
   return false;
+}
+
+// Rows of nz cells between the caller's arrays and copies with a pitch of pz
+// cells, for grids whose rows are no multiple of 16 bytes (TMA strides)
+__global__ void k3_pitch(const float* __restrict__ src, float* __restrict__ dst, long long rows, int nz, int ps,
+                         int pd) {
+  const long long n = rows * pd;
+  for (long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += (long long)gridDim.x * blockDim.x) {
+    const long long r = q / pd;
+    const int k = (int)(q - r * pd);
+    dst[q] = k < nz ? src[r * ps + k] : 0.f;
+  }
+}
+
+cudaError_t sw3_pitch_rows(const float* src, float* dst, long long rows, int nz, int ps, int pd, cudaStream_t st) {
+  if (rows <= 0) return cudaSuccess;
+  const long long blocks = (rows * pd + 255) / 256;
+  k3_pitch<<<(int)(blocks < 4736 ? blocks : 4736), 256, 0, st>>>(src, dst, rows, nz, ps, pd);
+  return cudaGetLastError();
 }
 
 // Resident CTAs per SM of each pass (registers, shared memory and threads

@@ -83,6 +83,8 @@ struct P3 {
   T rd[3];                  // RN(1/dx), RN(1/dy), RN(1/dz)
   int fast_div;             // div_c may use the verified constant-divisor path
   T cs[3][SW_MAX_ORDER];    // c_m / dx, c_m / dy, c_m / dz (fast numeric mode)
+  int pz;                   // row pitch of the fields, materials and x/y memory variables (staged kernels;
+                            // nz except in the plan's pitched copies)
 };
 
 // 2D memory-variable components, 4 per direction, shared by all schemes:
@@ -312,9 +314,9 @@ __device__ __forceinline__ float mk2_div_any(float x, float d, float y) {
   const float xs = __fmul_rn(x, up);
   return with_sign(scaled_finish(xs, mk2_core(xs, d, y), d, up, down), x);
 }
+__device__ __forceinline__ float mk2_signed(float x, float d, float y) { return with_sign(mk2_core(x, d, y), x); }
 template <typename T>
 __device__ __forceinline__ bool mk2_divisor(T d) { return d >= (T)0x1p-20 && d <= (T)0x1p20; }
-__device__ __forceinline__ float mk2_signed(float x, float d, float y) { return with_sign(mk2_core(x, d, y), x); }
 
 // Range test of a group of numerators (the tiers below).  Float, in three
 // instructions per value, the same predicate as mk_ok on every lane: the
