@@ -246,16 +246,15 @@ void fill_axis3(sw::P3<T>& p, int d, const sw_pml_axis& a, int n) {
   (void)n;
 }
 
+// x planes streamed by one CTA of the two-pass kernels: three, or two where
+// three would leave SMs without their four CTAs (double, order 2, us per step
+// with 2, 3, 4, 8 planes: 60 x 60 x 62 58, 72, 89, 144; 90^3 154, 167, 186, 222;
+// 128 x 120 x 112 324, 327, 340, 393; 200^3 1174, 1152, 1143, 1157)
 int choose_x_chunk(int nx, int ny, int nz) {
   int dev = 0, sms = 148;
   if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const long long tiles = (long long)((nz + 31) / 32) * ((ny + 7) / 8);
-  const long long target = (long long)sms * 8;  // ~8 resident-sized CTAs per SM
-  long long chunks = (target + tiles - 1) / tiles;
-  if (chunks < 1) chunks = 1;
-  int xc = (int)((nx + chunks - 1) / chunks);
-  if (xc < 4) xc = 4;
-  return xc;
+  return tiles * ((nx + 2) / 3) < 4LL * 4 * sms ? 2 : 3;
 }
 
 // ---------------------------------------------------------------------------

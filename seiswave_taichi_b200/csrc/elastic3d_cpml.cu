@@ -18,6 +18,13 @@ namespace sw {
 
 constexpr int T3Z = 32;
 constexpr int T3Y = 8;
+// Resident blocks per SM the passes are compiled for.  A thread waits on the
+// tap loads of one component after the other, so residency pays more than
+// registers: double, order 2, 128 x 120 x 112, us per step with the compiler's
+// own count (98-128 registers, two blocks) 448, for 3 blocks 359, 4 327, 5 344,
+// 6 384, 8 467 (spills); order 4 686, 456, 520, 527, 573, 656; 200^3 1492, 1278,
+// 1142, 1202, 1335; float 128 x 120 x 112 294, -, 213, 224, 267.
+constexpr int K3_MINB = 4;
 
 template <typename T>
 __device__ __forceinline__ void pml_apply(T* __restrict__ m, T b, T a, T kk, T& d) {
@@ -26,11 +33,31 @@ __device__ __forceinline__ void pml_apply(T* __restrict__ m, T b, T a, T kk, T& 
   d = div_v(d, kk) + psi;
 }
 
+// quotients of a component's derivatives by the spacings of axes A, B, C as one
+// range-tested group (div_c's bits): at 128 x 120 x 112 in double
+// 444 -> 410 us per step
+template <typename T, int A, int B, int C>
+__device__ __forceinline__ void spacings(const P3<T>& p, T& a, T& b, T& c) {
+  const T h[3] = {p.dx, p.dy, p.dz};
+  T x[3] = {a, b, c};
+  const T d[3] = {h[A], h[B], h[C]}, r[3] = {p.rd[A], p.rd[B], p.rd[C]};
+  divc_group<3>(x, d, r, p.fast_div);
+  a = x[0], b = x[1], c = x[2];
+}
+template <typename T, int A, int B>
+__device__ __forceinline__ void spacings(const P3<T>& p, T& a, T& b) {
+  const T h[3] = {p.dx, p.dy, p.dz};
+  T x[2] = {a, b};
+  const T d[2] = {h[A], h[B]}, r[2] = {p.rd[A], p.rd[B]};
+  divc_group<2>(x, d, r, p.fast_div);
+  a = x[0], b = x[1];
+}
+
 // ---------------------------------------------------------------------------
 // velocity pass
 // ---------------------------------------------------------------------------
 template <typename T, int N, bool TENSOR>
-__global__ void __launch_bounds__(T3Z * T3Y)
+__global__ void __launch_bounds__(T3Z * T3Y, K3_MINB)
 k3_velocity(const __grid_constant__ P3<T> p, int it, int force_here) {
   const int k = blockIdx.x * T3Z + threadIdx.x;
   const int j = blockIdx.y * T3Y + threadIdx.y;
@@ -112,9 +139,7 @@ k3_velocity(const __grid_constant__ P3<T> p, int it, int force_here) {
         const T hi = (m == 0) ? qxz[N] : ldg(sxz + idx + m);
         dsxzdz += c[m] * (hi - ldg(sxz + idx - (m + 1)));
       }
-      dsxxdx = div_c(dsxxdx, dx, p.rd[0], p.fast_div);
-      dsxydy = div_c(dsxydy, dy, p.rd[1], p.fast_div);
-      dsxzdz = div_c(dsxzdz, dz, p.rd[2], p.fast_div);
+      spacings<T, 0, 1, 2>(p, dsxxdx, dsxydy, dsxzdz);
       if ((xi >= 0 || yj >= 0 || zk >= 0) && ((fx & 2) || (fy & 1) || (fz & 1))) {
         if (xi >= 0)
           pml_apply(p.mem[0] + ((long long)xi * ny + j) * nz + k,
@@ -143,9 +168,7 @@ k3_velocity(const __grid_constant__ P3<T> p, int it, int force_here) {
 #pragma unroll
       for (int m = 0; m < N; ++m)
         dsyzdz += c[m] * (ldg(syz + idx + m) - ldg(syz + idx - (m + 1)));
-      dsxydx = div_c(dsxydx, dx, p.rd[0], p.fast_div);
-      dsyydy = div_c(dsyydy, dy, p.rd[1], p.fast_div);
-      dsyzdz = div_c(dsyzdz, dz, p.rd[2], p.fast_div);
+      spacings<T, 0, 1, 2>(p, dsxydx, dsyydy, dsyzdz);
       if ((xi >= 0 || yj >= 0 || zk >= 0) && ((fx & 1) || (fy & 2) || (fz & 1))) {
         if (xi >= 0)
           pml_apply(p.mem[0] + p.mcomp[0] + ((long long)xi * ny + j) * nz + k,
@@ -178,9 +201,7 @@ k3_velocity(const __grid_constant__ P3<T> p, int it, int force_here) {
 #pragma unroll
         for (int m = 0; m < N; ++m)
           dszzdz += c[m] * (ldg(szz + idx + (m + 1)) - ldg(szz + idx - m));
-        dsxzdx = div_c(dsxzdx, dx, p.rd[0], p.fast_div);
-        dsyzdy = div_c(dsyzdy, dy, p.rd[1], p.fast_div);
-        dszzdz = div_c(dszzdz, dz, p.rd[2], p.fast_div);
+        spacings<T, 0, 1, 2>(p, dsxzdx, dsyzdy, dszzdz);
         if ((xi >= 0 || yj >= 0 || zk >= 0) && ((fx & 1) || (fy & 1) || (fz & 2))) {
           if (xi >= 0)
             pml_apply(p.mem[0] + 2 * p.mcomp[0] + ((long long)xi * ny + j) * nz + k,
@@ -222,7 +243,7 @@ k3_velocity(const __grid_constant__ P3<T> p, int it, int force_here) {
 // stress pass
 // ---------------------------------------------------------------------------
 template <typename T, int N>
-__global__ void __launch_bounds__(T3Z * T3Y)
+__global__ void __launch_bounds__(T3Z * T3Y, K3_MINB)
 k3_stress(const __grid_constant__ P3<T> p, int it, int inject_next) {
   const int nx = p.nx, ny = p.ny, nz = p.nz;
   // receivers: the velocity fields are final for this step and are not
@@ -319,9 +340,7 @@ k3_stress(const __grid_constant__ P3<T> p, int it, int inject_next) {
           const T hi = (m == 0) ? qvz[N - 1] : ldg(vz + idx + m);
           dvzdz += c[m] * (hi - ldg(vz + idx - (m + 1)));
         }
-        dvxdx = div_c(dvxdx, dx, p.rd[0], p.fast_div);
-        dvydy = div_c(dvydy, dy, p.rd[1], p.fast_div);
-        dvzdz = div_c(dvzdz, dz, p.rd[2], p.fast_div);
+        spacings<T, 0, 1, 2>(p, dvxdx, dvydy, dvzdz);
         if (any_slab && ((fx | fy | fz) & 1)) {
           if (xi >= 0)
             pml_apply(p.mem[0] + 3 * p.mcomp[0] + ((long long)xi * ny + j) * nz + k,
@@ -362,8 +381,7 @@ k3_stress(const __grid_constant__ P3<T> p, int it, int inject_next) {
           const T lo = (m == 0) ? qvx[N] : ldg(vx + idx - (long long)m * nz);
           dvxdy += c[m] * (ldg(vx + idx + (long long)(m + 1) * nz) - lo);
         }
-        dvydx = div_c(dvydx, dx, p.rd[0], p.fast_div);
-        dvxdy = div_c(dvxdy, dy, p.rd[1], p.fast_div);
+        spacings<T, 0, 1>(p, dvydx, dvxdy);
         if (any_slab && ((fx & 2) || (fy & 2) || (fz & 1))) {
           if (xi >= 0)
             pml_apply(p.mem[0] + 4 * p.mcomp[0] + ((long long)xi * ny + j) * nz + k,
@@ -393,8 +411,7 @@ k3_stress(const __grid_constant__ P3<T> p, int it, int inject_next) {
           const T lo = (m == 0) ? qvx[N] : ldg(vx + idx - m);
           dvxdz += c[m] * (ldg(vx + idx + (m + 1)) - lo);
         }
-        dvzdx = div_c(dvzdx, dx, p.rd[0], p.fast_div);
-        dvxdz = div_c(dvxdz, dz, p.rd[2], p.fast_div);
+        spacings<T, 0, 2>(p, dvzdx, dvxdz);
         if (any_slab && ((fx & 2) || (fy & 1) || (fz & 2))) {
           if (xi >= 0)
             pml_apply(p.mem[0] + 5 * p.mcomp[0] + ((long long)xi * ny + j) * nz + k,
@@ -427,8 +444,7 @@ k3_stress(const __grid_constant__ P3<T> p, int it, int inject_next) {
           const T lo = (m == 0) ? qvy[N - 1] : ldg(vy + idx - m);
           dvydz += c[m] * (ldg(vy + idx + (m + 1)) - lo);
         }
-        dvzdy = div_c(dvzdy, dy, p.rd[1], p.fast_div);
-        dvydz = div_c(dvydz, dz, p.rd[2], p.fast_div);
+        spacings<T, 1, 2>(p, dvzdy, dvydz);
         if (any_slab && ((fx & 1) || (fy & 2) || (fz & 2))) {
           if (yj >= 0)
             pml_apply(p.mem[1] + 5 * p.mcomp[1] + ((long long)i * p.sn[1] + yj) * nz + k,

@@ -381,16 +381,13 @@ __device__ __forceinline__ float mk_div(float x, float d, float r) {
 // bits.
 template <int K>
 __device__ __forceinline__ void divc_group(float (&x)[K], const float (&d)[K], const float (&r)[K], int fast) {
-  bool ok = fast != 0, small = fast != 0;
+  RangeAcc acc;
 #pragma unroll
-  for (int k = 0; k < K; ++k) {
-    ok = ok & mk_ok(x[k]);
-    small = small & (fabsf(x[k]) < 0x1p100f);
-  }
-  if (ok) {
+  for (int k = 0; k < K; ++k) acc.add(x[k]);
+  if (fast != 0 && acc.ok()) {
 #pragma unroll
     for (int k = 0; k < K; ++k) x[k] = mk_div(x[k], d[k], r[k]);
-  } else if (small) {
+  } else if (fast != 0 && acc.below_huge()) {
 #pragma unroll
     for (int k = 0; k < K; ++k) x[k] = mk_div_any(x[k], d[k], r[k]);
   } else {
@@ -399,9 +396,21 @@ __device__ __forceinline__ void divc_group(float (&x)[K], const float (&d)[K], c
   }
 }
 template <int K>
-__device__ __forceinline__ void divc_group(double (&x)[K], const double (&d)[K], const double (&r)[K], int fast) {
+__device__ __forceinline__ void divc_group(double (&x)[K], const double (&d)[K], const double (&r)[K], int) {
+  RangeAccT<double> acc;
+  bool dok = true;
 #pragma unroll
-  for (int k = 0; k < K; ++k) x[k] = div_c(x[k], d[k], r[k], fast);
+  for (int k = 0; k < K; ++k) {
+    acc.add(x[k]);
+    dok = dok && mk2_divisor(d[k]);
+  }
+  if (dok && acc.ok()) {
+#pragma unroll
+    for (int k = 0; k < K; ++k) x[k] = x[k] == 0.0 ? x[k] : mk2_core(x[k], d[k], r[k]);
+  } else {
+#pragma unroll
+    for (int k = 0; k < K; ++k) x[k] = div_v(x[k], d[k]);
+  }
 }
 // quotients by per-cell positive divisors (densities), grouped likewise
 template <int K>
