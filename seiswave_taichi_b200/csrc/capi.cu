@@ -110,6 +110,42 @@ int cuda_fail(cudaError_t e, const char* where) {
   return fail(SW_ERR_CUDA, std::string(where) + ": " + cudaGetErrorString(e));
 }
 
+// Copy of several arrays in one launch, blockIdx.y the array: a state snapshot
+// was 7 (2D) or 12 (3D) device-to-device copies of 3 to 11 us each, most of
+// that their own start and end
+struct CopyList {
+  const void* src[12];
+  void* dst[12];
+  long long bytes[12];  // multiples of 4
+  int n = 0;
+  void add(const void* s, void* d, long long b) {
+    if (b <= 0) return;
+    src[n] = s;
+    dst[n] = d;
+    bytes[n++] = b;
+  }
+};
+__global__ void k_copy_arrays(const __grid_constant__ CopyList l) {
+  const char* s = (const char*)l.src[blockIdx.y];
+  char* d = (char*)l.dst[blockIdx.y];
+  const long long b = l.bytes[blockIdx.y], t = (long long)blockIdx.x * blockDim.x + threadIdx.x,
+                  nt = (long long)gridDim.x * blockDim.x;
+  long long done = 0;
+  if ((((uintptr_t)s | (uintptr_t)d) & 15) == 0) {
+    done = b / 16 * 16;
+    for (long long q = t; q < b / 16; q += nt) reinterpret_cast<float4*>(d)[q] = reinterpret_cast<const float4*>(s)[q];
+  }
+  for (long long q = done / 4 + t; q < b / 4; q += nt) reinterpret_cast<float*>(d)[q] = reinterpret_cast<const float*>(s)[q];
+}
+cudaError_t copy_arrays(const CopyList& l, cudaStream_t st) {
+  if (l.n == 0) return cudaSuccess;
+  long long most = 0;
+  for (int q = 0; q < l.n; ++q) most = std::max(most, l.bytes[q]);
+  const int blocks = (int)std::min<long long>((most + 4095) / 4096, 592);
+  k_copy_arrays<<<dim3(blocks, l.n), 256, 0, st>>>(l);
+  return cudaGetLastError();
+}
+
 // count of non-finite values over a set of arrays
 template <typename T>
 __global__ void k_count_nonfinite(const T* a, long long n, unsigned long long* out) {
@@ -1231,15 +1267,11 @@ long long snap_elems(const sw::P2<T>& p) {
 template <typename T>
 cudaError_t snap_store(const sw::P2<T>& p, T* slot, cudaStream_t st) {
   const long long nc = (long long)p.nx * p.nz;
-  cudaError_t e = cudaSuccess;
-  for (int q = 0; q < 5 && e == cudaSuccess; ++q)
-    e = cudaMemcpyAsync(slot + q * nc, p.f[q], nc * sizeof(T), cudaMemcpyDeviceToDevice, st);
-  if (e == cudaSuccess && p.mcomp[0] > 0)
-    e = cudaMemcpyAsync(slot + 5 * nc, p.mem[0], 4 * p.mcomp[0] * sizeof(T), cudaMemcpyDeviceToDevice, st);
-  if (e == cudaSuccess && p.mcomp[1] > 0)
-    e = cudaMemcpyAsync(slot + 5 * nc + 4 * p.mcomp[0], p.mem[1], 4 * p.mcomp[1] * sizeof(T),
-                        cudaMemcpyDeviceToDevice, st);
-  return e;
+  CopyList l;
+  for (int q = 0; q < 5; ++q) l.add(p.f[q], slot + q * nc, nc * sizeof(T));
+  l.add(p.mem[0], slot + 5 * nc, 4 * p.mcomp[0] * sizeof(T));
+  l.add(p.mem[1], slot + 5 * nc + 4 * p.mcomp[0], 4 * p.mcomp[1] * sizeof(T));
+  return copy_arrays(l, st);
 }
 
 template <typename T>
@@ -1293,16 +1325,14 @@ long long snap3_elems(const sw::P3<T>& p) {
 template <typename T>
 cudaError_t snap3_store(const sw::P3<T>& p, T* slot, cudaStream_t st) {
   const long long nc = (long long)p.nx * p.ny * p.nz;
-  cudaError_t e = cudaSuccess;
-  for (int q = 0; q < 9 && e == cudaSuccess; ++q)
-    e = cudaMemcpyAsync(slot + q * nc, p.f[q], nc * sizeof(T), cudaMemcpyDeviceToDevice, st);
+  CopyList l;
+  for (int q = 0; q < 9; ++q) l.add(p.f[q], slot + q * nc, nc * sizeof(T));
   long long off = 9 * nc;
-  for (int a = 0; a < 3 && e == cudaSuccess; ++a) {
-    if (p.mcomp[a] > 0)
-      e = cudaMemcpyAsync(slot + off, p.mem[a], 6 * p.mcomp[a] * sizeof(T), cudaMemcpyDeviceToDevice, st);
+  for (int a = 0; a < 3; ++a) {
+    l.add(p.mem[a], slot + off, 6 * p.mcomp[a] * sizeof(T));
     off += 6 * p.mcomp[a];
   }
-  return e;
+  return copy_arrays(l, st);
 }
 
 template <typename T>
@@ -1316,6 +1346,18 @@ cudaError_t record3(sw_plan* pl, const sw::P3<T>& p, int it0, int n, T* snap, cu
     const int it = it0 + k;
     cudaError_t e = moment ? sw::sw3_moment_inject<T>(p, it, st) : cudaSuccess;
     if (e == cudaSuccess) e = snap3_store(p, snap + k * se, st);
+    if constexpr (std::is_same<T, float>::value) {
+      if (pl->path == 1 && pl->staged) {  // the plan's own kernels, exact: the two-pass kernels' bits
+        sw::StagedArgs sa = pl->sa;
+        sa.exact = 1;
+        if (e == cudaSuccess)
+          e = sw::sw3_staged_step(pl->staged_N, pl->staged_tz, false, tensor, p, pl->svm, pl->ssm, sa, it, force,
+                                  false, pl->gather_in_stress, st);
+        if (e == cudaSuccess && !pl->gather_in_stress) e = sw::sw3_gather<T>(p, it, st);
+        if (e != cudaSuccess) return e;
+        continue;
+      }
+    }
     if (e == cudaSuccess) e = sw::sw3_velocity<T>(q, pl->order, it, tensor, force && pl->src_in_kernel, st);
     if (e == cudaSuccess && force && !pl->src_in_kernel) e = sw::sw3_force_inject<T>(p, it, st);
     if (e == cudaSuccess) e = sw::sw3_stress<T>(q, pl->order, it, false, st);

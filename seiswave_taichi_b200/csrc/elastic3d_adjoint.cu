@@ -38,6 +38,10 @@ struct A3 {
 
 constexpr int B3Z = 32;
 constexpr int B3Y = 8;
+// Resident blocks per SM the float kernels are compiled for: one thread per
+// cell waits on its loads (104 x 96 x 80, order 2, stress / velocity mid us: the
+// compiler's own count 90 / 74, 4 blocks 78 / 74, 6 70 / 68, 8 74 / 68).
+#define SW_ADJ3_MINB (sizeof(T) == 4 ? 6 : 1)
 
 // stencil along one axis (stride st), forward (D+) or backward (D-)
 template <typename T, int N, bool FWD>
@@ -122,6 +126,17 @@ __device__ __forceinline__ const T* snap_mem(const P3<T>& p, const T* snap) {
   _Pragma("unroll") for (int m = 0; m < N; ++m) c[m] = p.c[m];  \
   const uint8_t fx = p.fl[0][i], fy = p.fl[1][j], fz = p.fl[2][k];
 
+// The nearest cell whose taps all lie inside the grid.  The mid kernels form
+// their nine derivatives there before they look at any range: all tap loads
+// are in flight together and the quotients by the spacings form one group (a
+// cell outside a component's range never uses that component's derivatives).
+// What bounded these kernels was 18 IEEE divisions a cell, one after another
+// behind the loads of its own component: 104 x 96 x 80, order 2, stress /
+// velocity mid 104 / 111 -> 90 / 74 us.
+#define INNER3                                                                                  \
+  const long long in = min(max(i, N), nx - 1 - N) * sx + (long long)min(max(j, N), ny - 1 - N) * nz + \
+                       min(max(k, N), nz - 1 - N);
+
 template <typename T>
 __global__ void k3a_record(const __grid_constant__ P3<T> p, const __grid_constant__ A3<T> a, int it) {
   const long long r = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -130,9 +145,10 @@ __global__ void k3a_record(const __grid_constant__ P3<T> p, const __grid_constan
 
 // ---- stress phase ---------------------------------------------------------------
 template <typename T, int N>
-__global__ void __launch_bounds__(B3Z * B3Y)
+__global__ void __launch_bounds__(B3Z * B3Y, SW_ADJ3_MINB)
 k3a_stress_mid(const __grid_constant__ P3<T> p, const __grid_constant__ A3<T> a) {
   CELL3
+  INNER3
   const long long nc = (long long)nx * ny * nz;
   const T* vx = a.snap1;
   const T* vy = a.snap1 + nc;
@@ -140,20 +156,26 @@ k3a_stress_mid(const __grid_constant__ P3<T> p, const __grid_constant__ A3<T> a)
   const T* m0 = snap_mem<T, 0>(p, a.snap0);
   const T* m1 = snap_mem<T, 1>(p, a.snap0);
   const T* m2 = snap_mem<T, 2>(p, a.snap0);
-  const T dx = p.dx, dy = p.dy, dz = p.dz, dt = p.dt;
+  const T dt = p.dt;
+  // the nine derivatives before their ranges are looked at (INNER3)
+  const T hd[9] = {p.dx, p.dy, p.dz, p.dx, p.dy, p.dx, p.dz, p.dy, p.dz};
+  const T hr[9] = {p.rd[0], p.rd[1], p.rd[2], p.rd[0], p.rd[1], p.rd[0], p.rd[2], p.rd[1], p.rd[2]};
+  T dv[9] = {d3<T, N, false>(vx, in, sx, c), d3<T, N, false>(vy, in, sy, c), d3<T, N, false>(vz, in, 1, c),
+             d3<T, N, true>(vy, in, sx, c),  d3<T, N, true>(vx, in, sy, c),  d3<T, N, true>(vz, in, sx, c),
+             d3<T, N, true>(vx, in, 1, c),   d3<T, N, true>(vz, in, sy, c),  d3<T, N, true>(vy, in, 1, c)};
+  divc_group<9>(dv, hd, hr, p.fast_div);
   T out[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+  const T u0 = ldg(p.mu + in), ux = ldg(p.mu + in + sx), uy = ldg(p.mu + in + sy), uz = ldg(p.mu + in + 1);
   // normal stresses: i, j, k in [N+1, n-N)
   if (i >= N + 1 && i < nx - N && j >= N + 1 && j < ny - N && k >= N + 1 && k < nz - N) {
-    const T lhx = (T)0.5 * (p.lam[idx] + p.lam[idx + sx]);
-    const T mhx = (T)0.5 * (p.mu[idx] + p.mu[idx + sx]);
+    const T lhx = (T)0.5 * (ldg(p.lam + idx) + ldg(p.lam + idx + sx));
+    const T mhx = (T)0.5 * (u0 + ux);
     const T lpm = lhx + (T)2 * mhx;
     const bool P = ((fx | fy | fz) & 1) != 0;
     auto cx = cpml3<T, 0>(p, 3, false, P, i, j, k);
     auto cy = cpml3<T, 1>(p, 3, false, P, i, j, k);
     auto cz = cpml3<T, 2>(p, 3, false, P, i, j, k);
-    T e0 = d3<T, N, false>(vx, idx, sx, c) / dx;
-    T e1 = d3<T, N, false>(vy, idx, sy, c) / dy;
-    T e2 = d3<T, N, false>(vz, idx, 1, c) / dz;
+    T e0 = dv[0], e1 = dv[1], e2 = dv[2];
     if (cx.on) e0 = pml_fwd3(e0, m0[cx.off], cx.b, cx.a, cx.kk);
     if (cy.on) e1 = pml_fwd3(e1, m1[cy.off], cy.b, cy.a, cy.kk);
     if (cz.on) e2 = pml_fwd3(e2, m2[cz.off], cz.b, cz.a, cz.kk);
@@ -166,18 +188,17 @@ k3a_stress_mid(const __grid_constant__ P3<T> p, const __grid_constant__ A3<T> a)
     if (cx.on) g0 = pml_adj3(g0, a.mem[0] + cx.off, cx.b, cx.a, cx.kk);
     if (cy.on) g1 = pml_adj3(g1, a.mem[1] + cy.off, cy.b, cy.a, cy.kk);
     if (cz.on) g2 = pml_adj3(g2, a.mem[2] + cz.off, cz.b, cz.a, cz.kk);
-    out[0] = g0 / dx;
-    out[1] = g1 / dy;
-    out[2] = g2 / dz;
+    out[0] = g0;
+    out[1] = g1;
+    out[2] = g2;
   }
   // sxy: i, j in [N+1, n-N), k in [N, nz-N)
   if (i >= N + 1 && i < nx - N && j >= N + 1 && j < ny - N && k >= N && k < nz - N) {
-    const T m4 = (T)0.25 * (p.mu[idx + sy] + p.mu[idx] + p.mu[idx] + p.mu[idx + sx]);
+    const T m4 = (T)0.25 * (uy + u0 + u0 + ux);
     const bool P = (fx & 2) || (fy & 2) || (fz & 1);
     auto cx = cpml3<T, 0>(p, 4, true, P, i, j, k);
     auto cy = cpml3<T, 1>(p, 4, true, P, i, j, k);
-    T f0 = d3<T, N, true>(vy, idx, sx, c) / dx;
-    T f1 = d3<T, N, true>(vx, idx, sy, c) / dy;
+    T f0 = dv[3], f1 = dv[4];
     if (cx.on) f0 = pml_fwd3(f0, m0[cx.off], cx.b, cx.a, cx.kk);
     if (cy.on) f1 = pml_fwd3(f1, m1[cy.off], cy.b, cy.a, cy.kk);
     const T b = a.f[6][idx];
@@ -185,17 +206,16 @@ k3a_stress_mid(const __grid_constant__ P3<T> p, const __grid_constant__ A3<T> a)
     T g = m4 * dt * b, g0 = g, g1 = g;
     if (cx.on) g0 = pml_adj3(g0, a.mem[0] + cx.off, cx.b, cx.a, cx.kk);
     if (cy.on) g1 = pml_adj3(g1, a.mem[1] + cy.off, cy.b, cy.a, cy.kk);
-    out[3] = g0 / dx;
-    out[4] = g1 / dy;
+    out[3] = g0;
+    out[4] = g1;
   }
   // sxz: i in [N, nx-N-1), j in [N, ny-N), k in [N, nz-N-1)
   if (i >= N && i < nx - N - 1 && j >= N && j < ny - N && k >= N && k < nz - N - 1) {
-    const T m4 = (T)0.25 * (p.mu[idx] + p.mu[idx + sx] + p.mu[idx] + p.mu[idx + sy]);
+    const T m4 = (T)0.25 * (u0 + ux + u0 + uy);
     const bool P = (fx & 2) || (fy & 1) || (fz & 2);
     auto cx = cpml3<T, 0>(p, 5, true, P, i, j, k);
     auto cz = cpml3<T, 2>(p, 4, true, P, i, j, k);
-    T h0 = d3<T, N, true>(vz, idx, sx, c) / dx;
-    T h1 = d3<T, N, true>(vx, idx, 1, c) / dz;
+    T h0 = dv[5], h1 = dv[6];
     if (cx.on) h0 = pml_fwd3(h0, m0[cx.off], cx.b, cx.a, cx.kk);
     if (cz.on) h1 = pml_fwd3(h1, m2[cz.off], cz.b, cz.a, cz.kk);
     const T b = a.f[7][idx];
@@ -203,17 +223,16 @@ k3a_stress_mid(const __grid_constant__ P3<T> p, const __grid_constant__ A3<T> a)
     T g = m4 * dt * b, g0 = g, g1 = g;
     if (cx.on) g0 = pml_adj3(g0, a.mem[0] + cx.off, cx.b, cx.a, cx.kk);
     if (cz.on) g1 = pml_adj3(g1, a.mem[2] + cz.off, cz.b, cz.a, cz.kk);
-    out[5] = g0 / dx;
-    out[6] = g1 / dz;
+    out[5] = g0;
+    out[6] = g1;
   }
   // syz: i in [N, nx-N), j in [N, ny-N-1), k in [N, nz-N-1)
   if (i >= N && i < nx - N && j >= N && j < ny - N - 1 && k >= N && k < nz - N - 1) {
-    const T m4 = (T)0.25 * (p.mu[idx + sy] + p.mu[idx] + p.mu[idx + 1] + p.mu[idx]);
+    const T m4 = (T)0.25 * (uy + u0 + uz + u0);
     const bool P = (fx & 1) || (fy & 2) || (fz & 2);
     auto cy = cpml3<T, 1>(p, 5, true, P, i, j, k);
     auto cz = cpml3<T, 2>(p, 5, true, P, i, j, k);
-    T q0 = d3<T, N, true>(vz, idx, sy, c) / dy;
-    T q1 = d3<T, N, true>(vy, idx, 1, c) / dz;
+    T q0 = dv[7], q1 = dv[8];
     if (cy.on) q0 = pml_fwd3(q0, m1[cy.off], cy.b, cy.a, cy.kk);
     if (cz.on) q1 = pml_fwd3(q1, m2[cz.off], cz.b, cz.a, cz.kk);
     const T b = a.f[8][idx];
@@ -221,9 +240,10 @@ k3a_stress_mid(const __grid_constant__ P3<T> p, const __grid_constant__ A3<T> a)
     T g = m4 * dt * b, g0 = g, g1 = g;
     if (cy.on) g0 = pml_adj3(g0, a.mem[1] + cy.off, cy.b, cy.a, cy.kk);
     if (cz.on) g1 = pml_adj3(g1, a.mem[2] + cz.off, cz.b, cz.a, cz.kk);
-    out[7] = g0 / dy;
-    out[8] = g1 / dz;
+    out[7] = g0;
+    out[8] = g1;
   }
+  divc_group<9>(out, hd, hr, p.fast_div);
 #pragma unroll
   for (int q = 0; q < 9; ++q) a.tmp[q][idx] = out[q];
 }
@@ -231,7 +251,7 @@ k3a_stress_mid(const __grid_constant__ P3<T> p, const __grid_constant__ A3<T> a)
 // vx_bar += D-x^T t0 + D+y^T t4 + D+z^T t6; vy_bar += D-y^T t1 + D+x^T t3 + D+z^T t8;
 // vz_bar += D-z^T t2 + D+x^T t5 + D+y^T t7
 template <typename T, int N>
-__global__ void __launch_bounds__(B3Z * B3Y)
+__global__ void __launch_bounds__(B3Z * B3Y, SW_ADJ3_MINB)
 k3a_vel_gather(const __grid_constant__ P3<T> p, const __grid_constant__ A3<T> a) {
   CELL3
   (void)fx; (void)fy; (void)fz;
@@ -245,9 +265,10 @@ k3a_vel_gather(const __grid_constant__ P3<T> p, const __grid_constant__ A3<T> a)
 
 // ---- velocity phase -------------------------------------------------------------
 template <typename T, int N>
-__global__ void __launch_bounds__(B3Z * B3Y)
+__global__ void __launch_bounds__(B3Z * B3Y, SW_ADJ3_MINB)
 k3a_vel_mid(const __grid_constant__ P3<T> p, const __grid_constant__ A3<T> a) {
   CELL3
+  INNER3
   const long long nc = (long long)nx * ny * nz;
   const T* sxx = a.snap0 + 3 * nc;
   const T* syy = a.snap0 + 4 * nc;
@@ -258,41 +279,44 @@ k3a_vel_mid(const __grid_constant__ P3<T> p, const __grid_constant__ A3<T> a) {
   const T* m0 = snap_mem<T, 0>(p, a.snap0);
   const T* m1 = snap_mem<T, 1>(p, a.snap0);
   const T* m2 = snap_mem<T, 2>(p, a.snap0);
-  const T dx = p.dx, dy = p.dy, dz = p.dz, dt = p.dt;
+  const T dt = p.dt;
   const T* rho = p.rho;
+  const T hd[9] = {p.dx, p.dy, p.dz, p.dx, p.dy, p.dz, p.dx, p.dy, p.dz};
+  const T hr[9] = {p.rd[0], p.rd[1], p.rd[2], p.rd[0], p.rd[1], p.rd[2], p.rd[0], p.rd[1], p.rd[2]};
+  T dv[9] = {d3<T, N, true>(sxx, in, sx, c),  d3<T, N, false>(sxy, in, sy, c), d3<T, N, false>(sxz, in, 1, c),
+             d3<T, N, false>(sxy, in, sx, c), d3<T, N, true>(syy, in, sy, c),  d3<T, N, false>(syz, in, 1, c),
+             d3<T, N, false>(sxz, in, sx, c), d3<T, N, false>(syz, in, sy, c), d3<T, N, true>(szz, in, 1, c)};
+  divc_group<9>(dv, hd, hr, p.fast_div);
   T out[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+  const T r00 = ldg(rho + in), r01 = ldg(rho + in + sy), r11 = ldg(rho + in + sx + sy), r10 = ldg(rho + in + sx);
   // vx: i in [N, nx-N-1), j in [N+1, ny-N), k in [N+1, nz-N)
   if (i >= N && i < nx - N - 1 && j >= N + 1 && j < ny - N && k >= N + 1 && k < nz - N) {
     const bool P = (fx & 2) || (fy & 1) || (fz & 1);
     auto cx = cpml3<T, 0>(p, 0, true, P, i, j, k);
     auto cy = cpml3<T, 1>(p, 0, false, P, i, j, k);
     auto cz = cpml3<T, 2>(p, 0, false, P, i, j, k);
-    T d0 = d3<T, N, true>(sxx, idx, sx, c) / dx;
-    T d1 = d3<T, N, false>(sxy, idx, sy, c) / dy;
-    T d2 = d3<T, N, false>(sxz, idx, 1, c) / dz;
+    T d0 = dv[0], d1 = dv[1], d2 = dv[2];
     if (cx.on) d0 = pml_fwd3(d0, m0[cx.off], cx.b, cx.a, cx.kk);
     if (cy.on) d1 = pml_fwd3(d1, m1[cy.off], cy.b, cy.a, cy.kk);
     if (cz.on) d2 = pml_fwd3(d2, m2[cz.off], cz.b, cz.a, cz.kk);
     const T vb = a.f[0][idx];
     a.grad[0][idx] += vb * (d0 + d2 + d1) * dt;
-    T g = vb * dt / rho[idx], g0 = g, g1 = g, g2 = g;
+    T g = vb * dt / r00, g0 = g, g1 = g, g2 = g;
     if (cx.on) g0 = pml_adj3(g0, a.mem[0] + cx.off, cx.b, cx.a, cx.kk);
     if (cy.on) g1 = pml_adj3(g1, a.mem[1] + cy.off, cy.b, cy.a, cy.kk);
     if (cz.on) g2 = pml_adj3(g2, a.mem[2] + cz.off, cz.b, cz.a, cz.kk);
-    out[0] = g0 / dx;
-    out[1] = g1 / dy;
-    out[2] = g2 / dz;
+    out[0] = g0;
+    out[1] = g1;
+    out[2] = g2;
   }
   // vy: i in [N+1, nx-N), j in [N, ny-N-1), k in [N+1, nz-N)
   if (i >= N + 1 && i < nx - N && j >= N && j < ny - N - 1 && k >= N + 1 && k < nz - N) {
-    const T rhy = (T)0.5 * (rho[idx] + rho[idx + sy]);
+    const T rhy = (T)0.5 * (r00 + r01);
     const bool P = (fx & 1) || (fy & 2) || (fz & 1);
     auto cx = cpml3<T, 0>(p, 1, false, P, i, j, k);
     auto cy = cpml3<T, 1>(p, 1, true, P, i, j, k);
     auto cz = cpml3<T, 2>(p, 1, false, P, i, j, k);
-    T d0 = d3<T, N, false>(sxy, idx, sx, c) / dx;
-    T d1 = d3<T, N, true>(syy, idx, sy, c) / dy;
-    T d2 = d3<T, N, false>(syz, idx, 1, c) / dz;
+    T d0 = dv[3], d1 = dv[4], d2 = dv[5];
     if (cx.on) d0 = pml_fwd3(d0, m0[cx.off], cx.b, cx.a, cx.kk);
     if (cy.on) d1 = pml_fwd3(d1, m1[cy.off], cy.b, cy.a, cy.kk);
     if (cz.on) d2 = pml_fwd3(d2, m2[cz.off], cz.b, cz.a, cz.kk);
@@ -302,20 +326,18 @@ k3a_vel_mid(const __grid_constant__ P3<T> p, const __grid_constant__ A3<T> a) {
     if (cx.on) g0 = pml_adj3(g0, a.mem[0] + cx.off, cx.b, cx.a, cx.kk);
     if (cy.on) g1 = pml_adj3(g1, a.mem[1] + cy.off, cy.b, cy.a, cy.kk);
     if (cz.on) g2 = pml_adj3(g2, a.mem[2] + cz.off, cz.b, cz.a, cz.kk);
-    out[3] = g0 / dx;
-    out[4] = g1 / dy;
-    out[5] = g2 / dz;
+    out[3] = g0;
+    out[4] = g1;
+    out[5] = g2;
   }
   // vz: i in [N+1, nx-N), j in [N+1, ny-N), k in [N, nz-N-1)
   if (i >= N + 1 && i < nx - N && j >= N + 1 && j < ny - N && k >= N && k < nz - N - 1) {
-    const T r4 = (T)0.25 * (rho[idx] + rho[idx + sy] + rho[idx + sx + sy] + rho[idx + sx]);
+    const T r4 = (T)0.25 * (r00 + r01 + r11 + r10);
     const bool P = (fx & 1) || (fy & 1) || (fz & 2);
     auto cx = cpml3<T, 0>(p, 2, false, P, i, j, k);
     auto cy = cpml3<T, 1>(p, 2, false, P, i, j, k);
     auto cz = cpml3<T, 2>(p, 2, true, P, i, j, k);
-    T d0 = d3<T, N, false>(sxz, idx, sx, c) / dx;
-    T d1 = d3<T, N, false>(syz, idx, sy, c) / dy;
-    T d2 = d3<T, N, true>(szz, idx, 1, c) / dz;
+    T d0 = dv[6], d1 = dv[7], d2 = dv[8];
     if (cx.on) d0 = pml_fwd3(d0, m0[cx.off], cx.b, cx.a, cx.kk);
     if (cy.on) d1 = pml_fwd3(d1, m1[cy.off], cy.b, cy.a, cy.kk);
     if (cz.on) d2 = pml_fwd3(d2, m2[cz.off], cz.b, cz.a, cz.kk);
@@ -325,10 +347,11 @@ k3a_vel_mid(const __grid_constant__ P3<T> p, const __grid_constant__ A3<T> a) {
     if (cx.on) g0 = pml_adj3(g0, a.mem[0] + cx.off, cx.b, cx.a, cx.kk);
     if (cy.on) g1 = pml_adj3(g1, a.mem[1] + cy.off, cy.b, cy.a, cy.kk);
     if (cz.on) g2 = pml_adj3(g2, a.mem[2] + cz.off, cz.b, cz.a, cz.kk);
-    out[6] = g0 / dx;
-    out[7] = g1 / dy;
-    out[8] = g2 / dz;
+    out[6] = g0;
+    out[7] = g1;
+    out[8] = g2;
   }
+  divc_group<9>(out, hd, hr, p.fast_div);
 #pragma unroll
   for (int q = 0; q < 9; ++q) a.tmp[q][idx] = out[q];
 }
@@ -336,7 +359,7 @@ k3a_vel_mid(const __grid_constant__ P3<T> p, const __grid_constant__ A3<T> a) {
 // sxx_bar += D+x^T t0; syy_bar += D+y^T t4; szz_bar += D+z^T t8;
 // sxy_bar += D-y^T t1 + D-x^T t3; sxz_bar += D-z^T t2 + D-x^T t6; syz_bar += D-z^T t5 + D-y^T t7
 template <typename T, int N>
-__global__ void __launch_bounds__(B3Z * B3Y)
+__global__ void __launch_bounds__(B3Z * B3Y, SW_ADJ3_MINB)
 k3a_str_gather(const __grid_constant__ P3<T> p, const __grid_constant__ A3<T> a) {
   CELL3
   (void)fx; (void)fy; (void)fz;
@@ -349,6 +372,7 @@ k3a_str_gather(const __grid_constant__ P3<T> p, const __grid_constant__ A3<T> a)
 }
 
 #undef CELL3
+#undef INNER3
 
 // The point force (Elastic3D_SSG_CPML.py:245) adds t/rho[src], t = dt*w(it),
 // to vz after the velocity phase; its adjoint leaves vz_bar as it is and adds
