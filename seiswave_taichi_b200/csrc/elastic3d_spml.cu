@@ -12,6 +12,11 @@
 
 namespace sw {
 
+// Resident blocks per SM the float kernels are compiled for: one thread per
+// cell waits on its loads (100^3 order 4 / 100 x 90 x 103 order 3, us per step:
+// the compiler's own count 165 / 181, 4 blocks 152 / 162, 6 125 / 132, 8 112 /
+// 120)
+#define SW_KS_MINB (sizeof(T) == 4 ? 8 : 1)
 constexpr int TSZ = 32;
 constexpr int TSY = 8;
 
@@ -31,7 +36,7 @@ __device__ __forceinline__ T d_bm(const T* f, long long idx, long long s, const 
 }
 
 template <typename T, int N>
-__global__ void __launch_bounds__(TSZ * TSY)
+__global__ void __launch_bounds__(TSZ * TSY, SW_KS_MINB)
 ks_velocity(const __grid_constant__ P3<T> p, int it, int src_here) {
   const int k = blockIdx.x * TSZ + threadIdx.x;
   const int j = blockIdx.y * TSY + threadIdx.y;
@@ -131,7 +136,7 @@ ks_velocity(const __grid_constant__ P3<T> p, int it, int src_here) {
 }
 
 template <typename T, int N>
-__global__ void __launch_bounds__(TSZ * TSY)
+__global__ void __launch_bounds__(TSZ * TSY, SW_KS_MINB)
 ks_stress(const __grid_constant__ P3<T> p, int it) {
   {
     const long long b = blockIdx.x + (long long)gridDim.x * (blockIdx.y + (long long)gridDim.y * blockIdx.z);
