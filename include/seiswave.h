@@ -168,8 +168,9 @@ SW_API int sw2d_plan_create(const sw2d_desc* desc, sw_plan** plan);
  * Elastic3D_SSG_SPML.py:8-138 and their SetADEPML3D. */
 SW_API int sw3d_plan_create(const sw3d_desc* desc, sw_plan** plan);
 
-/* Override the number of x planes one CTA streams in the 3D CPML passes
- * (the autotuner's knob; the plan picks a default from the grid and SM count). */
+/* Accepted for 3D plans and without effect: the kernels of path 0 give each
+ * cell its own thread and stream no x planes (path 1 and 2 take their planes
+ * per work unit through sw_plan_set_path). */
 SW_API int sw_plan_set_tile(sw_plan* plan, int32_t x_chunk);
 
 /* No reference counterpart (a self-check of this library's exact division).
@@ -194,13 +195,15 @@ SW_API int sw_check_division(float divisor, int32_t mode, uint64_t* mismatches, 
 SW_API int sw_plan_status(sw_plan* plan, void* stream);
 
 /* Describe the plan's execution path: info[0] current path of sw_step/sw_run
- * (0 register-queue two-pass kernels; 2D: sw_step and sw_run without a graph
+ * (0 per-cell two-pass kernels, the default of 3D float64 plans, of split
+ * PML and of orders 3 and 4 in exact numerics; 2D: sw_step and sw_run without a graph
  * make two launches per step, sw_run with one keeps runs of at least 4 steps of
  * orders up to 4 that record a velocity on the chip where their tiles fit --
  * one cooperative launch, neighbouring tiles exchange their rims -- and
- * replays the launches otherwise; 3D float: a run of at least 6 steps whose
- * rows are no multiple of 16 bytes steps pitched copies of the state with the
- * kernels of path 1 and copies them back; 1 TMA-staged
+ * replays the launches otherwise; 3D float CPML of orders 1 and 2: a run of at
+ * least 6 steps of a large grid whose rows are no multiple of 16 bytes steps
+ * pitched copies of the state with the kernels of path 1 and copies them back;
+ * 1 TMA-staged
  * two-pass kernels, 2 fused single-pass kernel, 3 2D persistent: sw_run is
  * one cooperative launch for all its steps, the phases separated by a
  * bounded grid barrier; opt-in, as path 0 is faster on B200 at every grid

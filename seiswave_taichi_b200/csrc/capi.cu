@@ -201,6 +201,7 @@ struct sw_plan {
   // two-pass, 2: fused single pass, 3: 2D persistent (one cooperative launch
   // per run)
   int path = 0;
+  bool path_chosen = false;  // by sw_plan_set_path
   unsigned int* d_bar = nullptr;  // 2D persistent path: grid-barrier arrival and generation words
   bool aea = false;               // free-surface hook before every step (sw_plan_set_free_surface)
   // 2D on-chip loop (sw_run of path 0): tiles (0: not available) and the rim inbox
@@ -282,17 +283,6 @@ void fill_axis3(sw::P3<T>& p, int d, const sw_pml_axis& a, int n) {
   (void)n;
 }
 
-// x planes streamed by one CTA of the two-pass kernels: three, or two where
-// three would leave SMs without their four CTAs (double, order 2, us per step
-// with 2, 3, 4, 8 planes: 60 x 60 x 62 58, 72, 89, 144; 90^3 154, 167, 186, 222;
-// 128 x 120 x 112 324, 327, 340, 393; 200^3 1174, 1152, 1143, 1157)
-int choose_x_chunk(int nx, int ny, int nz) {
-  int dev = 0, sms = 148;
-  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const long long tiles = (long long)((nz + 31) / 32) * ((ny + 7) / 8);
-  return tiles * ((nx + 2) / 3) < 4LL * 4 * sms ? 2 : 3;
-}
-
 // ---------------------------------------------------------------------------
 // constant divisors: enable div_c's Markstein path only where it equals IEEE
 // division for every finite float numerator (checked once per divisor value)
@@ -352,7 +342,6 @@ int make_p3(sw_plan* pl, const sw3d_desc* d, sw::P3<T>& p) {
   p.nrec = d->rec.nrec; p.rec_field = d->rec.field;
   p.rec_idx = (const long long*)d->rec.index; p.rec_data = d->rec.data;
   p.rec_f64 = d->rec.dtype == SW_F64;
-  p.x_chunk = choose_x_chunk(d->nx, d->ny, d->nz);
   const double hs[3] = {d->dx, d->dy, d->dz};
   set_divisors<T>(p.rd, &p.fast_div, hs, 3);
   for (int a = 0; a < 3; ++a)
@@ -621,6 +610,18 @@ void staged_chunks(sw_plan* pl, int len) {
   a.chunks = (p.nx + len - 1) / len;
 }
 
+// The path of a 3D plan that its caller has not chosen: the staged kernels in
+// the fast numeric mode (only they have it) and for CPML of orders 1 and 2; the
+// per-cell kernels for split PML and orders 3 and 4, whose staged tiles leave
+// too few warps on an SM (us per step at 200^3, staged / per cell: order 2 412
+// / 573, order 3 683 / 615, order 4 736 / 636; split PML order 2 738 / 622,
+// order 4 1229 / 718).
+int default_path3(const sw_plan* pl) {
+  if (!pl->staged) return 0;
+  if (pl->scheme == SW3D_SPML) return 0;
+  return pl->sa.exact == 0 || pl->order <= 2 ? 1 : 0;
+}
+
 void setup_staged(sw_plan* pl) {
   pl->staged = false;
   if (pl->dim != 3 || pl->dtype != SW_F32) return;
@@ -642,16 +643,11 @@ void setup_staged(sw_plan* pl) {
   bool direct = p.nz % 4 == 0;
   for (int q = 0; q < 9; ++q) direct = direct && aligned(p.f[q], 16);
   direct = direct && aligned(p.rho, 16) && aligned(p.lam, 16) && aligned(p.mu, 16);
-  // Split PML of orders 3 and 4 on small grids: their staged tiles leave one CTA
-  // per SM, and the per-cell kernels are faster below about two million cells
-  // (us per step, staged / per cell: order 3 100^3 242 / 216, 140^3 354 / 533;
-  // order 4 60 x 60 x 64 68 / 41, 100^3 247 / 169, 140^3 491 / 502, 200^3
-  // 1229 / 1342)
-  const bool worth = pl->scheme != SW3D_SPML || pl->order <= 2 || (long long)p.nx * p.ny * p.nz >= 2000000LL;
-  // Rows that are no multiple of 16 bytes: a run steps pitched copies (us per
-  // step, the caller's rows with the two-pass kernels -> pitched: 60 x 61 x 62
-  // 68 -> 35, 153 x 131 x 117 order 3 462 -> 302, 200 x 190 x 201 1320 -> 422)
-  pl->pitch_ok = p.nz % 4 != 0 && pl->gather_in_stress && worth;
+  // Rows that are no multiple of 16 bytes: a run steps pitched copies where the
+  // staged kernels are the faster path by more than the way in and out (us per
+  // step, per cell -> pitched: 200 x 190 x 201 order 2 560 -> 422)
+  pl->pitch_ok = p.nz % 4 != 0 && pl->gather_in_stress && pl->scheme != SW3D_SPML && pl->order <= 2 &&
+                 (long long)p.nx * p.ny * p.nz >= 1500000LL;
   if (!direct && !pl->pitch_ok) return;
   if (!pl->d_err) {
     if (cudaMalloc(&pl->d_err, 3 * sizeof(int)) != cudaSuccess) {
@@ -667,10 +663,9 @@ void setup_staged(sw_plan* pl) {
   pl->sa.err = pl->d_err;
   pl->sa.next = pl->d_err + 1;
   pl->sa.exact = 1;
-  staged_chunks(pl, 0);
-  if (!direct) return;
-  pl->staged = true;
-  if (worth) pl->path = 1;
+  pl->staged = direct;
+  pl->path = default_path3(pl);
+  if (pl->path == 1 || pl->pitch_ok) staged_chunks(pl, 0);  // else when the path is chosen
 }
 
 // The pitched copies of a plan: true when they exist.  They are allocated by
@@ -688,8 +683,7 @@ bool pitch_ready(sw_plan* pl, int nsteps, cudaStream_t st) {
   const int pz = (p.nz + 3) / 4 * 4;
   const size_t cells = (size_t)p.nx * p.ny * pz;
   const size_t m0 = (size_t)p.sn[0] * p.ny * pz, m1 = (size_t)p.nx * p.sn[1] * pz;
-  const bool mem = pl->scheme != SW3D_SPML;
-  const size_t total = 12 * cells + (mem ? 6 * (m0 + m1) : 0);
+  const size_t total = 12 * cells + 6 * (m0 + m1);
   float* b = nullptr;
   if (cudaMalloc(&b, total * sizeof(float)) != cudaSuccess) {
     cudaGetLastError();
@@ -702,12 +696,10 @@ bool pitch_ready(sw_plan* pl, int nsteps, cudaStream_t st) {
   q.rho = cur, cur += cells;
   q.lam = cur, cur += cells;
   q.mu = cur, cur += cells;
-  if (mem) {
-    q.mem[0] = cur, cur += 6 * m0;
-    q.mem[1] = cur;
-    q.mcomp[0] = (long long)m0;
-    q.mcomp[1] = (long long)m1;
-  }
+  q.mem[0] = cur, cur += 6 * m0;
+  q.mem[1] = cur;
+  q.mcomp[0] = (long long)m0;
+  q.mcomp[1] = (long long)m1;
   if (!sw::sw3_staged_maps(pl->staged_N, pl->staged_tz, q, &pl->pvm, &pl->psm)) {
     cudaFree(b);
     pl->pitch_ok = false;
@@ -721,7 +713,7 @@ bool pitch_ready(sw_plan* pl, int nsteps, cudaStream_t st) {
 cudaError_t enqueue_pitched_run(sw_plan* pl, int it0, int nsteps, cudaStream_t st) {
   const auto& p = pl->p3f;
   const auto& q = pl->pp;
-  const bool spml = pl->scheme == SW3D_SPML, tensor = pl->scheme == SW3D_CPML_TENSOR;
+  const bool tensor = pl->scheme == SW3D_CPML_TENSOR;
   const bool moment = pl->src_kind == SW_SRC_MOMENT, force = pl->src_kind == SW_SRC_FORCE;
   cudaError_t e = cudaSuccess;
   if (moment) e = sw::sw3_moment_inject<float>(p, it0, st);
@@ -736,13 +728,13 @@ cudaError_t enqueue_pitched_run(sw_plan* pl, int it0, int nsteps, cudaStream_t s
   in(p.rho, q.rho, rows);
   in(p.lam, q.lam, rows);
   in(p.mu, q.mu, rows);
-  const long long r0 = spml ? 0 : 6LL * p.sn[0] * p.ny, r1 = spml ? 0 : 6LL * p.nx * p.sn[1];
+  const long long r0 = 6LL * p.sn[0] * p.ny, r1 = 6LL * p.nx * p.sn[1];
   in(p.mem[0], q.mem[0], r0);
   in(p.mem[1], q.mem[1], r1);
   sw::StagedArgs a = pl->sa;
   a.exact = 1;  // path 0 is always exact
   for (int s = 0; s < nsteps && e == cudaSuccess; ++s)
-    e = sw::sw3_staged_step(pl->staged_N, pl->staged_tz, spml, tensor, q, pl->pvm, pl->psm, a, it0 + s, force,
+    e = sw::sw3_staged_step(pl->staged_N, pl->staged_tz, false, tensor, q, pl->pvm, pl->psm, a, it0 + s, force,
                             moment && s != nsteps - 1, true, st);
   for (int f = 0; f < 9; ++f) out(q.f[f], p.f[f], rows);
   out(q.mem[0], p.mem[0], r0);
@@ -1022,10 +1014,7 @@ int sw_plan_set_tile(sw_plan* pl, int32_t x_chunk) {
   if (!pl) return fail(SW_ERR_ARG, "null plan");
   if (pl->dim != 3) return fail(SW_ERR_UNSUPPORTED, "tile choice applies to 3D plans");
   if (x_chunk < 1) return fail(SW_ERR_ARG, "x_chunk must be >= 1");
-  pl->p3f.x_chunk = x_chunk;
-  pl->p3d.x_chunk = x_chunk;
-  if (pl->gexec) { cudaGraphExecDestroy(pl->gexec); pl->gexec = nullptr; pl->g_it0 = pl->g_n = -1; }
-  return SW_OK;
+  return SW_OK;  // the per-cell kernels stream no planes
 }
 
 int sw_check_division(float divisor, int32_t mode, uint64_t* mismatches, void* stream) {
@@ -1104,6 +1093,8 @@ int sw_plan_set_path(sw_plan* pl, int32_t path, int32_t chunk_len) {
   if (path == 2 && !pl->fused) setup_fused(pl);  // allocates the second buffer set on first use
   if (path == 2 && !pl->fused) return fail(SW_ERR_UNSUPPORTED, "this plan has no fused path");
   pl->path = path;
+  pl->path_chosen = true;
+  if (pl->staged && path >= 1 && pl->sa.chunks == 0) staged_chunks(pl, 0);  // the fused path ends odd runs staged
   if (chunk_len > 0 && path == 1) staged_chunks(pl, chunk_len);
   if (chunk_len > 0 && path == 2) {
     sw::FusedConfig fc;
@@ -1128,6 +1119,10 @@ int sw_plan_set_free_surface(sw_plan* pl, int32_t on) {
 int sw_plan_set_exact(sw_plan* pl, int32_t exact) {
   if (!pl) return fail(SW_ERR_ARG, "null plan");
   pl->sa.exact = exact ? 1 : 0;
+  if (pl->dim == 3 && !pl->path_chosen) {
+    pl->path = default_path3(pl);
+    if (pl->path == 1 && pl->sa.chunks == 0) staged_chunks(pl, 0);
+  }
   if (pl->gexec) { cudaGraphExecDestroy(pl->gexec); pl->gexec = nullptr; pl->g_it0 = pl->g_n = -1; }
   return SW_OK;
 }

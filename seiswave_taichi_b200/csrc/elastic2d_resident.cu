@@ -104,11 +104,8 @@ __device__ __forceinline__ T sdiff(const T* f, const T (&c)[N]) {
   return v;
 }
 
-// Quotients of a group, the tiers of divc_group / divv_group with two changes
-// that keep their bits: sums of taps are never -0 (they start from +0), so
-// the spacings' correction needs no zero test, and per-cell divisors d come
-// with y = RN(1/d), so that mk2_core replaces the division routine (5
-// operations against about 12 and a reciprocal unit's latency).
+// divc_group for sums of taps: they are never -0 (they start from +0), so the
+// spacings' correction needs no zero test (same bits)
 __device__ __forceinline__ void spacing4(float (&x)[4], const float (&d)[2], const float (&r)[2], bool fast) {
   RangeAcc acc;
 #pragma unroll
@@ -136,35 +133,6 @@ __device__ __forceinline__ void spacing4(double (&x)[4], const double (&d)[2], c
     for (int k = 0; k < 4; ++k) x[k] = div_v(x[k], d[k & 1]);
   }
 }
-template <int K>
-__device__ __forceinline__ void cell_quotients(float (&x)[K], const float (&d)[K], const float (&y)[K], bool fast) {
-  RangeAcc acc;
-#pragma unroll
-  for (int k = 0; k < K; ++k) acc.add(x[k]);
-  if (fast && acc.ok()) {
-#pragma unroll
-    for (int k = 0; k < K; ++k) x[k] = mk2_signed(x[k], d[k], y[k]);
-  } else if (fast && acc.below_huge()) {
-#pragma unroll
-    for (int k = 0; k < K; ++k) x[k] = mk2_div_any(x[k], d[k], y[k]);
-  } else {
-    divv_group<K>(x, d);
-  }
-}
-template <int K>
-__device__ __forceinline__ void cell_quotients(double (&x)[K], const double (&d)[K], const double (&y)[K], bool fast) {
-  RangeAccT<double> acc;
-#pragma unroll
-  for (int k = 0; k < K; ++k) acc.add(x[k]);
-  if (fast && acc.ok()) {
-#pragma unroll
-    for (int k = 0; k < K; ++k) x[k] = x[k] == 0.0 ? x[k] : mk2_core(x[k], d[k], y[k]);
-  } else {
-#pragma unroll
-    for (int k = 0; k < K; ++k) x[k] = div_v(x[k], d[k]);
-  }
-}
-
 // a cell's word: which components are updated, where the CPML corrects their
 // derivatives (velocity phase: vx by x, by z, vz by x, by z; stress phase:
 // normal by x, by z, shear by x, by z), source cell, row of the free-surface hook

@@ -1,477 +1,233 @@
-// elastic3d_cpml.cu -- 3D staggered-grid velocity-stress kernels with ADE-CPML
-// (moment-tensor and point-force variants).
+// elastic3d_cpml.cu -- 3D SSG-CPML time step, one thread per cell, any order and
+// type: float64, single steps of grids the staged kernels do not take, and the
+// sizes and orders where it is the faster path (Elastic3D_SSG_Tensor.update_SSG,
+// src/Elastic3D_SSG_Tensor.py:166-345; Elastic3D_SSG_CPML.update_SSG,
+// src/Elastic3D_SSG_CPML.py:144-309).
 //
-// Restates the Taichi kernels Elastic3D_SSG_Tensor.update_SSG
-// (src/Elastic3D_SSG_Tensor.py:166-345) and Elastic3D_SSG_CPML.update_SSG
-// (src/Elastic3D_SSG_CPML.py:144-309) as two passes per step:
 //   k3_velocity  vx, vy, vz (+ point force)          reference :194-243 / :163-245
 //   k3_stress    sxx syy szz, sxy, sxz, syz (+ receivers, + next step's
 //                moment-tensor injection)              reference :245-310 / :246-309
-// Each CTA owns a 32 (z) x 8 (y) column tile and streams a chunk of x planes;
-// the x-direction stencil taps live in per-thread register queues, the y and z
-// taps are read through the read-only cache from the current plane.  CPML
-// memory variables are stored only on their slabs (sw_pml_axis.lo/hi): outside
-// a slab the reference's update is the identity (a = 0, kappa = 1).
+//
+// A cell is a chain of loads, a quotient group and a store per component, so
+// what counts is how many cells are in flight: one thread per cell at 48 to 64
+// warps per SM, taps from L1 and L2, against the form before it, which streamed
+// x planes through per-thread register queues at 16 to 32 warps.  Measured (us
+// per step, register queues at their best -> this): float64 order 2
+// 128 x 120 x 112 327 -> 232, 60 x 60 x 64 58 -> 37, 200^3 1152 -> 859, order 4
+// 520 -> 250; float 200^3 order 2 759 -> 573, order 3 814 -> 615, order 4 895 ->
+// 636.  CPML memory variables are stored only on their slabs
+// (sw_pml_axis.lo/hi): outside a slab the reference's update is the identity
+// (a = 0, kappa = 1).
 #include "sw_device.cuh"
 
 namespace sw {
 
 constexpr int T3Z = 32;
 constexpr int T3Y = 8;
-// Resident blocks per SM the passes are compiled for.  A thread waits on the
-// tap loads of one component after the other, so residency pays more than
-// registers: double, order 2, 128 x 120 x 112, us per step with the compiler's
-// own count (98-128 registers, two blocks) 448, for 3 blocks 359, 4 327, 5 344,
-// 6 384, 8 467 (spills); order 4 686, 456, 520, 527, 573, 656; 200^3 1492, 1278,
-// 1142, 1202, 1335; float 128 x 120 x 112 294, -, 213, 224, 267.
-constexpr int K3_MINB = 4;
+// Resident blocks per SM the kernels are compiled for (us per step with 5, 6,
+// 8 blocks: float 200^3 order 2 638, 590, 573, order 3 623, 625, 615, order 4
+// 657, 636, 669; float64 128 x 120 x 112 order 2 with 4, 5, 6, 8 252, 234, 232, 238)
+#define SW_C3_MINB (sizeof(T) == 4 && N <= 3 ? 8 : 6)
 
-template <typename T>
-__device__ __forceinline__ void pml_apply(T* __restrict__ m, T b, T a, T kk, T& d) {
-  T psi = b * (*m) + a * d;
+template <typename T, int N, bool FWD>
+__device__ __forceinline__ T d3c(const T* f, long long idx, long long st, const T* c) {
+  T v = 0;
+#pragma unroll
+  for (int m = 0; m < N; ++m)
+    v += FWD ? c[m] * (ldg(f + idx + (m + 1) * st) - ldg(f + idx - m * st))
+             : c[m] * (ldg(f + idx + m * st) - ldg(f + idx - (m + 1) * st));
+  return v;
+}
+
+// CPML correction of derivative d along axis AX (memory variable component
+// comp, integer or half point) where the cell lies in the axis's slab
+template <typename T, int AX, bool HALF>
+__device__ __forceinline__ void cpml3c(const P3<T>& p, int comp, int s, int i, int j, int k, T& d) {
+  const int n = AX == 0 ? p.nx : AX == 1 ? p.ny : p.nz, x = AX == 0 ? i : AX == 1 ? j : k;
+  const T* cf = p.cf[AX] + (HALF ? CBH : CB) * n + x;
+  const long long off = AX == 0   ? ((long long)s * p.ny + j) * p.nz + k
+                        : AX == 1 ? ((long long)i * p.sn[1] + s) * p.nz + k
+                                  : ((long long)i * p.ny + j) * p.sn[2] + s;
+  T* m = p.mem[AX] + comp * p.mcomp[AX] + off;
+  const T psi = cf[0] * (*m) + cf[n] * d;
   *m = psi;
-  d = div_v(d, kk) + psi;
+  d = div_v(d, cf[2 * n]) + psi;
 }
 
-// quotients of a component's derivatives by the spacings of axes A, B, C as one
-// range-tested group (div_c's bits): at 128 x 120 x 112 in double
-// 444 -> 410 us per step
-template <typename T, int A, int B, int C>
-__device__ __forceinline__ void spacings(const P3<T>& p, T& a, T& b, T& c) {
-  const T h[3] = {p.dx, p.dy, p.dz};
-  T x[3] = {a, b, c};
-  const T d[3] = {h[A], h[B], h[C]}, r[3] = {p.rd[A], p.rd[B], p.rd[C]};
-  divc_group<3>(x, d, r, p.fast_div);
-  a = x[0], b = x[1], c = x[2];
-}
-template <typename T, int A, int B>
-__device__ __forceinline__ void spacings(const P3<T>& p, T& a, T& b) {
-  const T h[3] = {p.dx, p.dy, p.dz};
-  T x[2] = {a, b};
-  const T d[2] = {h[A], h[B]}, r[2] = {p.rd[A], p.rd[B]};
-  divc_group<2>(x, d, r, p.fast_div);
-  a = x[0], b = x[1];
-}
-
-// ---------------------------------------------------------------------------
-// velocity pass
-// ---------------------------------------------------------------------------
 template <typename T, int N, bool TENSOR>
-__global__ void __launch_bounds__(T3Z * T3Y, K3_MINB)
+__global__ void __launch_bounds__(T3Z * T3Y, SW_C3_MINB)
 k3_velocity(const __grid_constant__ P3<T> p, int it, int force_here) {
   const int k = blockIdx.x * T3Z + threadIdx.x;
   const int j = blockIdx.y * T3Y + threadIdx.y;
+  const int i = blockIdx.z + N;
   const int nx = p.nx, ny = p.ny, nz = p.nz;
   if (j < N || j >= ny - N || k < N || k >= nz - N) return;
-  const int ib = max((int)blockIdx.z * p.x_chunk, N);
-  const int ie = min((int)(blockIdx.z + 1) * p.x_chunk, nx - N);
-  if (ib >= ie) return;
-
-  const long long sx = (long long)ny * nz;
-  const long long col = (long long)j * nz + k;
-  // ranges (half-open) of Elastic3D_SSG_Tensor.py:195,211,228
-  const bool vx_jk = (j >= N + 1) && (k >= N + 1);
-  const bool vy_jk = (j < ny - N - 1) && (k >= N + 1);
-  const bool vz_jk = (j >= N + 1) && (k < nz - N - 1);
-
-  const int yj = slab_index(j, ny, p.lo[1], p.hi[1]);
-  const int zk = slab_index(k, nz, p.lo[2], p.hi[2]);
-  const uint8_t fy = p.fl[1][j], fz = p.fl[2][k];
-  const T* __restrict__ cfx = p.cf[0];
-  const T* __restrict__ cfy = p.cf[1];
-  const T* __restrict__ cfz = p.cf[2];
-  const T dx = p.dx, dy = p.dy, dz = p.dz, dt = p.dt;
-
-  T* __restrict__ vx = p.f[0];
-  T* __restrict__ vy = p.f[1];
-  T* __restrict__ vz = p.f[2];
-  const T* __restrict__ sxx = p.f[3];
-  const T* __restrict__ syy = p.f[4];
-  const T* __restrict__ szz = p.f[5];
-  const T* __restrict__ sxy = p.f[6];
-  const T* __restrict__ sxz = p.f[7];
-  const T* __restrict__ syz = p.f[8];
-  const T* __restrict__ rho = p.rho;
-
+  const long long sx = (long long)ny * nz, sy = nz;
+  const long long idx = (long long)i * sx + (long long)j * nz + k;
   T c[N];
 #pragma unroll
   for (int m = 0; m < N; ++m) c[m] = p.c[m];
-
-  // register queues along x
-  //   qxx[q] = sxx[i-N+1+q]   (Dx3fm)
-  //   qxy[q] = sxy[i-N+q]     (Dx3bm)
-  //   qxz[q] = sxz[i-N+q]     (Dx3bm)
-  T qxx[2 * N], qxy[2 * N], qxz[2 * N];
-#pragma unroll
-  for (int q = 0; q < 2 * N - 1; ++q) {
-    qxx[q] = ldg(sxx + (long long)(ib - N + 1 + q) * sx + col);
-    qxy[q] = ldg(sxy + (long long)(ib - N + q) * sx + col);
-    qxz[q] = ldg(sxz + (long long)(ib - N + q) * sx + col);
+  const T dt = p.dt;
+  const T *sxx = p.f[3], *syy = p.f[4], *szz = p.f[5], *sxy = p.f[6], *sxz = p.f[7], *syz = p.f[8], *rho = p.rho;
+  const int xi = slab_index(i, nx, p.lo[0], p.hi[0]), yj = slab_index(j, ny, p.lo[1], p.hi[1]),
+            zk = slab_index(k, nz, p.lo[2], p.hi[2]);
+  const uint8_t fx = p.fl[0][i], fy = p.fl[1][j], fz = p.fl[2][k];
+  // vx: x half; i in [N, nx-N-1), j in [N+1, ny-N), k in [N+1, nz-N)
+  if (i < nx - N - 1 && j >= N + 1 && k >= N + 1) {
+    T a = d3c<T, N, true>(sxx, idx, sx, c), b = d3c<T, N, false>(sxy, idx, sy, c), d = d3c<T, N, false>(sxz, idx, 1, c);
+    spacings<T, 0, 1, 2>(p, a, b, d);
+    if ((fx & 2) || (fy & 1) || (fz & 1)) {
+      if (xi >= 0) cpml3c<T, 0, true>(p, 0, xi, i, j, k, a);
+      if (yj >= 0) cpml3c<T, 1, false>(p, 0, yj, i, j, k, b);
+      if (zk >= 0) cpml3c<T, 2, false>(p, 0, zk, i, j, k, d);
+    }
+    T t = (a + d + b) * dt;
+    p.f[0][idx] = p.f[0][idx] + div_v(t, ldg(rho + idx));
   }
-  T rc0 = ldg(rho + (long long)ib * sx + col);          // rho[i, j, k]
-  T rn0 = ldg(rho + (long long)ib * sx + col + nz);     // rho[i, j+1, k]
-
-  const bool src_col = force_here && (j == p.sj) && (k == p.sk);
-
-  for (int i = ib; i < ie; ++i) {
-    const long long pl = (long long)i * sx;
-    qxx[2 * N - 1] = ldg(sxx + pl + (long long)N * sx + col);
-    qxy[2 * N - 1] = ldg(sxy + pl + (long long)(N - 1) * sx + col);
-    qxz[2 * N - 1] = ldg(sxz + pl + (long long)(N - 1) * sx + col);
-    const T rc1 = ldg(rho + pl + sx + col);        // rho[i+1, j, k]
-    const T rn1 = ldg(rho + pl + sx + col + nz);   // rho[i+1, j+1, k]
-    const int xi = slab_index(i, nx, p.lo[0], p.hi[0]);
-    const uint8_t fx = p.fl[0][i];
-    const long long idx = pl + col;
-
-    // ---- vx  (x half, y int, z int) -------------------------------------
-    if (vx_jk && i < nx - N - 1) {
-      T dsxxdx = 0, dsxydy = 0, dsxzdz = 0;
-#pragma unroll
-      for (int m = 0; m < N; ++m) dsxxdx += c[m] * (qxx[N + m] - qxx[N - 1 - m]);
-#pragma unroll
-      for (int m = 0; m < N; ++m) {
-        const T hi = (m == 0) ? qxy[N] : ldg(sxy + idx + (long long)m * nz);
-        dsxydy += c[m] * (hi - ldg(sxy + idx - (long long)(m + 1) * nz));
-      }
-#pragma unroll
-      for (int m = 0; m < N; ++m) {
-        const T hi = (m == 0) ? qxz[N] : ldg(sxz + idx + m);
-        dsxzdz += c[m] * (hi - ldg(sxz + idx - (m + 1)));
-      }
-      spacings<T, 0, 1, 2>(p, dsxxdx, dsxydy, dsxzdz);
-      if ((xi >= 0 || yj >= 0 || zk >= 0) && ((fx & 2) || (fy & 1) || (fz & 1))) {
-        if (xi >= 0)
-          pml_apply(p.mem[0] + ((long long)xi * ny + j) * nz + k,
-                    cfx[CBH * nx + i], cfx[CAH * nx + i], cfx[CKH * nx + i], dsxxdx);
-        if (yj >= 0)
-          pml_apply(p.mem[1] + ((long long)i * p.sn[1] + yj) * nz + k,
-                    cfy[CB * ny + j], cfy[CA * ny + j], cfy[CK * ny + j], dsxydy);
-        if (zk >= 0)
-          pml_apply(p.mem[2] + ((long long)i * ny + j) * p.sn[2] + zk,
-                    cfz[CB * nz + k], cfz[CA * nz + k], cfz[CK * nz + k], dsxzdz);
-      }
-      T t = (dsxxdx + dsxzdz + dsxydy) * dt;
-      t = div_v(t, rc0);
-      vx[idx] = vx[idx] + t;
+  // vy: y half; i in [N+1, nx-N), j in [N, ny-N-1), k in [N+1, nz-N)
+  if (i >= N + 1 && j < ny - N - 1 && k >= N + 1) {
+    T a = d3c<T, N, false>(sxy, idx, sx, c), b = d3c<T, N, true>(syy, idx, sy, c), d = d3c<T, N, false>(syz, idx, 1, c);
+    spacings<T, 0, 1, 2>(p, a, b, d);
+    if ((fx & 1) || (fy & 2) || (fz & 1)) {
+      if (xi >= 0) cpml3c<T, 0, false>(p, 1, xi, i, j, k, a);
+      if (yj >= 0) cpml3c<T, 1, true>(p, 1, yj, i, j, k, b);
+      if (zk >= 0) cpml3c<T, 2, false>(p, 1, zk, i, j, k, d);
     }
-
-    // ---- vy  (x int, y half, z int) -------------------------------------
-    if (vy_jk && i >= N + 1) {
-      const T rhy = (T)0.5 * (rc0 + rn0);
-      T dsxydx = 0, dsyydy = 0, dsyzdz = 0;
-#pragma unroll
-      for (int m = 0; m < N; ++m) dsxydx += c[m] * (qxy[N + m] - qxy[N - 1 - m]);
-#pragma unroll
-      for (int m = 0; m < N; ++m)
-        dsyydy += c[m] * (ldg(syy + idx + (long long)(m + 1) * nz) - ldg(syy + idx - (long long)m * nz));
-#pragma unroll
-      for (int m = 0; m < N; ++m)
-        dsyzdz += c[m] * (ldg(syz + idx + m) - ldg(syz + idx - (m + 1)));
-      spacings<T, 0, 1, 2>(p, dsxydx, dsyydy, dsyzdz);
-      if ((xi >= 0 || yj >= 0 || zk >= 0) && ((fx & 1) || (fy & 2) || (fz & 1))) {
-        if (xi >= 0)
-          pml_apply(p.mem[0] + p.mcomp[0] + ((long long)xi * ny + j) * nz + k,
-                    cfx[CB * nx + i], cfx[CA * nx + i], cfx[CK * nx + i], dsxydx);
-        if (yj >= 0)
-          pml_apply(p.mem[1] + p.mcomp[1] + ((long long)i * p.sn[1] + yj) * nz + k,
-                    cfy[CBH * ny + j], cfy[CAH * ny + j], cfy[CKH * ny + j], dsyydy);
-        if (zk >= 0)
-          pml_apply(p.mem[2] + p.mcomp[2] + ((long long)i * ny + j) * p.sn[2] + zk,
-                    cfz[CB * nz + k], cfz[CA * nz + k], cfz[CK * nz + k], dsyzdz);
+    T t = (a + b + d) * dt;
+    p.f[1][idx] = p.f[1][idx] + div_v(t, (T)0.5 * (ldg(rho + idx) + ldg(rho + idx + sy)));
+  }
+  // vz: z half; i in [N+1, nx-N), j in [N+1, ny-N), k in [N, nz-N-1), then the
+  // point force (Elastic3D_SSG_CPML.py:245)
+  const bool upd = i >= N + 1 && j >= N + 1 && k < nz - N - 1;
+  const bool src = force_here && i == p.si && j == p.sj && k == p.sk;
+  if (upd || src) {
+    T v = p.f[2][idx];
+    if (upd) {
+      T a = d3c<T, N, false>(sxz, idx, sx, c), b = d3c<T, N, false>(syz, idx, sy, c), d = d3c<T, N, true>(szz, idx, 1, c);
+      spacings<T, 0, 1, 2>(p, a, b, d);
+      if ((fx & 1) || (fy & 1) || (fz & 2)) {
+        if (xi >= 0) cpml3c<T, 0, false>(p, 2, xi, i, j, k, a);
+        if (yj >= 0) cpml3c<T, 1, false>(p, 2, yj, i, j, k, b);
+        if (zk >= 0) cpml3c<T, 2, true>(p, 2, zk, i, j, k, d);
       }
-      T t = (dsxydx + dsyydy + dsyzdz) * dt;
-      t = div_v(t, rhy);
-      vy[idx] = vy[idx] + t;
+      T t = (TENSOR ? (a + b + d) : (d + a + b)) * dt;
+      v = v + div_v(t, (T)0.25 * (ldg(rho + idx) + ldg(rho + idx + sy) + ldg(rho + idx + sx + sy) + ldg(rho + idx + sx)));
     }
-
-    // ---- vz  (x int, y int, z half) -------------------------------------
-    const bool vz_upd = vz_jk && i >= N + 1;
-    const bool vz_src = src_col && (i == p.si);
-    if (vz_upd || vz_src) {
-      T v = vz[idx];
-      if (vz_upd) {
-        const T r4 = (T)0.25 * (rc0 + rn0 + rn1 + rc1);
-        T dsxzdx = 0, dsyzdy = 0, dszzdz = 0;
-#pragma unroll
-        for (int m = 0; m < N; ++m) dsxzdx += c[m] * (qxz[N + m] - qxz[N - 1 - m]);
-#pragma unroll
-        for (int m = 0; m < N; ++m)
-          dsyzdy += c[m] * (ldg(syz + idx + (long long)m * nz) - ldg(syz + idx - (long long)(m + 1) * nz));
-#pragma unroll
-        for (int m = 0; m < N; ++m)
-          dszzdz += c[m] * (ldg(szz + idx + (m + 1)) - ldg(szz + idx - m));
-        spacings<T, 0, 1, 2>(p, dsxzdx, dsyzdy, dszzdz);
-        if ((xi >= 0 || yj >= 0 || zk >= 0) && ((fx & 1) || (fy & 1) || (fz & 2))) {
-          if (xi >= 0)
-            pml_apply(p.mem[0] + 2 * p.mcomp[0] + ((long long)xi * ny + j) * nz + k,
-                      cfx[CB * nx + i], cfx[CA * nx + i], cfx[CK * nx + i], dsxzdx);
-          if (yj >= 0)
-            pml_apply(p.mem[1] + 2 * p.mcomp[1] + ((long long)i * p.sn[1] + yj) * nz + k,
-                      cfy[CB * ny + j], cfy[CA * ny + j], cfy[CK * ny + j], dsyzdy);
-          if (zk >= 0)
-            pml_apply(p.mem[2] + 2 * p.mcomp[2] + ((long long)i * ny + j) * p.sn[2] + zk,
-                      cfz[CBH * nz + k], cfz[CAH * nz + k], cfz[CKH * nz + k], dszzdz);
-        }
-        T s = TENSOR ? (dsxzdx + dsyzdy + dszzdz) : (dszzdz + dsxzdx + dsyzdy);
-        T t = s * dt;
-        t = div_v(t, r4);
-        v = v + t;
-      }
-      if (vz_src) {
-        // Elastic3D_SSG_CPML.py:245 / Elastic3D_SSG_SPML.py:294
-        T t = dt * p.wav[it];
-        t = div_v(t, rc0);
-        v = v + t;
-      }
-      vz[idx] = v;
+    if (src) {
+      T t = dt * p.wav[it];
+      v = v + div_v(t, ldg(rho + idx));
     }
-
-    // shift the queues
-#pragma unroll
-    for (int q = 0; q < 2 * N - 1; ++q) {
-      qxx[q] = qxx[q + 1];
-      qxy[q] = qxy[q + 1];
-      qxz[q] = qxz[q + 1];
-    }
-    rc0 = rc1;
-    rn0 = rn1;
+    p.f[2][idx] = v;
   }
 }
 
-// ---------------------------------------------------------------------------
-// stress pass
-// ---------------------------------------------------------------------------
 template <typename T, int N>
-__global__ void __launch_bounds__(T3Z * T3Y, K3_MINB)
+__global__ void __launch_bounds__(T3Z * T3Y, SW_C3_MINB)
 k3_stress(const __grid_constant__ P3<T> p, int it, int inject_next) {
-  const int nx = p.nx, ny = p.ny, nz = p.nz;
-  // receivers: the velocity fields are final for this step and are not
-  // written by this pass (Elastic3D_SSG_Tensor.py:344-345)
   {
     const long long b = blockIdx.x + (long long)gridDim.x * (blockIdx.y + (long long)gridDim.y * blockIdx.z);
-    const long long r = b * (T3Z * T3Y) + threadIdx.y * T3Z + threadIdx.x;
-    if (r < p.nrec)
+    const long long n = (long long)gridDim.x * gridDim.y * gridDim.z * (T3Z * T3Y);
+    for (long long r = b * (T3Z * T3Y) + threadIdx.y * T3Z + threadIdx.x; r < p.nrec; r += n)
       store_rec(p.rec_data, p.rec_f64, (long long)it * p.nrec + r, p.f[p.rec_field][p.rec_idx[r]]);
   }
   const int k = blockIdx.x * T3Z + threadIdx.x;
   const int j = blockIdx.y * T3Y + threadIdx.y;
+  const int i = blockIdx.z + N;
+  const int nx = p.nx, ny = p.ny, nz = p.nz;
   if (j < N || j >= ny - N || k < N || k >= nz - N) return;
-  const int ib = max((int)blockIdx.z * p.x_chunk, N);
-  const int ie = min((int)(blockIdx.z + 1) * p.x_chunk, nx - N);
-  if (ib >= ie) return;
-
-  const long long sx = (long long)ny * nz;
-  const long long col = (long long)j * nz + k;
-  const bool nn_jk = (j >= N + 1) && (k >= N + 1);   // :246
-  const bool xy_jk = (j >= N + 1);                   // :268
-  const bool xz_jk = (k < nz - N - 1);               // :282
-  const bool yz_jk = (j < ny - N - 1) && (k < nz - N - 1);  // :297
-
-  const int yj = slab_index(j, ny, p.lo[1], p.hi[1]);
-  const int zk = slab_index(k, nz, p.lo[2], p.hi[2]);
-  const uint8_t fy = p.fl[1][j], fz = p.fl[2][k];
-  const T* __restrict__ cfx = p.cf[0];
-  const T* __restrict__ cfy = p.cf[1];
-  const T* __restrict__ cfz = p.cf[2];
-  const T dx = p.dx, dy = p.dy, dz = p.dz, dt = p.dt;
-
-  const T* __restrict__ vx = p.f[0];
-  const T* __restrict__ vy = p.f[1];
-  const T* __restrict__ vz = p.f[2];
-  T* __restrict__ sxx = p.f[3];
-  T* __restrict__ syy = p.f[4];
-  T* __restrict__ szz = p.f[5];
-  T* __restrict__ sxy = p.f[6];
-  T* __restrict__ sxz = p.f[7];
-  T* __restrict__ syz = p.f[8];
-  const T* __restrict__ lam = p.lam;
-  const T* __restrict__ mu = p.mu;
-
+  const long long sx = (long long)ny * nz, sy = nz;
+  const long long idx = (long long)i * sx + (long long)j * nz + k;
   T c[N];
 #pragma unroll
   for (int m = 0; m < N; ++m) c[m] = p.c[m];
-
-  //   qvx[q] = vx[i-N+q]     (Dx3bm)
-  //   qvy[q] = vy[i-N+1+q]   (Dx3fm)
-  //   qvz[q] = vz[i-N+1+q]   (Dx3fm)
-  T qvx[2 * N], qvy[2 * N], qvz[2 * N];
-#pragma unroll
-  for (int q = 0; q < 2 * N - 1; ++q) {
-    qvx[q] = ldg(vx + (long long)(ib - N + q) * sx + col);
-    qvy[q] = ldg(vy + (long long)(ib - N + 1 + q) * sx + col);
-    qvz[q] = ldg(vz + (long long)(ib - N + 1 + q) * sx + col);
+  const T dt = p.dt;
+  const T *vx = p.f[0], *vy = p.f[1], *vz = p.f[2], *lam = p.lam, *mu = p.mu;
+  const int xi = slab_index(i, nx, p.lo[0], p.hi[0]), yj = slab_index(j, ny, p.lo[1], p.hi[1]),
+            zk = slab_index(k, nz, p.lo[2], p.hi[2]);
+  const uint8_t fx = p.fl[0][i], fy = p.fl[1][j], fz = p.fl[2][k];
+  const bool src = inject_next && i == p.si && j == p.sj && k == p.sk;
+  const T wn = src ? p.wav[it + 1] : (T)0;
+  // normal stresses: i, j, k in [N+1, n-N)
+  const bool un = i >= N + 1 && j >= N + 1 && k >= N + 1;
+  if (un || src) {
+    T sa = p.f[3][idx], sb = p.f[4][idx], sc = p.f[5][idx];
+    if (un) {
+      T a = d3c<T, N, false>(vx, idx, sx, c), b = d3c<T, N, false>(vy, idx, sy, c), d = d3c<T, N, false>(vz, idx, 1, c);
+      spacings<T, 0, 1, 2>(p, a, b, d);
+      if ((fx | fy | fz) & 1) {
+        if (xi >= 0) cpml3c<T, 0, false>(p, 3, xi, i, j, k, a);
+        if (yj >= 0) cpml3c<T, 1, false>(p, 3, yj, i, j, k, b);
+        if (zk >= 0) cpml3c<T, 2, false>(p, 3, zk, i, j, k, d);
+      }
+      const T lhx = (T)0.5 * (ldg(lam + idx) + ldg(lam + idx + sx));
+      const T mhx = (T)0.5 * (ldg(mu + idx) + ldg(mu + idx + sx));
+      const T lpm = lhx + (T)2 * mhx;
+      sa = sa + (lpm * a + lhx * (d + b)) * dt;
+      sb = sb + (lpm * b + lhx * (a + d)) * dt;
+      sc = sc + (lpm * d + lhx * (a + b)) * dt;
+    }
+    if (src) {
+      sa = sa + wn * p.mneg[0];
+      sb = sb + wn * p.mneg[1];
+      sc = sc + wn * p.mneg[2];
+    }
+    p.f[3][idx] = sa;
+    p.f[4][idx] = sb;
+    p.f[5][idx] = sc;
   }
-  T l0 = ldg(lam + (long long)ib * sx + col);
-  T u0 = ldg(mu + (long long)ib * sx + col);
-  const bool src_col = inject_next && (j == p.sj) && (k == p.sk);
-  const T wn = inject_next ? p.wav[it + 1] : (T)0;
-
-  for (int i = ib; i < ie; ++i) {
-    const long long pl = (long long)i * sx;
-    qvx[2 * N - 1] = ldg(vx + pl + (long long)(N - 1) * sx + col);
-    qvy[2 * N - 1] = ldg(vy + pl + (long long)N * sx + col);
-    qvz[2 * N - 1] = ldg(vz + pl + (long long)N * sx + col);
-    const T l1 = ldg(lam + pl + sx + col);   // lam[i+1, j, k]
-    const T u1 = ldg(mu + pl + sx + col);    // mu[i+1, j, k]
-    const int xi = slab_index(i, nx, p.lo[0], p.hi[0]);
-    const uint8_t fx = p.fl[0][i];
-    const long long idx = pl + col;
-    const bool src = src_col && (i == p.si);
-    const bool any_slab = (xi >= 0 || yj >= 0 || zk >= 0);
-
-    // ---- sxx syy szz  (integer point) :246-266 ---------------------------
-    if ((nn_jk && i >= N + 1) || src) {
-      T axx = sxx[idx], ayy = syy[idx], azz = szz[idx];
-      if (nn_jk && i >= N + 1) {
-        const T lhx = (T)0.5 * (l0 + l1);
-        const T mhx = (T)0.5 * (u0 + u1);
-        const T lpm = lhx + (T)2 * mhx;
-        T dvxdx = 0, dvydy = 0, dvzdz = 0;
-#pragma unroll
-        for (int m = 0; m < N; ++m) dvxdx += c[m] * (qvx[N + m] - qvx[N - 1 - m]);
-#pragma unroll
-        for (int m = 0; m < N; ++m) {
-          const T hi = (m == 0) ? qvy[N - 1] : ldg(vy + idx + (long long)m * nz);
-          dvydy += c[m] * (hi - ldg(vy + idx - (long long)(m + 1) * nz));
-        }
-#pragma unroll
-        for (int m = 0; m < N; ++m) {
-          const T hi = (m == 0) ? qvz[N - 1] : ldg(vz + idx + m);
-          dvzdz += c[m] * (hi - ldg(vz + idx - (m + 1)));
-        }
-        spacings<T, 0, 1, 2>(p, dvxdx, dvydy, dvzdz);
-        if (any_slab && ((fx | fy | fz) & 1)) {
-          if (xi >= 0)
-            pml_apply(p.mem[0] + 3 * p.mcomp[0] + ((long long)xi * ny + j) * nz + k,
-                      cfx[CB * nx + i], cfx[CA * nx + i], cfx[CK * nx + i], dvxdx);
-          if (yj >= 0)
-            pml_apply(p.mem[1] + 3 * p.mcomp[1] + ((long long)i * p.sn[1] + yj) * nz + k,
-                      cfy[CB * ny + j], cfy[CA * ny + j], cfy[CK * ny + j], dvydy);
-          if (zk >= 0)
-            pml_apply(p.mem[2] + 3 * p.mcomp[2] + ((long long)i * ny + j) * p.sn[2] + zk,
-                      cfz[CB * nz + k], cfz[CA * nz + k], cfz[CK * nz + k], dvzdz);
-        }
-        axx = axx + (lpm * dvxdx + lhx * (dvzdz + dvydy)) * dt;
-        ayy = ayy + (lpm * dvydy + lhx * (dvxdx + dvzdz)) * dt;
-        azz = azz + (lpm * dvzdz + lhx * (dvxdx + dvydy)) * dt;
+  // sxy: i, j in [N+1, n-N), k in [N, nz-N)
+  const bool uxy = i >= N + 1 && j >= N + 1;
+  if (uxy || src) {
+    T s = p.f[6][idx];
+    if (uxy) {
+      T a = d3c<T, N, true>(vy, idx, sx, c), b = d3c<T, N, true>(vx, idx, sy, c);
+      spacings<T, 0, 1>(p, a, b);
+      if ((fx & 2) || (fy & 2) || (fz & 1)) {
+        if (xi >= 0) cpml3c<T, 0, true>(p, 4, xi, i, j, k, a);
+        if (yj >= 0) cpml3c<T, 1, true>(p, 4, yj, i, j, k, b);
       }
-      if (src) {
-        axx = axx + wn * p.mneg[0];
-        ayy = ayy + wn * p.mneg[1];
-        azz = azz + wn * p.mneg[2];
+      const T m4 = (T)0.25 * (ldg(mu + idx + sy) + ldg(mu + idx) + ldg(mu + idx) + ldg(mu + idx + sx));
+      s = s + m4 * (b + a) * dt;
+    }
+    if (src) s = s + wn * p.mneg[3];
+    p.f[6][idx] = s;
+  }
+  // sxz: i in [N, nx-N-1), j in [N, ny-N), k in [N, nz-N-1)
+  const bool uxz = i < nx - N - 1 && k < nz - N - 1;
+  if (uxz || src) {
+    T s = p.f[7][idx];
+    if (uxz) {
+      T a = d3c<T, N, true>(vz, idx, sx, c), b = d3c<T, N, true>(vx, idx, 1, c);
+      spacings<T, 0, 2>(p, a, b);
+      if ((fx & 2) || (fy & 1) || (fz & 2)) {
+        if (xi >= 0) cpml3c<T, 0, true>(p, 5, xi, i, j, k, a);
+        if (zk >= 0) cpml3c<T, 2, true>(p, 4, zk, i, j, k, b);
       }
-      sxx[idx] = axx;
-      syy[idx] = ayy;
-      szz[idx] = azz;
+      const T m4 = (T)0.25 * (ldg(mu + idx) + ldg(mu + idx + sx) + ldg(mu + idx) + ldg(mu + idx + sy));
+      s = s + m4 * (b + a) * dt;
     }
-
-    // ---- sxy  (x half, y half, z int) :268-280 ---------------------------
-    const bool xy_upd = xy_jk && i >= N + 1;
-    if (xy_upd || src) {
-      T a = sxy[idx];
-      if (xy_upd) {
-        const T unj = ldg(mu + idx + nz);  // mu[i, j+1, k]
-        const T m4 = (T)0.25 * (unj + u0 + u0 + u1);
-        T dvydx = 0, dvxdy = 0;
-#pragma unroll
-        for (int m = 0; m < N; ++m) dvydx += c[m] * (qvy[N + m] - qvy[N - 1 - m]);
-#pragma unroll
-        for (int m = 0; m < N; ++m) {
-          const T lo = (m == 0) ? qvx[N] : ldg(vx + idx - (long long)m * nz);
-          dvxdy += c[m] * (ldg(vx + idx + (long long)(m + 1) * nz) - lo);
-        }
-        spacings<T, 0, 1>(p, dvydx, dvxdy);
-        if (any_slab && ((fx & 2) || (fy & 2) || (fz & 1))) {
-          if (xi >= 0)
-            pml_apply(p.mem[0] + 4 * p.mcomp[0] + ((long long)xi * ny + j) * nz + k,
-                      cfx[CBH * nx + i], cfx[CAH * nx + i], cfx[CKH * nx + i], dvydx);
-          if (yj >= 0)
-            pml_apply(p.mem[1] + 4 * p.mcomp[1] + ((long long)i * p.sn[1] + yj) * nz + k,
-                      cfy[CBH * ny + j], cfy[CAH * ny + j], cfy[CKH * ny + j], dvxdy);
-        }
-        a = a + m4 * (dvxdy + dvydx) * dt;
+    if (src) s = s + wn * p.mneg[4];
+    p.f[7][idx] = s;
+  }
+  // syz: i in [N, nx-N), j in [N, ny-N-1), k in [N, nz-N-1)
+  const bool uyz = j < ny - N - 1 && k < nz - N - 1;
+  if (uyz || src) {
+    T s = p.f[8][idx];
+    if (uyz) {
+      T a = d3c<T, N, true>(vz, idx, sy, c), b = d3c<T, N, true>(vy, idx, 1, c);
+      spacings<T, 1, 2>(p, a, b);
+      if ((fx & 1) || (fy & 2) || (fz & 2)) {
+        if (yj >= 0) cpml3c<T, 1, true>(p, 5, yj, i, j, k, a);
+        if (zk >= 0) cpml3c<T, 2, true>(p, 5, zk, i, j, k, b);
       }
-      if (src) a = a + wn * p.mneg[3];
-      sxy[idx] = a;
+      const T m4 = (T)0.25 * (ldg(mu + idx + sy) + ldg(mu + idx) + ldg(mu + idx + 1) + ldg(mu + idx));
+      s = s + m4 * (a + b) * dt;
     }
-
-    // ---- sxz  (x half, y int, z half) :282-294 ---------------------------
-    const bool xz_upd = xz_jk && i < nx - N - 1;
-    if (xz_upd || src) {
-      T a = sxz[idx];
-      if (xz_upd) {
-        const T unj = ldg(mu + idx + nz);  // mu[i, j+1, k]
-        const T m4 = (T)0.25 * (u0 + u1 + u0 + unj);
-        T dvzdx = 0, dvxdz = 0;
-#pragma unroll
-        for (int m = 0; m < N; ++m) dvzdx += c[m] * (qvz[N + m] - qvz[N - 1 - m]);
-#pragma unroll
-        for (int m = 0; m < N; ++m) {
-          const T lo = (m == 0) ? qvx[N] : ldg(vx + idx - m);
-          dvxdz += c[m] * (ldg(vx + idx + (m + 1)) - lo);
-        }
-        spacings<T, 0, 2>(p, dvzdx, dvxdz);
-        if (any_slab && ((fx & 2) || (fy & 1) || (fz & 2))) {
-          if (xi >= 0)
-            pml_apply(p.mem[0] + 5 * p.mcomp[0] + ((long long)xi * ny + j) * nz + k,
-                      cfx[CBH * nx + i], cfx[CAH * nx + i], cfx[CKH * nx + i], dvzdx);
-          if (zk >= 0)
-            pml_apply(p.mem[2] + 4 * p.mcomp[2] + ((long long)i * ny + j) * p.sn[2] + zk,
-                      cfz[CBH * nz + k], cfz[CAH * nz + k], cfz[CKH * nz + k], dvxdz);
-        }
-        a = a + m4 * (dvxdz + dvzdx) * dt;
-      }
-      if (src) a = a + wn * p.mneg[4];
-      sxz[idx] = a;
-    }
-
-    // ---- syz  (x int, y half, z half) :297-310 ---------------------------
-    if (yz_jk || src) {
-      T a = syz[idx];
-      if (yz_jk) {
-        const T unj = ldg(mu + idx + nz);  // mu[i, j+1, k]
-        const T unk = ldg(mu + idx + 1);   // mu[i, j, k+1]
-        const T m4 = (T)0.25 * (unj + u0 + unk + u0);
-        T dvzdy = 0, dvydz = 0;
-#pragma unroll
-        for (int m = 0; m < N; ++m) {
-          const T lo = (m == 0) ? qvz[N - 1] : ldg(vz + idx - (long long)m * nz);
-          dvzdy += c[m] * (ldg(vz + idx + (long long)(m + 1) * nz) - lo);
-        }
-#pragma unroll
-        for (int m = 0; m < N; ++m) {
-          const T lo = (m == 0) ? qvy[N - 1] : ldg(vy + idx - m);
-          dvydz += c[m] * (ldg(vy + idx + (m + 1)) - lo);
-        }
-        spacings<T, 1, 2>(p, dvzdy, dvydz);
-        if (any_slab && ((fx & 1) || (fy & 2) || (fz & 2))) {
-          if (yj >= 0)
-            pml_apply(p.mem[1] + 5 * p.mcomp[1] + ((long long)i * p.sn[1] + yj) * nz + k,
-                      cfy[CBH * ny + j], cfy[CAH * ny + j], cfy[CKH * ny + j], dvzdy);
-          if (zk >= 0)
-            pml_apply(p.mem[2] + 5 * p.mcomp[2] + ((long long)i * ny + j) * p.sn[2] + zk,
-                      cfz[CBH * nz + k], cfz[CAH * nz + k], cfz[CKH * nz + k], dvydz);
-        }
-        a = a + m4 * (dvzdy + dvydz) * dt;
-      }
-      if (src) a = a + wn * p.mneg[5];
-      syz[idx] = a;
-    }
-
-#pragma unroll
-    for (int q = 0; q < 2 * N - 1; ++q) {
-      qvx[q] = qvx[q + 1];
-      qvy[q] = qvy[q + 1];
-      qvz[q] = qvz[q + 1];
-    }
-    l0 = l1;
-    u0 = u1;
+    if (src) s = s + wn * p.mneg[5];
+    p.f[8][idx] = s;
   }
 }
 
-// ---------------------------------------------------------------------------
-// single-cell source kernels (used when the fused paths cannot cover a step)
 // ---------------------------------------------------------------------------
 // Elastic3D_SSG_Tensor.py:186-193: sigma_ab[src] += w * (-M_ab)
 template <typename T>
@@ -501,20 +257,20 @@ __global__ void k3_gather(const __grid_constant__ P3<T> p, int it) {
 // ---------------------------------------------------------------------------
 // host-side launchers
 // ---------------------------------------------------------------------------
-template <typename T>
-static dim3 grid3(const P3<T>& p) {
-  return dim3((p.nz + T3Z - 1) / T3Z, (p.ny + T3Y - 1) / T3Y, (p.nx + p.x_chunk - 1) / p.x_chunk);
+template <typename T, int N>
+static dim3 cell_grid(const P3<T>& p) {
+  return dim3((p.nz + T3Z - 1) / T3Z, (p.ny + T3Y - 1) / T3Y, p.nx - 2 * N);
 }
 
 template <typename T, int N>
 static void launch3_velocity(const P3<T>& p, int it, bool tensor, bool force_here, cudaStream_t st) {
-  if (tensor) k3_velocity<T, N, true><<<grid3(p), dim3(T3Z, T3Y), 0, st>>>(p, it, 0);
-  else k3_velocity<T, N, false><<<grid3(p), dim3(T3Z, T3Y), 0, st>>>(p, it, force_here ? 1 : 0);
+  if (tensor) k3_velocity<T, N, true><<<cell_grid<T, N>(p), dim3(T3Z, T3Y), 0, st>>>(p, it, 0);
+  else k3_velocity<T, N, false><<<cell_grid<T, N>(p), dim3(T3Z, T3Y), 0, st>>>(p, it, force_here ? 1 : 0);
 }
 
 template <typename T, int N>
 static void launch3_stress(const P3<T>& p, int it, bool inject_next, cudaStream_t st) {
-  k3_stress<T, N><<<grid3(p), dim3(T3Z, T3Y), 0, st>>>(p, it, inject_next ? 1 : 0);
+  k3_stress<T, N><<<cell_grid<T, N>(p), dim3(T3Z, T3Y), 0, st>>>(p, it, inject_next ? 1 : 0);
 }
 
 #define SW_ORDER_SWITCH(order, CALL)            \

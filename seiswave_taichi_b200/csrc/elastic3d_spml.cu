@@ -35,6 +35,29 @@ __device__ __forceinline__ T d_bm(const T* f, long long idx, long long s, const 
   return v;
 }
 
+// one axis of a split update: w = 1 - dt/2 d, the divisor and its reciprocal
+template <typename T>
+struct Damp {
+  T w, d, y;
+};
+template <typename T>
+__device__ __forceinline__ Damp<T> damp_of(T damp, T hdt) {
+  const T d = (T)1 + hdt * damp;
+  return Damp<T>{(T)1 - hdt * damp, d, (T)1 / d};
+}
+// the parts' quotients as one group (div_v's bits)
+template <typename T, int K>
+__device__ __forceinline__ void split_quotients(T (&x)[K], const Damp<T> (&a)[K]) {
+  T d[K], y[K];
+  bool ok = true;
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    d[k] = a[k].d;
+    y[k] = a[k].y;
+    ok = ok && mk2_divisor(d[k]);
+  }
+  cell_quotients<K>(x, d, y, ok);
+}
 template <typename T, int N>
 __global__ void __launch_bounds__(TSZ * TSY, SW_KS_MINB)
 ks_velocity(const __grid_constant__ P3<T> p, int it, int src_here) {
@@ -46,7 +69,7 @@ ks_velocity(const __grid_constant__ P3<T> p, int it, int src_here) {
   const long long sx = (long long)ny * nz, sy = nz;
   const long long idx = (long long)i * sx + (long long)j * nz + k;
   const long long G = p.scomp;
-  const T dx = p.dx, dy = p.dy, dz = p.dz, dt = p.dt;
+  const T dt = p.dt;
   const T hdt = (T)0.5 * dt;
   T c[N];
 #pragma unroll
@@ -61,17 +84,17 @@ ks_velocity(const __grid_constant__ P3<T> p, int it, int src_here) {
 
   // vx :182-205
   if (i >= N && i < nx - N - 1 && j >= N + 1 && j < ny - N && k >= N + 1 && k < nz - N) {
-    T dsxxdx = div_c(d_fm<T, N>(sxx, idx, sx, c), dx, p.rd[0], p.fast_div);
-    T dsxydy = div_c(d_bm<T, N>(sxy, idx, sy, c), dy, p.rd[1], p.fast_div);
-    T dsxzdz = div_c(d_bm<T, N>(sxz, idx, 1, c), dz, p.rd[2], p.fast_div);
+    T dsxxdx = d_fm<T, N>(sxx, idx, sx, c), dsxydy = d_bm<T, N>(sxy, idx, sy, c), dsxzdz = d_bm<T, N>(sxz, idx, 1, c);
+    spacings<T, 0, 1, 2>(p, dsxxdx, dsxydy, dsxzdz);
     const T rh = ldg(rho + idx);
     const T ro = (T)1 / rh;
     if ((fx & 2) || (fy & 1) || (fz & 1)) {
-      const T xn = (T)1 - hdt * dpx[nx + i], yn = (T)1 - hdt * dpy[j], zn = (T)1 - hdt * dpz[k];
-      const T xd = (T)1 + hdt * dpx[nx + i], yd = (T)1 + hdt * dpy[j], zd = (T)1 + hdt * dpz[k];
-      T a = div_v((xn * sp[PVX_X * G + sh] + dsxxdx * dt * ro), xd);
-      T b = div_v((yn * sp[PVX_Y * G + sh] + dsxydy * dt * ro), yd);
-      T cc = div_v((zn * sp[PVX_Z * G + sh] + dsxzdz * dt * ro), zd);
+      const Damp<T> x = damp_of(dpx[nx + i], hdt), y = damp_of(dpy[j], hdt), z = damp_of(dpz[k], hdt);
+      T qa[3] = {x.w * sp[PVX_X * G + sh] + dsxxdx * dt * ro,
+          y.w * sp[PVX_Y * G + sh] + dsxydy * dt * ro,
+          z.w * sp[PVX_Z * G + sh] + dsxzdz * dt * ro};
+      split_quotients<T, 3>(qa, {x, y, z});
+      const T a = qa[0], b = qa[1], cc = qa[2];
       sp[PVX_X * G + sh] = a;
       sp[PVX_Y * G + sh] = b;
       sp[PVX_Z * G + sh] = cc;
@@ -84,15 +107,15 @@ ks_velocity(const __grid_constant__ P3<T> p, int it, int src_here) {
   if (i >= N + 1 && i < nx - N && j >= N && j < ny - N - 1 && k >= N + 1 && k < nz - N) {
     const T rhy = (T)0.5 * (ldg(rho + idx) + ldg(rho + idx + sy));
     const T ro = (T)1 / rhy;
-    T dsxydx = div_c(d_bm<T, N>(sxy, idx, sx, c), dx, p.rd[0], p.fast_div);
-    T dsyydy = div_c(d_fm<T, N>(syy, idx, sy, c), dy, p.rd[1], p.fast_div);
-    T dsyzdz = div_c(d_bm<T, N>(syz, idx, 1, c), dz, p.rd[2], p.fast_div);
+    T dsxydx = d_bm<T, N>(sxy, idx, sx, c), dsyydy = d_fm<T, N>(syy, idx, sy, c), dsyzdz = d_bm<T, N>(syz, idx, 1, c);
+    spacings<T, 0, 1, 2>(p, dsxydx, dsyydy, dsyzdz);
     if ((fx & 1) || (fy & 2) || (fz & 1)) {
-      const T xn = (T)1 - hdt * dpx[i], yn = (T)1 - hdt * dpy[ny + j], zn = (T)1 - hdt * dpz[k];
-      const T xd = (T)1 + hdt * dpx[i], yd = (T)1 + hdt * dpy[ny + j], zd = (T)1 + hdt * dpz[k];
-      T a = div_v((xn * sp[PVY_X * G + sh] + dt * dsxydx * ro), xd);
-      T b = div_v((yn * sp[PVY_Y * G + sh] + dt * dsyydy * ro), yd);
-      T cc = div_v((zn * sp[PVY_Z * G + sh] + dt * dsyzdz * ro), zd);
+      const Damp<T> x = damp_of(dpx[i], hdt), y = damp_of(dpy[ny + j], hdt), z = damp_of(dpz[k], hdt);
+      T qa[3] = {x.w * sp[PVY_X * G + sh] + dt * dsxydx * ro,
+          y.w * sp[PVY_Y * G + sh] + dt * dsyydy * ro,
+          z.w * sp[PVY_Z * G + sh] + dt * dsyzdz * ro};
+      split_quotients<T, 3>(qa, {x, y, z});
+      const T a = qa[0], b = qa[1], cc = qa[2];
       sp[PVY_X * G + sh] = a;
       sp[PVY_Y * G + sh] = b;
       sp[PVY_Z * G + sh] = cc;
@@ -109,15 +132,15 @@ ks_velocity(const __grid_constant__ P3<T> p, int it, int src_here) {
     if (upd) {
       const T r4 = (T)0.25 * (ldg(rho + idx) + ldg(rho + idx + sy) + ldg(rho + idx + sx + sy) + ldg(rho + idx + sx));
       const T ro = (T)1 / r4;
-      T dsxzdx = div_c(d_bm<T, N>(sxz, idx, sx, c), dx, p.rd[0], p.fast_div);
-      T dsyzdy = div_c(d_bm<T, N>(syz, idx, sy, c), dy, p.rd[1], p.fast_div);
-      T dszzdz = div_c(d_fm<T, N>(szz, idx, 1, c), dz, p.rd[2], p.fast_div);
+      T dsxzdx = d_bm<T, N>(sxz, idx, sx, c), dsyzdy = d_bm<T, N>(syz, idx, sy, c), dszzdz = d_fm<T, N>(szz, idx, 1, c);
+      spacings<T, 0, 1, 2>(p, dsxzdx, dsyzdy, dszzdz);
       if ((fx & 1) || (fy & 1) || (fz & 2)) {
-        const T xn = (T)1 - hdt * dpx[i], yn = (T)1 - hdt * dpy[j], zn = (T)1 - hdt * dpz[nz + k];
-        const T xd = (T)1 + hdt * dpx[i], yd = (T)1 + hdt * dpy[j], zd = (T)1 + hdt * dpz[nz + k];
-        T a = div_v((xn * sp[PVZ_X * G + sh] + dt * dsxzdx * ro), xd);
-        T b = div_v((yn * sp[PVZ_Y * G + sh] + dt * dsyzdy * ro), yd);
-        T cc = div_v((zn * sp[PVZ_Z * G + sh] + dt * dszzdz * ro), zd);
+        const Damp<T> x = damp_of(dpx[i], hdt), y = damp_of(dpy[j], hdt), z = damp_of(dpz[nz + k], hdt);
+        T qa[3] = {x.w * sp[PVZ_X * G + sh] + dt * dsxzdx * ro,
+            y.w * sp[PVZ_Y * G + sh] + dt * dsyzdy * ro,
+            z.w * sp[PVZ_Z * G + sh] + dt * dszzdz * ro};
+        split_quotients<T, 3>(qa, {x, y, z});
+        const T a = qa[0], b = qa[1], cc = qa[2];
         sp[PVZ_X * G + sh] = a;
         sp[PVZ_Y * G + sh] = b;
         sp[PVZ_Z * G + sh] = cc;
@@ -151,7 +174,7 @@ ks_stress(const __grid_constant__ P3<T> p, int it) {
   const long long sx = (long long)ny * nz, sy = nz;
   const long long idx = (long long)i * sx + (long long)j * nz + k;
   const long long G = p.scomp;
-  const T dx = p.dx, dy = p.dy, dz = p.dz, dt = p.dt;
+  const T dt = p.dt;
   const T hdt = (T)0.5 * dt;
   T c[N];
 #pragma unroll
@@ -168,21 +191,25 @@ ks_stress(const __grid_constant__ P3<T> p, int it) {
   if (i >= N + 1 && i < nx - N && j >= N + 1 && j < ny - N && k >= N + 1 && k < nz - N) {
     const T lm = ldg(lam + idx), u = ldg(mu + idx);
     const T l2m = lm + (T)2 * u;
-    T dvxdx = div_c(d_bm<T, N>(vx, idx, sx, c), dx, p.rd[0], p.fast_div);
-    T dvydy = div_c(d_bm<T, N>(vy, idx, sy, c), dy, p.rd[1], p.fast_div);
-    T dvzdz = div_c(d_bm<T, N>(vz, idx, 1, c), dz, p.rd[2], p.fast_div);
+    T dvxdx = d_bm<T, N>(vx, idx, sx, c), dvydy = d_bm<T, N>(vy, idx, sy, c), dvzdz = d_bm<T, N>(vz, idx, 1, c);
+    spacings<T, 0, 1, 2>(p, dvxdx, dvydy, dvzdz);
     if ((fx | fy | fz) & 1) {
-      const T xn = (T)1 - hdt * dpx[i], yn = (T)1 - hdt * dpy[j], zn = (T)1 - hdt * dpz[k];
-      const T xd = (T)1 + hdt * dpx[i], yd = (T)1 + hdt * dpy[j], zd = (T)1 + hdt * dpz[k];
-      T xx = div_v((xn * sp[PSXX_X * G + sh] + dt * l2m * dvxdx), xd);
-      T xy = div_v((yn * sp[PSXX_Y * G + sh] + dt * lm * dvydy), yd);
-      T xz = div_v((zn * sp[PSXX_Z * G + sh] + dt * lm * dvzdz), zd);
-      T yx = div_v((xn * sp[PSYY_X * G + sh] + dt * lm * dvxdx), xd);
-      T yy = div_v((yn * sp[PSYY_Y * G + sh] + dt * l2m * dvydy), yd);
-      T yz = div_v((zn * sp[PSYY_Z * G + sh] + dt * lm * dvzdz), zd);
-      T zx = div_v((xn * sp[PSZZ_X * G + sh] + dt * lm * dvxdx), xd);
-      T zy = div_v((yn * sp[PSZZ_Y * G + sh] + dt * lm * dvydy), yd);
-      T zz = div_v((zn * sp[PSZZ_Z * G + sh] + dt * l2m * dvzdz), zd);
+      const Damp<T> x = damp_of(dpx[i], hdt), y = damp_of(dpy[j], hdt), z = damp_of(dpz[k], hdt);
+      T qxx[3] = {x.w * sp[PSXX_X * G + sh] + dt * l2m * dvxdx,
+          y.w * sp[PSXX_Y * G + sh] + dt * lm * dvydy,
+          z.w * sp[PSXX_Z * G + sh] + dt * lm * dvzdz};
+      split_quotients<T, 3>(qxx, {x, y, z});
+      const T xx = qxx[0], xy = qxx[1], xz = qxx[2];
+      T qyx[3] = {x.w * sp[PSYY_X * G + sh] + dt * lm * dvxdx,
+          y.w * sp[PSYY_Y * G + sh] + dt * l2m * dvydy,
+          z.w * sp[PSYY_Z * G + sh] + dt * lm * dvzdz};
+      split_quotients<T, 3>(qyx, {x, y, z});
+      const T yx = qyx[0], yy = qyx[1], yz = qyx[2];
+      T qzx[3] = {x.w * sp[PSZZ_X * G + sh] + dt * lm * dvxdx,
+          y.w * sp[PSZZ_Y * G + sh] + dt * lm * dvydy,
+          z.w * sp[PSZZ_Z * G + sh] + dt * l2m * dvzdz};
+      split_quotients<T, 3>(qzx, {x, y, z});
+      const T zx = qzx[0], zy = qzx[1], zz = qzx[2];
       sp[PSXX_X * G + sh] = xx; sp[PSXX_Y * G + sh] = xy; sp[PSXX_Z * G + sh] = xz;
       sp[PSYY_X * G + sh] = yx; sp[PSYY_Y * G + sh] = yy; sp[PSYY_Z * G + sh] = yz;
       sp[PSZZ_X * G + sh] = zx; sp[PSZZ_Y * G + sh] = zy; sp[PSZZ_Z * G + sh] = zz;
@@ -198,13 +225,14 @@ ks_stress(const __grid_constant__ P3<T> p, int it) {
   // sxy :334-350
   if (i >= N + 1 && i < nx - N && j >= N + 1 && j < ny - N && k >= N && k < nz - N) {
     const T m4 = (T)0.25 * (ldg(mu + idx + sy) + ldg(mu + idx) + ldg(mu + idx) + ldg(mu + idx + sx));
-    T dvydx = div_c(d_fm<T, N>(vy, idx, sx, c), dx, p.rd[0], p.fast_div);
-    T dvxdy = div_c(d_fm<T, N>(vx, idx, sy, c), dy, p.rd[1], p.fast_div);
+    T dvydx = d_fm<T, N>(vy, idx, sx, c), dvxdy = d_fm<T, N>(vx, idx, sy, c);
+    spacings<T, 0, 1>(p, dvydx, dvxdy);
     if ((fx & 2) || (fy & 2) || (fz & 1)) {
-      const T xn = (T)1 - hdt * dpx[nx + i], yn = (T)1 - hdt * dpy[ny + j];
-      const T xd = (T)1 + hdt * dpx[nx + i], yd = (T)1 + hdt * dpy[ny + j];
-      T a = div_v((xn * sp[PSXY_X * G + sh] + dt * m4 * dvydx), xd);
-      T b = div_v((yn * sp[PSXY_Y * G + sh] + dt * m4 * dvxdy), yd);
+      const Damp<T> x = damp_of(dpx[nx + i], hdt), y = damp_of(dpy[ny + j], hdt);
+      T qa[2] = {x.w * sp[PSXY_X * G + sh] + dt * m4 * dvydx,
+          y.w * sp[PSXY_Y * G + sh] + dt * m4 * dvxdy};
+      split_quotients<T, 2>(qa, {x, y});
+      const T a = qa[0], b = qa[1];
       sp[PSXY_X * G + sh] = a;
       sp[PSXY_Y * G + sh] = b;
       sxy[idx] = a + b;
@@ -215,13 +243,14 @@ ks_stress(const __grid_constant__ P3<T> p, int it) {
   // sxz :352-371
   if (i >= N && i < nx - N - 1 && j >= N && j < ny - N && k >= N && k < nz - N - 1) {
     const T m4 = (T)0.25 * (ldg(mu + idx) + ldg(mu + idx + sx) + ldg(mu + idx) + ldg(mu + idx + sy));
-    T dvzdx = div_c(d_fm<T, N>(vz, idx, sx, c), dx, p.rd[0], p.fast_div);
-    T dvxdz = div_c(d_fm<T, N>(vx, idx, 1, c), dz, p.rd[2], p.fast_div);
+    T dvzdx = d_fm<T, N>(vz, idx, sx, c), dvxdz = d_fm<T, N>(vx, idx, 1, c);
+    spacings<T, 0, 2>(p, dvzdx, dvxdz);
     if ((fx & 2) || (fy & 1) || (fz & 2)) {
-      const T xn = (T)1 - hdt * dpx[nx + i], zn = (T)1 - hdt * dpz[nz + k];
-      const T xd = (T)1 + hdt * dpx[nx + i], zd = (T)1 + hdt * dpz[nz + k];
-      T a = div_v((xn * sp[PSXZ_X * G + sh] + dt * m4 * dvzdx), xd);
-      T b = div_v((zn * sp[PSXZ_Z * G + sh] + dt * m4 * dvxdz), zd);
+      const Damp<T> x = damp_of(dpx[nx + i], hdt), z = damp_of(dpz[nz + k], hdt);
+      T qa[2] = {x.w * sp[PSXZ_X * G + sh] + dt * m4 * dvzdx,
+          z.w * sp[PSXZ_Z * G + sh] + dt * m4 * dvxdz};
+      split_quotients<T, 2>(qa, {x, z});
+      const T a = qa[0], b = qa[1];
       sp[PSXZ_X * G + sh] = a;
       sp[PSXZ_Z * G + sh] = b;
       sxz[idx] = a + b;
@@ -232,13 +261,14 @@ ks_stress(const __grid_constant__ P3<T> p, int it) {
   // syz :373-391
   if (i >= N && i < nx - N && j >= N && j < ny - N - 1 && k >= N && k < nz - N - 1) {
     const T m4 = (T)0.25 * (ldg(mu + idx + sy) + ldg(mu + idx) + ldg(mu + idx + 1) + ldg(mu + idx));
-    T dvzdy = div_c(d_fm<T, N>(vz, idx, sy, c), dy, p.rd[1], p.fast_div);
-    T dvydz = div_c(d_fm<T, N>(vy, idx, 1, c), dz, p.rd[2], p.fast_div);
+    T dvzdy = d_fm<T, N>(vz, idx, sy, c), dvydz = d_fm<T, N>(vy, idx, 1, c);
+    spacings<T, 1, 2>(p, dvzdy, dvydz);
     if ((fx & 1) || (fy & 2) || (fz & 2)) {
-      const T yn = (T)1 - hdt * dpy[ny + j], zn = (T)1 - hdt * dpz[nz + k];
-      const T yd = (T)1 + hdt * dpy[ny + j], zd = (T)1 + hdt * dpz[nz + k];
-      T a = div_v((yn * sp[PSYZ_Y * G + sh] + dt * m4 * dvzdy), yd);
-      T b = div_v((zn * sp[PSYZ_Z * G + sh] + dt * m4 * dvydz), zd);
+      const Damp<T> y = damp_of(dpy[ny + j], hdt), z = damp_of(dpz[nz + k], hdt);
+      T qa[2] = {y.w * sp[PSYZ_Y * G + sh] + dt * m4 * dvzdy,
+          z.w * sp[PSYZ_Z * G + sh] + dt * m4 * dvydz};
+      split_quotients<T, 2>(qa, {y, z});
+      const T a = qa[0], b = qa[1];
       sp[PSYZ_Y * G + sh] = a;
       sp[PSYZ_Z * G + sh] = b;
       syz[idx] = a + b;

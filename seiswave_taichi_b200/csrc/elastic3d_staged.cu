@@ -553,7 +553,7 @@ template <int Q>
 __device__ __forceinline__ SplitAt<Q> split_at(const P3<float>& p, int i, int j, int k, uint8_t fxy,
                                                const uint8_t (&fz)[Q]) {
   SplitAt<Q> at;
-  const bool in0 = fxy | fz[0], in1 = k + Q - 1 < p.nz && (fxy | fz[Q - 1]);
+  const bool in0 = fxy | fz[0], in1 = fxy | fz[Q - 1];
   const long long s0 = in0 ? shell_index(p, i, j, k) : 0;
   const long long s1 = in1 ? shell_index(p, i, j, k + Q - 1) : 0;
   const long long base = in0 ? s0 : s1;
