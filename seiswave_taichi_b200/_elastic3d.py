@@ -355,11 +355,11 @@ class Elastic3DBase:
         (self._plan or self._build_plan()).set_tile(int(x_chunk))
 
     # -- autotuner (no reference counterpart) ------------------------------------
-    AUTOTUNE_CHUNKS = (6, 8, 12, 16, 25, 50)
+    AUTOTUNE_CHUNKS = (2, 3, 4, 6, 8, 12, 16, 25, 50)
 
     def autotune(self, steps: int = 6, force: bool = False) -> int:
         """Choose the x planes per work unit of the plan's current path (the
-        staged or fused chunk, or the two-pass kernels' x_chunk) by timing
+        staged or fused chunk; the per-cell kernels have none) by timing
         `steps` steps of each candidate on this solver's own grid, with its
         state replaced by random values for the trials and restored
         afterwards (results do not depend on the choice).  The winner is

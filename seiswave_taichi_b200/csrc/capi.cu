@@ -197,7 +197,7 @@ struct sw_plan {
   float* pitch_buf = nullptr;
   sw::P3<float> pp{};
   sw::StagedMaps pvm{}, psm{};
-  // 0: register-queue two-pass kernels (2D: two launches per step), 1: staged
+  // 0: per-cell two-pass kernels (2D: two launches per step), 1: staged
   // two-pass, 2: fused single pass, 3: 2D persistent (one cooperative launch
   // per run)
   int path = 0;
@@ -822,8 +822,8 @@ void setup_resident(sw_plan* pl) {
   resident_limits(&blocks, &smem);
   int tx, tz, words, width;
   size_t bytes;
-  const bool ok = pl->dtype == SW_F32 ? sw::sw2r_tiles<float>(pl->p2f, pl->order, blocks, smem, 0, &tx, &tz, &words, &bytes, &width)
-                                      : sw::sw2r_tiles<double>(pl->p2d, pl->order, blocks, smem, 0, &tx, &tz, &words, &bytes, &width);
+  const bool ok = pl->dtype == SW_F32 ? sw::sw2r_tiles<float>(pl->p2f, pl->order, blocks, smem, &tx, &tz, &words, &bytes, &width)
+                                      : sw::sw2r_tiles<double>(pl->p2d, pl->order, blocks, smem, &tx, &tz, &words, &bytes, &width);
   if (!ok) return;
   pl->res_tx = tx;
   pl->res_tz = tz;
@@ -835,12 +835,10 @@ void setup_resident(sw_plan* pl) {
 template <typename T>
 cudaError_t resident_run_t(sw_plan* pl, const sw::P2<T>& p, int it0, int nsteps, cudaStream_t st) {
   sw::Res2<T> r{};
-  r.shots[0] = p;
-  r.n = 1;
-  r.tx[0] = pl->res_tx;
-  r.tz[0] = pl->res_tz;
-  r.stride[0] = pl->res_words;
-  r.blocks = pl->res_tx * pl->res_tz;
+  r.shot = p;
+  r.tx = pl->res_tx;
+  r.tz = pl->res_tz;
+  r.stride = pl->res_words;
   r.width = pl->res_width;
   r.smem = pl->res_smem;
   r.inbox = pl->d_inbox;

@@ -1,6 +1,7 @@
 // elastic2d_resident.cu -- 2D SSG_VS / SSG_SV time loops that stay on the chip
-// (src/Elastic2D_CPML.py:128-275): one cooperative launch runs all steps of
-// one shot, or of several shots side by side.
+// (src/Elastic2D_CPML.py:128-275): one cooperative launch runs all steps.
+// (Waves of a batch's shots side by side in one launch measured 0.98-1.03x the
+// batch's own two launches per step, so batches keep those.)
 //
 // What bounds the two-launch step is not memory but the chain of one short
 // kernel after another: at 400 x 400 each of the two launches takes 6.2 us
@@ -23,7 +24,7 @@
 // launch, on its stream.
 //
 // Measured on B200 (us per step from rest, two launches per step from a graph
-// -> on the chip): 60 x 64 9.9 -> 4.7, 200^2 10.2 -> 4.5, 400^2 11.6 -> 6.6,
+// -> on the chip): 60 x 64 9.9 -> 4.7, 200^2 10.2 -> 4.5, 400^2 11.7 -> 6.2,
 // 700 x 400 15.0 -> 9.6, 1000 x 420 18.8 -> 12.6; float64 100^2 10.9 -> 4.2.
 // What is left: two exchanges of about 1.2 us, instruction issue (about 190
 // warp instructions per 32 cells and phase, more in the slabs and where
@@ -150,12 +151,10 @@ k2r_run(const __grid_constant__ Res2<T> rs, int it0, int nsteps, int aea) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ int n_own;
 
-  // this block's shot and tile
-  int sh = 0;
-  while (sh + 1 < rs.n && (int)blockIdx.x >= rs.first[sh + 1]) ++sh;
-  const P2<T>& p = rs.shots[sh];
-  const int tiles_x = rs.tx[sh], tiles_z = rs.tz[sh];
-  const int tile = blockIdx.x - rs.first[sh];
+  // this block's tile
+  const P2<T>& p = rs.shot;
+  const int tiles_x = rs.tx, tiles_z = rs.tz;
+  const int tile = blockIdx.x;
   const int tix = tile / tiles_z, tiz = tile % tiles_z;
   const int nx = p.nx, nz = p.nz;
   const int i0 = res2_cut_x(nx, p.lo[0], p.hi[0], tix, tiles_x), i1 = res2_cut_x(nx, p.lo[0], p.hi[0], tix + 1, tiles_x);
@@ -320,7 +319,7 @@ k2r_run(const __grid_constant__ Res2<T> rs, int it0, int nsteps, int aea) {
   // N on the z sides (lo, hi)
   const int nrim = 2 * N * (bx + bz);
   constexpr int W = Rim<T>::WORDS;
-  auto buffer = [&](int t, int phase) { return rs.inbox + rs.base[sh] + ((long long)t * 2 + phase) * rs.stride[sh]; };
+  auto buffer = [&](int t, int phase) { return rs.inbox + ((long long)t * 2 + phase) * rs.stride; };
   const int bz_lo = j0 - res2_cut_z(nz, max(tiz - 1, 0), tiles_z);  // columns of the z neighbours
   const int bz_hi = res2_cut_z(nz, min(tiz + 2, tiles_z), tiles_z) - j1;
   // Send new values where a neighbour's rim needs them.  The rows of the x rims
@@ -585,7 +584,7 @@ size_t tile_smem(const P2<T>& p, int N, int tx, int tz, long long* work, int* wo
 }  // namespace
 
 template <typename T>
-bool sw2r_tiles(const P2<T>& p, int N, int blocks, size_t smem, int width, int* tx, int* tz, int* words,
+bool sw2r_tiles(const P2<T>& p, int N, int blocks, size_t smem, int* tx, int* tz, int* words,
                 size_t* bytes, int* got) {
   if (N > SW_RES_ORDER) return false;
   long long best = -1;
@@ -595,7 +594,7 @@ bool sw2r_tiles(const P2<T>& p, int N, int blocks, size_t smem, int width, int* 
       int w, bw;
       const size_t s = tile_smem(p, N, a, b, &work, &w, &bw);
       if (s == 0) break;  // shorter rows only from here on
-      if (s > smem || (width && bw > width) || (best >= 0 && work >= best)) continue;
+      if (s > smem || (best >= 0 && work >= best)) continue;
       best = work;
       *tx = a;
       *tz = b;
@@ -604,21 +603,6 @@ bool sw2r_tiles(const P2<T>& p, int N, int blocks, size_t smem, int width, int* 
       *got = bw;
     }
   return best >= 0;
-}
-
-template <typename T>
-int sw2r_min_tiles(const P2<T>& p, int N, int blocks, size_t smem) {
-  if (N > SW_RES_ORDER) return 0;
-  int best = 0;
-  for (int b = 1; b <= blocks; ++b)
-    for (int a = 1; a * b <= (best ? best - 1 : blocks); ++a) {
-      long long work;
-      int w, bw;
-      const size_t s = tile_smem(p, N, a, b, &work, &w, &bw);
-      if (s == 0) break;
-      if (s <= smem) best = a * b;
-    }
-  return best;
 }
 
 template <typename T, int N, int S, int BZ>
@@ -640,7 +624,7 @@ static cudaError_t launch2r(const Res2<T>& rs, int it0, int nsteps, int aea, cud
   if (e != cudaSuccess) return e;
   Res2<T> r = rs;
   void* args[] = {&r, &it0, &nsteps, &aea};
-  return cudaLaunchCooperativeKernel((const void*)kern, dim3(rs.blocks), dim3(NT), args, rs.smem, st);
+  return cudaLaunchCooperativeKernel((const void*)kern, dim3(rs.tx * rs.tz), dim3(NT), args, rs.smem, st);
 }
 
 template <typename T, int S>
@@ -656,10 +640,7 @@ static cudaError_t order2r(const Res2<T>& rs, int order, int it0, int n, int aea
 
 template <typename T>
 cudaError_t sw2r_run(const Res2<T>& rs, int scheme, int order, int it0, int nsteps, int aea, cudaStream_t st) {
-  // zero the tags of the buffers that this launch uses
-  size_t words = 0;
-  for (int s = 0; s < rs.n; ++s)
-    words = std::max(words, (size_t)rs.base[s] + 2 * (size_t)rs.tx[s] * rs.tz[s] * rs.stride[s]);
+  const size_t words = 2 * (size_t)rs.tx * rs.tz * rs.stride;
   cudaError_t e = cudaMemsetAsync(rs.inbox, 0, words * sizeof(uint64_t), st);
   if (e != cudaSuccess) return e;
   return scheme == SW2D_SSG_VS ? order2r<T, SW2D_SSG_VS>(rs, order, it0, nsteps, aea, st)
@@ -667,8 +648,7 @@ cudaError_t sw2r_run(const Res2<T>& rs, int scheme, int order, int it0, int nste
 }
 
 #define SW_RES_INST(T)                                                                          \
-  template bool sw2r_tiles<T>(const P2<T>&, int, int, size_t, int, int*, int*, int*, size_t*, int*); \
-  template int sw2r_min_tiles<T>(const P2<T>&, int, int, size_t);                               \
+  template bool sw2r_tiles<T>(const P2<T>&, int, int, size_t, int*, int*, int*, size_t*, int*); \
   template cudaError_t sw2r_run<T>(const Res2<T>&, int, int, int, int, int, cudaStream_t);
 SW_RES_INST(float)
 SW_RES_INST(double)

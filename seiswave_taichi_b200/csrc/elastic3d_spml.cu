@@ -13,9 +13,9 @@
 namespace sw {
 
 // Resident blocks per SM the float kernels are compiled for: one thread per
-// cell waits on its loads (100^3 order 4 / 100 x 90 x 103 order 3, us per step:
-// the compiler's own count 165 / 181, 4 blocks 152 / 162, 6 125 / 132, 8 112 /
-// 120)
+// cell waits on its loads (us per step with 4, 5, 6, 8 blocks: 200^3 order 2
+// 874, 780, 729, 622, order 4 897, 830, 812, 718; 100^3 order 4 107, 106, 107,
+// 102)
 #define SW_KS_MINB (sizeof(T) == 4 ? 8 : 1)
 constexpr int TSZ = 32;
 constexpr int TSY = 8;

@@ -13,17 +13,15 @@ namespace sw {
 #define SW_RES_MIN 8     // smallest tile side
 #define SW_RES_STEPS 4   // fewest steps of a run that the on-chip loop takes
 
-// The shots of one launch (by value in kernel parameter space, as Batch2) and
-// their tiles: shot s has tx[s] x tz[s] tiles, the blocks first[s] ..; tile
-// (a, b) covers the rows between the cuts a and a+1 (res2_cut_x) and the
-// columns between the cuts b and b+1 (res2_cut_z).  Its rim buffers (one per phase, stride[s] 8-byte words each) start at word
-// base[s] + 2*tile*stride[s] of the inbox.
+// One launch: the shot and its tx x tz tiles, one per block; tile (a, b) covers
+// the rows between the cuts a and a+1 (res2_cut_x) and the columns between the
+// cuts b and b+1 (res2_cut_z).  A tile's rim buffers (one per phase, `stride`
+// 8-byte words each) start at word 2*tile*stride of the inbox.
 template <typename T>
 struct Res2 {
-  P2<T> shots[SW_BATCH_GROUP];
-  int first[SW_BATCH_GROUP], tx[SW_BATCH_GROUP], tz[SW_BATCH_GROUP], stride[SW_BATCH_GROUP];
-  int base[SW_BATCH_GROUP];
-  int n, blocks, width;  // width: columns of a row block, 32 or 64 (every tile is at most that wide)
+  P2<T> shot;
+  int tx, tz, stride;
+  int width;  // columns of a row block, 32 or 64 (every tile is at most that wide)
   size_t smem;
   uint64_t* inbox;
   int* err;
@@ -53,18 +51,14 @@ __host__ __device__ __forceinline__ size_t res2_smem(int bx, int bz, int width, 
   return res2_align16(v * esz) + 8 * SW_RES_RECV + 4 * (size_t)bx * width;
 }
 
-// Tiles for shot p on at most `blocks` SMs with `smem` bytes each, at most
-// `width` columns wide (0: any): the split with the least work per tile, or
-// false when none fits.  *words: 8-byte words of one rim buffer, *got: the row
-// block's width.
+// Tiles for shot p on at most `blocks` SMs with `smem` bytes each: the split
+// with the least work per tile, or false when none fits.  *words: 8-byte words
+// of one rim buffer, *width: the row block's width.
 template <typename T>
-bool sw2r_tiles(const P2<T>& p, int N, int blocks, size_t smem, int width, int* tx, int* tz, int* words, size_t* bytes,
-                int* got);
-// the fewest tiles that fit, 0 when more than `blocks` would be needed
-template <typename T>
-int sw2r_min_tiles(const P2<T>& p, int N, int blocks, size_t smem);
+bool sw2r_tiles(const P2<T>& p, int N, int blocks, size_t smem, int* tx, int* tz, int* words, size_t* bytes,
+                int* width);
 
-// nsteps >= 1 steps of every shot of rs; aea: the free-surface hook precedes
+// nsteps >= 1 steps of rs; aea: the free-surface hook precedes
 // every step
 template <typename T>
 cudaError_t sw2r_run(const Res2<T>& rs, int scheme, int order, int it0, int nsteps, int aea, cudaStream_t st);
