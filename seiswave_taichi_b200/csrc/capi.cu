@@ -488,6 +488,32 @@ int check_it(sw_plan* pl, int it0, int n) {
 }
 
 
+// Device scratch that holds zeros when the call returns.  The kernels that use
+// it run on the caller's streams, and nothing orders those behind a memset of
+// the default stream: a unit counter or barrier word that a pass read before
+// its zero arrived would send it to units that do not exist, and a late zero
+// would hand units out twice.
+cudaError_t zeroed_scratch(void** out, size_t bytes) {
+  void* b = nullptr;
+  cudaStream_t st = nullptr;
+  cudaError_t e = cudaMalloc(&b, bytes);
+  if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
+  if (e == cudaSuccess) e = cudaMemsetAsync(b, 0, bytes, st);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+  if (st) cudaStreamDestroy(st);
+  if (e != cudaSuccess) {
+    if (b) cudaFree(b);
+    return e;
+  }
+  *out = b;
+  return cudaSuccess;
+}
+
+// the error word and the staged passes' two unit counters, on first use
+cudaError_t plan_words(sw_plan* pl) {
+  return pl->d_err ? cudaSuccess : zeroed_scratch((void**)&pl->d_err, 3 * sizeof(int));
+}
+
 // ---------------------------------------------------------------------------
 // fused single-pass path: second buffer set, tensor maps, divisor check
 // ---------------------------------------------------------------------------
@@ -536,12 +562,10 @@ void setup_fused(sw_plan* pl) {
     total += (mv[d] + 63) / 64 * 64;
   }
   float* buf = nullptr;
-  if (cudaMalloc(&buf, total * sizeof(float)) != cudaSuccess) { cudaGetLastError(); return; }
-  if (!pl->d_err) {
-    if (cudaMalloc(&pl->d_err, 3 * sizeof(int)) != cudaSuccess) { cudaFree(buf); cudaGetLastError(); return; }
-    cudaMemset(pl->d_err, 0, 3 * sizeof(int));
+  if (plan_words(pl) != cudaSuccess || zeroed_scratch((void**)&buf, total * sizeof(float)) != cudaSuccess) {
+    cudaGetLastError();
+    return;
   }
-  cudaMemset(buf, 0, total * sizeof(float));
   auto& x = pl->fx;
   float* cur = buf;
   for (int q = 0; q < 9; ++q) { x.fB[q] = cur; cur += ncell; }
@@ -649,13 +673,10 @@ void setup_staged(sw_plan* pl) {
   pl->pitch_ok = p.nz % 4 != 0 && pl->gather_in_stress && pl->scheme != SW3D_SPML && pl->order <= 2 &&
                  (long long)p.nx * p.ny * p.nz >= 1500000LL;
   if (!direct && !pl->pitch_ok) return;
-  if (!pl->d_err) {
-    if (cudaMalloc(&pl->d_err, 3 * sizeof(int)) != cudaSuccess) {
-      cudaGetLastError();
-      pl->pitch_ok = false;
-      return;
-    }
-    cudaMemset(pl->d_err, 0, 3 * sizeof(int));
+  if (plan_words(pl) != cudaSuccess) {
+    cudaGetLastError();
+    pl->pitch_ok = false;
+    return;
   }
   if (direct && !sw::sw3_staged_maps(pl->order, tz, p, &pl->svm, &pl->ssm)) return;
   pl->staged_N = pl->order;
@@ -768,18 +789,9 @@ cudaError_t enqueue_fused_run(sw_plan* pl, int it0, int nsteps, cudaStream_t st)
 
 // 2D persistent path: the barrier words and the error word on first use
 cudaError_t persistent_run2(sw_plan* pl, int it0, int nsteps, cudaStream_t st) {
-  if (!pl->d_bar) {
-    cudaError_t e = cudaMalloc(&pl->d_bar, 2 * sizeof(unsigned int));
-    if (e != cudaSuccess) return e;
-    e = cudaMemset(pl->d_bar, 0, 2 * sizeof(unsigned int));
-    if (e != cudaSuccess) return e;
-  }
-  if (!pl->d_err) {
-    cudaError_t e = cudaMalloc(&pl->d_err, 3 * sizeof(int));
-    if (e != cudaSuccess) return e;
-    e = cudaMemset(pl->d_err, 0, 3 * sizeof(int));
-    if (e != cudaSuccess) return e;
-  }
+  cudaError_t e = plan_words(pl);
+  if (e == cudaSuccess && !pl->d_bar) e = zeroed_scratch((void**)&pl->d_bar, 2 * sizeof(unsigned int));
+  if (e != cudaSuccess) return e;
   if (pl->dtype == SW_F32)
     return sw::sw2_persistent<float>(pl->p2f, pl->scheme, pl->order, it0, nsteps, pl->gather_in_stress,
                                      pl->gather_in_stress, pl->d_bar, pl->d_err, st);
@@ -857,10 +869,9 @@ cudaError_t resident_run(sw_plan* pl, int it0, int nsteps, cudaStream_t st, bool
     return cudaSuccess;
   }
   if (!pl->d_inbox || !pl->d_err) {
-    if (!pl->d_err) {
-      if (cudaMalloc(&pl->d_err, 3 * sizeof(int)) != cudaSuccess) { cudaGetLastError(); return cudaSuccess; }
-      cudaError_t e = cudaMemset(pl->d_err, 0, 3 * sizeof(int));
-      if (e != cudaSuccess) return e;
+    if (plan_words(pl) != cudaSuccess) {
+      cudaGetLastError();
+      return cudaSuccess;
     }
     const size_t words = 2 * (size_t)pl->res_tx * pl->res_tz * pl->res_words;
     if (!pl->d_inbox && cudaMalloc(&pl->d_inbox, words * sizeof(uint64_t)) != cudaSuccess) {
@@ -1038,12 +1049,15 @@ int sw_plan_status(sw_plan* pl, void* stream) {
   if (e != cudaSuccess) return cuda_fail(e, "sw_plan_status");
   if (pl->d_err) {
     int h = 0;
-    e = cudaMemcpy(&h, pl->d_err, sizeof h, cudaMemcpyDeviceToHost);
+    e = cudaMemcpyAsync(&h, pl->d_err, sizeof h, cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) return cuda_fail(e, "sw_plan_status");
     if (h != 0) {
       // reported once: clear the word so that a retry after a transient
-      // timeout reads the status of the runs since this read
-      e = cudaMemset(pl->d_err, 0, sizeof(int));
+      // timeout reads the status of the runs since this read (on this stream,
+      // ahead of those runs)
+      e = cudaMemsetAsync(pl->d_err, 0, sizeof(int), st);
+      if (e == cudaSuccess) e = cudaStreamSynchronize(st);
       if (e != cudaSuccess) return cuda_fail(e, "sw_plan_status");
     }
     if (h & 1) return fail(SW_ERR_TIMEOUT, "a bounded device wait gave up (TMA data never arrived)");

@@ -1,0 +1,86 @@
+"""Solvers on streams of their own: a plan built and first run on a side stream
+while another host thread keeps the default stream busy gives the bits of one
+that has the device to itself (the device words of a plan are zero before any
+stream can reach them)."""
+import threading
+
+import pytest
+import torch
+
+from cases import case2d, case3d, product2d, product3d, to_np
+
+pytestmark = pytest.mark.gpu
+
+F2 = ("vx", "vz", "sxx", "szz", "sxz")
+F3 = ("vx", "vy", "vz", "sxx", "syy", "szz", "sxy", "sxz", "syz")
+
+
+class _Busy:
+    """Another host thread that always has work queued on the default stream."""
+
+    def __enter__(self):
+        self.stop = threading.Event()
+        self.started = threading.Event()
+        self.thread = threading.Thread(target=self._work)
+        self.thread.start()
+        assert self.started.wait(60)
+
+    def _work(self):
+        a = torch.randn(4096, 4096, device="cuda")
+        queued = []
+        while not self.stop.is_set():
+            a = (a @ a).clamp_(-1, 1)
+            queued.append(torch.cuda.Event())
+            queued[-1].record()
+            self.started.set()
+            if len(queued) > 4:
+                queued.pop(0).synchronize()
+        torch.cuda.current_stream().synchronize()
+
+    def __exit__(self, *_):
+        self.stop.set()
+        self.thread.join()
+
+
+def _state(w, plan, fields):
+    plan.status(w._stream())
+    out = {f: to_np(getattr(w, f)).copy() for f in fields}
+    out["data"] = to_np(w.data).copy()
+    return out
+
+
+def _run3(c, path, **kw):
+    w = product3d(c, **kw)
+    plan = w._build_plan()
+    plan.set_path(path)
+    w.run(c["nt"])
+    return _state(w, plan, F3)
+
+
+def _run2(c, path, graph=True):
+    w = product2d(c)
+    plan = w._plan(0)
+    plan.set_path(path)
+    w.run(c["nt"], use_graph=graph)
+    return _state(w, plan, F2)
+
+
+@pytest.mark.parametrize("run,case", [
+    (lambda c: _run3(c, "staged"), lambda: case3d(shape=(40, 36, 44), nt=40)),
+    (lambda c: _run3(c, "staged"), lambda: case3d(shape=(40, 36, 44), nt=40, scheme="SPML")),
+    (lambda c: _run3(c, "fused"), lambda: case3d(shape=(40, 36, 44), nt=41)),
+    (lambda c: _run3(c, "two_pass"), lambda: case3d(shape=(130, 111, 105), nt=20)),  # pitched copies
+    (lambda c: _run2(c, "two_pass"), lambda: case2d(nt=60, nrec=5)),
+    (lambda c: _run2(c, "persistent"), lambda: case2d(nt=60, nrec=5)),
+], ids=["staged", "staged_spml", "fused", "pitched", "on_chip", "persistent"])
+def test_first_run_on_a_side_stream(cuda, run, case):
+    c = case()
+    ref = run(c)
+    torch.cuda.synchronize()
+    with _Busy():
+        for _ in range(6):
+            s = torch.cuda.Stream()
+            with torch.cuda.stream(s):
+                got = run(c)
+            for k in ref:
+                assert got[k].tobytes() == ref[k].tobytes(), k
