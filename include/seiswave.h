@@ -209,7 +209,8 @@ SW_API int sw_plan_status(sw_plan* plan, void* stream);
  * bounded grid barrier; opt-in, as path 0 is faster on B200 at every grid
  * size measured; sw_step keeps the two launches), [1] constant-divisor fast path verified, [2] staged
  * path available, [3] its grid, [4] its x-chunk length, [5] fused path set
- * up, [6] its grid, [7] its x-chunk length, [8] exact numerics (see
+ * up, [6] its grid (2D: the tiles of the on-chip loop, 0 where sw_run replays
+ * the launches), [7] its x-chunk length, [8] exact numerics (see
  * sw_plan_set_exact).  info must hold 9 int32. */
 SW_API int sw_plan_info(sw_plan* plan, int32_t* info);
 
@@ -218,6 +219,17 @@ SW_API int sw_plan_info(sw_plan* plan, int32_t* info);
  * x planes per work unit of the staged or fused path (the autotuner's knob).
  * Every path gives the same result bit for bit. */
 SW_API int sw_plan_set_path(sw_plan* plan, int32_t path, int32_t chunk_len);
+
+/* The SMs that the on-chip loop of a 2D plan's sw_run may take: -1 (the
+ * default) as many as the device has, 0 none (sw_run replays the two launches
+ * of a step), n > 0 at most n, one tile each.  The loop holds its SMs, and most
+ * of their registers and shared memory, from its first step to its last, so
+ * solvers on several streams run side by side only while their tiles fit the
+ * device together.  A launch that the device refuses -- more tiles than can be
+ * resident at once on what the stream's context owns -- is not an error: this
+ * and the later runs replay the launches.  All choices give the same bits.
+ * No reference counterpart. */
+SW_API int sw_plan_set_on_chip(sw_plan* plan, int32_t blocks);
 
 /* Free-surface mode: when on != 0 every step first applies the reference's
  * free-surface hook AEA, as a driver loop `AEA(); update_SSG_VS(i)` does

@@ -107,6 +107,7 @@ class ElasticWAVE:
         self._prof = None
         self._plans = {}
         self._free_surface = False
+        self._on_chip = -1
         self._wavelets = {}
         self._mem = [None, None]
         self.MT = None if MT is None else moment_2d(MT)
@@ -282,6 +283,8 @@ class ElasticWAVE:
         plan = N.Plan(d, keep, three_d=False)
         if self._free_surface:
             plan.set_free_surface(True)
+        if self._on_chip >= 0:
+            plan.set_on_chip(self._on_chip)
         self._plans[scheme] = plan
         return plan
 
@@ -325,10 +328,26 @@ class ElasticWAVE:
             plan.set_free_surface(self._free_surface)
         return self
 
+    def set_on_chip(self, blocks: int = -1):
+        """The SMs that run()'s on-chip loop may take: -1 all, 0 none (its
+        steps are replayed as two launches each), n > 0 at most n.  The loop
+        holds its SMs for the whole run, so of several solvers on streams of
+        their own only those run side by side whose tiles fit the GPU together
+        (Plan.info()["on_chip_tiles"]); the results do not depend on it."""
+        if int(blocks) < -1:
+            raise ValueError("blocks is -1 (all), 0 (off) or the SMs to take at most")
+        self._on_chip = int(blocks)
+        for plan in self._plans.values():
+            plan.set_on_chip(self._on_chip)
+        return self
+
     def run(self, nt=None, it0: int = 0, scheme: str = "VS", use_graph: bool = True, free_surface=None):
         """Steps it0 .. it0+nt-1 of update_SSG_VS ("VS") or update_SSG_SV ("SV")
-        in one enqueue (CUDA graph); free_surface=True/False sets the
-        free-surface mode first (set_free_surface)."""
+        in one enqueue: one launch that keeps the state on the chip (runs of at
+        least 4 steps whose tiles fit, set_on_chip), else a replayed CUDA graph
+        of two launches per step, without use_graph the launches themselves.
+        free_surface=True/False sets the free-surface mode first
+        (set_free_surface)."""
         if free_surface is not None:
             self.set_free_surface(free_surface)
         nt = self.nt - it0 if nt is None else int(nt)

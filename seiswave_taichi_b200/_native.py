@@ -35,7 +35,7 @@ EXPORTS = (
     "sw_batch_destroy", "sw2d_abc_correct", "sw2d_abc_features", "sw_mlp_grad", "sw_mlp_forward",
     "sw_mlp_backward", "sw2d_abc_adjoint", "sw3d_snapshot_elems", "sw3d_record", "sw3d_adjoint_run",
     "sw3d_abc_correct", "sw3d_abc_features", "sw3d_abc_adjoint", "sw3d_mlp_grad", "sw3d_mlp_forward",
-    "sw3d_mlp_backward", "sw_segy_decode", "sw_plan_set_free_surface",
+    "sw3d_mlp_backward", "sw_segy_decode", "sw_plan_set_free_surface", "sw_plan_set_on_chip",
 )
 
 SW_ABC_DEPTH = 6
@@ -159,6 +159,7 @@ def load() -> C.CDLL:
         "sw2d_snapshot_elems": (C.c_int, [vp, C.POINTER(C.c_int64)]),
         "sw_segy_decode": (C.c_int, [vp, C.c_int64, C.c_int32, C.c_int32, vp, vp, vp]),
         "sw_plan_set_free_surface": (C.c_int, [vp, C.c_int32]),
+        "sw_plan_set_on_chip": (C.c_int, [vp, C.c_int32]),
         "sw2d_record": (C.c_int, [vp, C.c_int32, C.c_int32, vp, vp]),
         "sw2d_adjoint_run": (C.c_int, [vp, C.POINTER(Adjoint2D), C.c_int32, C.c_int32, vp, vp]),
         "sw2d_batch_create": (C.c_int, [C.POINTER(Desc2D), C.c_int32, C.POINTER(vp)]),
@@ -286,6 +287,7 @@ class Plan:
         else:
             check(lib.sw2d_plan_create(C.byref(desc), C.byref(h)))
         self._h = h
+        self._three_d = three_d
         self._desc = desc
         self._keep = keep
 
@@ -322,13 +324,20 @@ class Plan:
         a = (C.c_int32 * 9)()
         check(load().sw_plan_info(self._h, a))
         names = {v: k for k, v in self.PATHS.items()}
-        return {"path": names[a[0]], "fast_div": bool(a[1]), "staged": bool(a[2]), "staged_grid": a[3],
-                "staged_chunk": a[4], "fused": bool(a[5]), "fused_grid": a[6], "fused_chunk": a[7],
-                "exact": bool(a[8])}
+        d = {"path": names[a[0]], "fast_div": bool(a[1]), "staged": bool(a[2]), "staged_grid": a[3],
+             "staged_chunk": a[4], "fused": bool(a[5]), "fused_grid": a[6], "fused_chunk": a[7],
+             "exact": bool(a[8])}
+        if not self._three_d:
+            d["on_chip_tiles"], d["fused_grid"] = d["fused_grid"], 0
+        return d
 
     def set_free_surface(self, on: bool = True) -> None:
         """2D: apply the free-surface hook AEA before every step (sticky)."""
         check(load().sw_plan_set_free_surface(self._h, 1 if on else 0))
+
+    def set_on_chip(self, blocks: int) -> None:
+        """2D: the SMs the on-chip loop of run may take (-1 all, 0 off)."""
+        check(load().sw_plan_set_on_chip(self._h, int(blocks)))
 
     def set_exact(self, exact: bool) -> None:
         """Numeric mode of the staged path (the other paths are always exact)."""

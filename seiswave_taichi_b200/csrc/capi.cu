@@ -206,7 +206,7 @@ struct sw_plan {
   bool aea = false;               // free-surface hook before every step (sw_plan_set_free_surface)
   // 2D on-chip loop (sw_run of path 0): tiles (0: not available) and the rim inbox
   int res_tx = 0, res_tz = 0, res_words = 0, res_width = 0;
-  size_t res_smem = 0;
+  size_t res_smem = 0, inbox_words = 0;
   uint64_t* d_inbox = nullptr;
 };
 
@@ -826,12 +826,14 @@ bool resident_covers(const sw_plan* pl) {
          pl->gather_in_stress;
 }
 
-void setup_resident(sw_plan* pl) {
+// most: the SMs it may take, -1 all of the device (sw_plan_set_on_chip)
+void setup_resident(sw_plan* pl, int most) {
   pl->res_tx = 0;
   if (!resident_covers(pl)) return;
   int blocks;
   size_t smem;
   resident_limits(&blocks, &smem);
+  if (blocks > 0 && most >= 0) blocks = most;
   int tx, tz, words, width;
   size_t bytes;
   const bool ok = pl->dtype == SW_F32 ? sw::sw2r_tiles<float>(pl->p2f, pl->order, blocks, smem, &tx, &tz, &words, &bytes, &width)
@@ -858,9 +860,16 @@ cudaError_t resident_run_t(sw_plan* pl, const sw::P2<T>& p, int it0, int nsteps,
   return sw::sw2r_run<T>(r, pl->scheme, pl->order, it0, nsteps, pl->aea ? 1 : 0, st);
 }
 
+// The launch's refusals: its tiles cannot all be resident at once on what this
+// stream's context owns of the device (tiles are counted from the device)
+bool launch_refused(cudaError_t e) {
+  return e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorNotSupported || e == cudaErrorLaunchOutOfResources;
+}
+
 // *done = false when the graph of the other path has to run instead: the
-// scratch could not be allocated, or the stream is being captured (a run that
-// replays a graph is refused there, and stays refused)
+// scratch could not be allocated, the launch was refused (the plan then keeps
+// to the other path), or the stream is being captured (a run that replays a
+// graph is refused there, and stays refused)
 cudaError_t resident_run(sw_plan* pl, int it0, int nsteps, cudaStream_t st, bool* done) {
   *done = false;
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
@@ -868,20 +877,30 @@ cudaError_t resident_run(sw_plan* pl, int it0, int nsteps, cudaStream_t st, bool
     cudaGetLastError();
     return cudaSuccess;
   }
-  if (!pl->d_inbox || !pl->d_err) {
-    if (plan_words(pl) != cudaSuccess) {
+  const size_t words = 2 * (size_t)pl->res_tx * pl->res_tz * pl->res_words;
+  if (plan_words(pl) != cudaSuccess) {
+    cudaGetLastError();
+    return cudaSuccess;
+  }
+  if (pl->inbox_words < words) {
+    if (pl->d_inbox) cudaFree(pl->d_inbox);
+    pl->d_inbox = nullptr;
+    pl->inbox_words = 0;
+    if (cudaMalloc(&pl->d_inbox, words * sizeof(uint64_t)) != cudaSuccess) {
       cudaGetLastError();
       return cudaSuccess;
     }
-    const size_t words = 2 * (size_t)pl->res_tx * pl->res_tz * pl->res_words;
-    if (!pl->d_inbox && cudaMalloc(&pl->d_inbox, words * sizeof(uint64_t)) != cudaSuccess) {
-      cudaGetLastError();
-      return cudaSuccess;
-    }
+    pl->inbox_words = words;
+  }
+  const cudaError_t e = pl->dtype == SW_F32 ? resident_run_t<float>(pl, pl->p2f, it0, nsteps, st)
+                                            : resident_run_t<double>(pl, pl->p2d, it0, nsteps, st);
+  if (launch_refused(e)) {
+    cudaGetLastError();
+    pl->res_tx = 0;
+    return cudaSuccess;
   }
   *done = true;
-  return pl->dtype == SW_F32 ? resident_run_t<float>(pl, pl->p2f, it0, nsteps, st)
-                             : resident_run_t<double>(pl, pl->p2d, it0, nsteps, st);
+  return e;
 }
 
 cudaError_t enqueue_sequence(sw_plan* pl, int it0, int nsteps, cudaStream_t st) {
@@ -956,7 +975,7 @@ int sw2d_plan_create(const sw2d_desc* d, sw_plan** out) {
   for (int q = 0; q < 5; ++q) pl->fields[q] = d->field[q];
   if (d->dtype == SW_F32) make_p2<float>(d, pl->p2f);
   else make_p2<double>(d, pl->p2d);
-  setup_resident(pl);
+  setup_resident(pl, -1);
   *out = pl;
   return SW_OK;
 }
@@ -1084,7 +1103,7 @@ int sw_plan_info(sw_plan* pl, int32_t* info) {
   }
   info[4] = pl->staged ? pl->sa.chunk_len : 0;
   info[5] = pl->fused ? 1 : 0;
-  info[6] = pl->fused ? pl->fused_grid : 0;
+  info[6] = pl->dim == 2 ? pl->res_tx * pl->res_tz : (pl->fused ? pl->fused_grid : 0);
   info[7] = pl->fused ? pl->fx.chunk_len : 0;
   info[8] = pl->staged ? pl->sa.exact : 1;
   return SW_OK;
@@ -1117,6 +1136,14 @@ int sw_plan_set_path(sw_plan* pl, int32_t path, int32_t chunk_len) {
     pl->fused_grid = units_grid(pl->fx.tiles_y * pl->fx.tiles_z * pl->fx.chunks, 1);
   }
   if (pl->gexec) { cudaGraphExecDestroy(pl->gexec); pl->gexec = nullptr; pl->g_it0 = pl->g_n = -1; }
+  return SW_OK;
+}
+
+int sw_plan_set_on_chip(sw_plan* pl, int32_t blocks) {
+  if (!pl) return fail(SW_ERR_ARG, "null plan");
+  if (pl->dim != 2) return fail(SW_ERR_UNSUPPORTED, "the on-chip loop is for 2D plans");
+  if (blocks < -1) return fail(SW_ERR_ARG, "blocks must be -1 (all), 0 (off) or the SMs to take at most");
+  setup_resident(pl, blocks);
   return SW_OK;
 }
 

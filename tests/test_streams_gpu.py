@@ -1,7 +1,8 @@
 """Solvers on streams of their own: a plan built and first run on a side stream
 while another host thread keeps the default stream busy gives the bits of one
 that has the device to itself (the device words of a plan are zero before any
-stream can reach them)."""
+stream can reach them); several 2D solvers whose on-chip loops share the device
+keep their bits; and a loop that the device refuses to hold is replayed."""
 import threading
 
 import pytest
@@ -84,3 +85,49 @@ def test_first_run_on_a_side_stream(cuda, run, case):
                 got = run(c)
             for k in ref:
                 assert got[k].tobytes() == ref[k].tobytes(), k
+
+
+def _solvers(n, blocks, shape=(121, 90), nt=120):
+    out = []
+    for k in range(n):
+        w = product2d(case2d(shape=shape, nt=nt, nrec=5, seed=k, MT="explosive", src_scale=1e5))
+        w.set_on_chip(blocks)
+        out.append(w)
+    return out
+
+
+@pytest.mark.parametrize("blocks", [-1, 20, 1])
+def test_several_solvers_on_streams(cuda, blocks):
+    refs = _solvers(6, 0)
+    for w in refs:
+        w.run(w.nt)
+        assert w._plans[0].info()["on_chip_tiles"] == 0
+    ws = _solvers(6, blocks)
+    streams = [torch.cuda.Stream() for _ in ws]
+    torch.cuda.synchronize()
+    for w, s in zip(ws, streams):
+        with torch.cuda.stream(s):
+            w.run(50)
+            w.run(w.nt - 50, it0=50)
+    torch.cuda.synchronize()
+    for w, r in zip(ws, refs):
+        tiles = w._plans[0].info()["on_chip_tiles"]
+        assert 0 < tiles <= (blocks if blocks > 0 else 1000) or blocks == 1
+        a, b = _state(w, w._plans[0], F2), _state(r, r._plans[0], F2)
+        for k in a:
+            assert a[k].tobytes() == b[k].tobytes(), k
+
+
+def test_refused_launch_is_replayed(cuda):
+    """More tiles than the device has SMs can never be resident at once: the
+    cooperative launch is refused, and the run replays the two launches."""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    (ref,), (w,) = _solvers(1, 0, shape=(403, 391)), _solvers(1, 4 * sms, shape=(403, 391))
+    ref.run(ref.nt)
+    assert w._plan(0).info()["on_chip_tiles"] > sms
+    w.run(60)
+    assert w._plan(0).info()["on_chip_tiles"] == 0
+    w.run(w.nt - 60, it0=60)
+    a, b = _state(w, w._plan(0), F2), _state(ref, ref._plan(0), F2)
+    for k in a:
+        assert a[k].tobytes() == b[k].tobytes(), k
