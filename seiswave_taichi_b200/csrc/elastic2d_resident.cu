@@ -551,8 +551,8 @@ k2r_run(const __grid_constant__ Res2<T> rs, int it0, int nsteps, int aea) {
 namespace {
 
 // Shot p cut into tx x tz tiles: the largest shared memory of a tile (0 when a
-// side would be too short), its work per step in warp units and the 8-byte
-// words of its rim buffer.
+// side would be too short), its work per step in warp units, the 8-byte words
+// of its rim buffer.
 template <typename T>
 size_t tile_smem(const P2<T>& p, int N, int tx, int tz, long long* work, int* words, int* width) {
   const int lim = std::max(2 * N, SW_RES_MIN);
@@ -572,7 +572,7 @@ size_t tile_smem(const P2<T>& p, int N, int tx, int tz, long long* work, int* wo
     bz = std::max(bz, j1 - j0);
     nsz = std::max(nsz, ns);
   }
-  // a row counts 2 (3 in an x slab) per 32 columns; a rim packet costs about
+  // a row counts 32 (48 in an x slab) per 32 columns; a rim packet costs about
   // a third of a cell
   if (bz > 64) return SIZE_MAX;
   *width = bz <= 32 ? 32 : 64;
@@ -583,19 +583,30 @@ size_t tile_smem(const P2<T>& p, int N, int tx, int tz, long long* work, int* wo
 
 }  // namespace
 
+// Tiles of up to SW_RES_FLOOR work all take the same time, that of an exchange
+// and one unit's latency, so among those the split with the fewest tiles is
+// taken: the SMs that it leaves are free for other solvers' runs.  One solver
+// (us per step, tiles in brackets): float order 2 121 x 90 [110] 3.61, [30] 3.45,
+// [18] 4.59; 200^2 [136] 3.46, [105] 3.58, [77] 3.75, [63] 4.65; order 4 200^2
+// [136] 3.80, [91] 4.06; float64 order 4 121 x 90 [110] 4.74, [44] 4.64, [24] 6.04.
+// Four solvers of 121 x 90 on streams of their own, us per step for all: 14.1
+// with the least work per tile, 10.4 replayed, 3.7 with this rule.
 template <typename T>
 bool sw2r_tiles(const P2<T>& p, int N, int blocks, size_t smem, int* tx, int* tz, int* words,
                 size_t* bytes, int* got) {
   if (N > SW_RES_ORDER) return false;
   long long best = -1;
+  int tiles = 0;
   for (int b = 1; b <= blocks; ++b)
     for (int a = 1; a * b <= blocks; ++a) {
       long long work;
       int w, bw;
       const size_t s = tile_smem(p, N, a, b, &work, &w, &bw);
       if (s == 0) break;  // shorter rows only from here on
-      if (s > smem || (best >= 0 && work >= best)) continue;
+      if (work <= SW_RES_FLOOR) work = 0;
+      if (s > smem || (best >= 0 && (work > best || (work == best && a * b >= tiles)))) continue;
       best = work;
+      tiles = a * b;
       *tx = a;
       *tz = b;
       *words = w;

@@ -11,6 +11,7 @@ namespace sw {
 #define SW_RES_ORDER 4   // highest order with an on-chip loop
 #define SW_RES_RECV 512  // receivers of one tile kept in its shared-memory table
 #define SW_RES_MIN 8     // smallest tile side
+#define SW_RES_FLOOR 540 // work of a tile (about its cells) below which less saves no time
 #define SW_RES_STEPS 4   // fewest steps of a run that the on-chip loop takes
 
 // One launch: the shot and its tx x tz tiles, one per block; tile (a, b) covers
@@ -52,7 +53,8 @@ __host__ __device__ __forceinline__ size_t res2_smem(int bx, int bz, int width, 
 }
 
 // Tiles for shot p on at most `blocks` SMs with `smem` bytes each: the split
-// with the least work per tile, or false when none fits.  *words: 8-byte words
+// with the least work per tile (the fewest tiles among those of at most
+// SW_RES_FLOOR), or false when none fits.  *words: 8-byte words
 // of one rim buffer, *width: the row block's width.
 template <typename T>
 bool sw2r_tiles(const P2<T>& p, int N, int blocks, size_t smem, int* tx, int* tz, int* words, size_t* bytes,

@@ -131,3 +131,12 @@ def test_refused_launch_is_replayed(cuda):
     a, b = _state(w, w._plan(0), F2), _state(ref, ref._plan(0), F2)
     for k in a:
         assert a[k].tobytes() == b[k].tobytes(), k
+
+
+def test_small_grids_leave_room(cuda):
+    """A small grid takes no more SMs than save it time, so that several
+    solvers' on-chip loops can be resident at once."""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    for shape, n in (((60, 64), 8), ((121, 90), 4), ((160, 160), 2)):
+        (w,) = _solvers(1, -1, shape=shape)
+        assert 0 < n * w._plan(0).info()["on_chip_tiles"] <= sms
