@@ -488,6 +488,18 @@ int check_it(sw_plan* pl, int it0, int n) {
 }
 
 
+// Lets this thread allocate (and query events) while another thread captures a
+// stream in the global mode, torch.cuda.graph's default: there such a call
+// would fail and break the other thread's capture.  A run of a plan that exists
+// made no such call before it had scratch of its own.
+struct CaptureTolerant {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  CaptureTolerant() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  ~CaptureTolerant() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  CaptureTolerant(const CaptureTolerant&) = delete;
+  CaptureTolerant& operator=(const CaptureTolerant&) = delete;
+};
+
 // Device scratch that holds zeros when the call returns.  The kernels that use
 // it run on the caller's streams, and nothing orders those behind a memset of
 // the default stream: a unit counter or barrier word that a pass read before
@@ -496,6 +508,7 @@ int check_it(sw_plan* pl, int it0, int n) {
 cudaError_t zeroed_scratch(void** out, size_t bytes) {
   void* b = nullptr;
   cudaStream_t st = nullptr;
+  CaptureTolerant others;
   cudaError_t e = cudaMalloc(&b, bytes);
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaMemsetAsync(b, 0, bytes, st);
@@ -695,6 +708,7 @@ void setup_staged(sw_plan* pl) {
 bool pitch_ready(sw_plan* pl, int nsteps, cudaStream_t st) {
   if (pl->dim != 3 || !pl->pitch_ok || pl->path != 0 || pl->aea || nsteps < SW_PITCH_STEPS) return false;
   if (pl->pitch_buf) return true;
+  CaptureTolerant others;
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) {
     cudaGetLastError();
@@ -872,6 +886,7 @@ bool launch_refused(cudaError_t e) {
 // graph is refused there, and stays refused)
 cudaError_t resident_run(sw_plan* pl, int it0, int nsteps, cudaStream_t st, bool* done) {
   *done = false;
+  CaptureTolerant others;
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) {
     cudaGetLastError();

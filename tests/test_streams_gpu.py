@@ -2,7 +2,9 @@
 while another host thread keeps the default stream busy gives the bits of one
 that has the device to itself (the device words of a plan are zero before any
 stream can reach them); several 2D solvers whose on-chip loops share the device
-keep their bits; and a loop that the device refuses to hold is replayed."""
+keep their bits; a loop that the device refuses to hold is replayed; and a
+plan's first run, which allocates its scratch, leaves another thread's stream
+capture whole."""
 import threading
 
 import pytest
@@ -140,3 +142,39 @@ def test_small_grids_leave_room(cuda):
     for shape, n in (((60, 64), 8), ((121, 90), 4), ((160, 160), 2)):
         (w,) = _solvers(1, -1, shape=shape)
         assert 0 < n * w._plan(0).info()["on_chip_tiles"] <= sms
+
+
+@pytest.mark.parametrize("case", [
+    lambda: (product2d(case2d(nt=60, nrec=5)), "vz", lambda w: w.run(60)),
+    lambda: (product3d(case3d(shape=(130, 111, 105), nt=20)), "vz", lambda w: w.run(20, use_graph=False)),
+], ids=["on_chip", "pitched"])
+def test_first_run_beside_a_capture(cuda, case):
+    (ref, f, run), (w, _, _) = case(), case()
+    run(ref)
+    plan = w._plan(0) if hasattr(w, "_plans") else w._build_plan()  # built before the capture
+    s = torch.cuda.Stream()
+    x = torch.ones(1000, device="cuda")
+    torch.cuda.synchronize()
+    failed = []
+
+    def other():
+        try:
+            with torch.cuda.stream(s):
+                run(w)
+        except Exception as e:  # noqa: BLE001 - reported below
+            failed.append(e)
+
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):  # the global mode
+        x += 1
+        t = threading.Thread(target=other)
+        t.start()
+        t.join()
+        x *= 2
+    assert not failed
+    g.replay()
+    torch.cuda.synchronize()
+    plan.status()
+    assert x.unique().tolist() == [4.0]
+    assert to_np(getattr(w, f)).tobytes() == to_np(getattr(ref, f)).tobytes()
+    assert to_np(w.data).tobytes() == to_np(ref.data).tobytes()
