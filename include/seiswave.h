@@ -210,7 +210,8 @@ SW_API int sw_plan_status(sw_plan* plan, void* stream);
  * size measured; sw_step keeps the two launches), [1] constant-divisor fast path verified, [2] staged
  * path available, [3] its grid, [4] its x-chunk length, [5] fused path set
  * up, [6] its grid (2D: the tiles of the on-chip loop, 0 where sw_run replays
- * the launches), [7] its x-chunk length, [8] exact numerics (see
+ * the launches), [7] its x-chunk length (2D: the tiles of the last such run, 0
+ * if it was replayed), [8] exact numerics (see
  * sw_plan_set_exact).  info must hold 9 int32. */
 SW_API int sw_plan_info(sw_plan* plan, int32_t* info);
 
@@ -225,7 +226,9 @@ SW_API int sw_plan_set_path(sw_plan* plan, int32_t path, int32_t chunk_len);
  * of a step), n > 0 at most n, one tile each.  The loop holds its SMs, and most
  * of their registers and shared memory, from its first step to its last, so
  * solvers on several streams run side by side only while their tiles fit the
- * device together.  A launch that the device refuses -- more tiles than can be
+ * device together: by default runs that meet others in flight on other
+ * streams, now or at one of the last 8 launches, take their share of the SMs,
+ * or are replayed where that is too little for their grid.  A launch that the device refuses -- more tiles than can be
  * resident at once on what the stream's context owns -- is not an error: this
  * and the later runs replay the launches.  All choices give the same bits.
  * No reference counterpart. */

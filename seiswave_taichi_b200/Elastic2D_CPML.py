@@ -331,9 +331,10 @@ class ElasticWAVE:
     def set_on_chip(self, blocks: int = -1):
         """The SMs that run()'s on-chip loop may take: -1 all, 0 none (its
         steps are replayed as two launches each), n > 0 at most n.  The loop
-        holds its SMs for the whole run, so of several solvers on streams of
-        their own only those run side by side whose tiles fit the GPU together
-        (Plan.info()["on_chip_tiles"]); the results do not depend on it."""
+        holds its SMs for the whole run, so solvers on streams of their own run
+        side by side only while their tiles fit the GPU together
+        (Plan.info()["on_chip_tiles"]); by default runs that meet others in
+        flight take a share of the SMs each.  The results do not depend on it."""
         if int(blocks) < -1:
             raise ValueError("blocks is -1 (all), 0 (off) or the SMs to take at most")
         self._on_chip = int(blocks)

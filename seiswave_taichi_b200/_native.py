@@ -328,7 +328,8 @@ class Plan:
              "staged_chunk": a[4], "fused": bool(a[5]), "fused_grid": a[6], "fused_chunk": a[7],
              "exact": bool(a[8])}
         if not self._three_d:
-            d["on_chip_tiles"], d["fused_grid"] = d["fused_grid"], 0
+            d["on_chip_tiles"], d["last_run_tiles"] = a[6], a[7]
+            d["fused_grid"] = d["fused_chunk"] = 0
         return d
 
     def set_free_surface(self, on: bool = True) -> None:

@@ -161,6 +161,12 @@ __global__ void k_count_nonfinite(const T* a, long long n, unsigned long long* o
 // (about as much traffic as 1.2 steps)
 #define SW_PITCH_STEPS 6
 
+// tiles of the 2D on-chip loop (tx = 0: none fit)
+struct ResTiles {
+  int tx = 0, tz = 0, words = 0, width = 0;
+  size_t smem = 0;
+};
+
 struct sw_plan {
   int dim = 0, scheme = 0, dtype = 0, order = 0, nt_max = 0;
   sw::P2<float> p2f{};
@@ -204,10 +210,18 @@ struct sw_plan {
   bool path_chosen = false;  // by sw_plan_set_path
   unsigned int* d_bar = nullptr;  // 2D persistent path: grid-barrier arrival and generation words
   bool aea = false;               // free-surface hook before every step (sw_plan_set_free_surface)
-  // 2D on-chip loop (sw_run of path 0): tiles (0: not available) and the rim inbox
-  int res_tx = 0, res_tz = 0, res_words = 0, res_width = 0;
-  size_t res_smem = 0, inbox_words = 0;
+  // 2D on-chip loop (sw_run of path 0): tiles, the SMs they may take (-1 all),
+  // tiles for one in res_share of the SMs, tiles of the last run (0: replayed)
+  // and the rim inbox
+  ResTiles res, res_part;
+  int res_most = -1, res_share = 1, res_last = 0;
+  size_t inbox_words = 0;
   uint64_t* d_inbox = nullptr;
+  // its run in flight (on_chip_runs; the last three under that lock)
+  cudaEvent_t res_done = nullptr;
+  int res_device = -1;
+  cudaStream_t res_stream = nullptr;
+  bool res_launching = false;
 };
 
 namespace {
@@ -840,38 +854,132 @@ bool resident_covers(const sw_plan* pl) {
          pl->gather_in_stress;
 }
 
-// most: the SMs it may take, -1 all of the device (sw_plan_set_on_chip)
-void setup_resident(sw_plan* pl, int most) {
-  pl->res_tx = 0;
-  if (!resident_covers(pl)) return;
+// tiles for at most `most` SMs (-1: all of the device), or for one in `share` of them
+ResTiles resident_tiles(const sw_plan* pl, int most, int share) {
+  ResTiles t;
+  if (!resident_covers(pl)) return t;
   int blocks;
   size_t smem;
   resident_limits(&blocks, &smem);
   if (blocks > 0 && most >= 0) blocks = most;
-  int tx, tz, words, width;
-  size_t bytes;
-  const bool ok = pl->dtype == SW_F32 ? sw::sw2r_tiles<float>(pl->p2f, pl->order, blocks, smem, &tx, &tz, &words, &bytes, &width)
-                                      : sw::sw2r_tiles<double>(pl->p2d, pl->order, blocks, smem, &tx, &tz, &words, &bytes, &width);
-  if (!ok) return;
-  pl->res_tx = tx;
-  pl->res_tz = tz;
-  pl->res_words = words;
-  pl->res_width = width;
-  pl->res_smem = bytes;
+  blocks /= share;
+  const bool ok =
+      pl->dtype == SW_F32
+          ? sw::sw2r_tiles<float>(pl->p2f, pl->order, blocks, smem, &t.tx, &t.tz, &t.words, &t.smem, &t.width)
+          : sw::sw2r_tiles<double>(pl->p2d, pl->order, blocks, smem, &t.tx, &t.tz, &t.words, &t.smem, &t.width);
+  return ok ? t : ResTiles();
+}
+
+void setup_resident(sw_plan* pl, int most) {
+  pl->res = resident_tiles(pl, most, 1);
+  pl->res_most = most;
+  pl->res_share = 1;
 }
 
 template <typename T>
-cudaError_t resident_run_t(sw_plan* pl, const sw::P2<T>& p, int it0, int nsteps, cudaStream_t st) {
+cudaError_t resident_run_t(sw_plan* pl, const sw::P2<T>& p, const ResTiles& t, int it0, int nsteps, cudaStream_t st) {
   sw::Res2<T> r{};
   r.shot = p;
-  r.tx = pl->res_tx;
-  r.tz = pl->res_tz;
-  r.stride = pl->res_words;
-  r.width = pl->res_width;
-  r.smem = pl->res_smem;
+  r.tx = t.tx;
+  r.tz = t.tz;
+  r.stride = t.words;
+  r.width = t.width;
+  r.smem = t.smem;
   r.inbox = pl->d_inbox;
   r.err = pl->d_err;
   return sw::sw2r_run<T>(r, pl->scheme, pl->order, it0, nsteps, pl->aea ? 1 : 0, st);
+}
+
+// Plans whose run, on the chip or replayed in its place, may be in flight.  A run holds its SMs to its end, so
+// where runs of several streams meet, each takes a share of the SMs and leaves
+// theirs to the others: they then run side by side, as replayed launches do.
+// How many meet is the most that were in flight together at one of the last
+// launches (the first of a burst finds the device empty).  Us per step for all,
+// each on the whole device / replayed / with shares: 8 solvers of 200^2
+// 28.0 / 12.8 / 11.2, 4 of 320^2 17.9 / 12.8 / 9.5, 4 of 400^2 20.1 / 18.1 /
+// 18.1, 8 of 1000 x 420 77 / 135 / 77.  The choice moves no bits.
+struct OnChipRuns {
+  static constexpr int LAST = 8;  // as many as the smallest share: a burst's first runs look back over the last burst
+  std::mutex mu;
+  std::vector<sw_plan*> plans;
+  int device[LAST] = {}, met[LAST] = {};  // of the last launches
+  unsigned launches = 0;
+};
+OnChipRuns& on_chip_runs() {
+  static OnChipRuns* r = new OnChipRuns;  // plans may be destroyed after the static objects
+  return *r;
+}
+
+// lists pl as launching on st; returns how many runs, itself included, share the device
+int on_chip_begin(sw_plan* pl, cudaStream_t st) {
+  auto& r = on_chip_runs();
+  std::lock_guard<std::mutex> lock(r.mu);
+  int n = 1;
+  size_t kept = 0;
+  for (sw_plan* o : r.plans) {
+    const bool in_flight = o->res_launching || cudaEventQuery(o->res_done) == cudaErrorNotReady;
+    if (o == pl || !in_flight) continue;
+    r.plans[kept++] = o;
+    if (o->res_device == pl->res_device && o->res_stream != st) ++n;
+  }
+  cudaGetLastError();  // not ready is an answer
+  r.plans.resize(kept);
+  r.plans.push_back(pl);
+  pl->res_launching = true;
+  pl->res_stream = st;
+  const unsigned at = r.launches++ % OnChipRuns::LAST;
+  r.device[at] = pl->res_device;
+  r.met[at] = n;
+  for (int q = 0; q < OnChipRuns::LAST; ++q)
+    if (r.device[q] == pl->res_device) n = std::max(n, r.met[q]);
+  return n;
+}
+// a run's listing: from before the choice of its tiles until its work, on the
+// chip or replayed, is enqueued and marked by its event
+struct OnChipRun {
+  sw_plan* pl = nullptr;
+  cudaStream_t st = nullptr;
+  int begin(sw_plan* p, cudaStream_t s) {
+    pl = p;
+    st = s;
+    return on_chip_begin(p, s);
+  }
+  ~OnChipRun() {
+    if (!pl) return;
+    if (cudaEventRecord(pl->res_done, st) != cudaSuccess) cudaGetLastError();
+    std::lock_guard<std::mutex> lock(on_chip_runs().mu);
+    pl->res_launching = false;
+  }
+};
+void on_chip_forget(sw_plan* pl) {
+  auto& r = on_chip_runs();
+  std::lock_guard<std::mutex> lock(r.mu);
+  for (size_t q = 0; q < r.plans.size(); ++q)
+    if (r.plans[q] == pl) {
+      r.plans[q] = r.plans.back();
+      r.plans.pop_back();
+      return;
+    }
+}
+
+// The tiles of a run that shares the device with n - 1 others: the plan's own
+// where they fit its share, else as many as the share holds.  A grid too large
+// for its share takes its turn on the whole device if one run alone fills the
+// memory system about as well as several replays do (1 MB per field: 3 solvers
+// of 700 x 400 22.9 us on the chip, 23.0 replayed; 4 of 400^2 19.9 and 18.1),
+// else it is replayed (no tiles).
+ResTiles shared_tiles(sw_plan* pl, int n) {
+  int blocks;
+  size_t smem;
+  resident_limits(&blocks, &smem);
+  n = std::min(n, 8);
+  if (n == 1 || pl->res_most >= 0 || pl->res.tx * pl->res.tz <= blocks / n) return pl->res;
+  if (pl->res_share != n) {
+    pl->res_part = resident_tiles(pl, -1, n);
+    pl->res_share = n;
+  }
+  if (pl->res_part.tx == 0 && pl->ncell * dsize(pl->dtype) >= 1000000) return pl->res;
+  return pl->res_part;
 }
 
 // The launch's refusals: its tiles cannot all be resident at once on what this
@@ -882,21 +990,26 @@ bool launch_refused(cudaError_t e) {
 
 // *done = false when the graph of the other path has to run instead: the
 // scratch could not be allocated, the launch was refused (the plan then keeps
-// to the other path), or the stream is being captured (a run that replays a
-// graph is refused there, and stays refused)
-cudaError_t resident_run(sw_plan* pl, int it0, int nsteps, cudaStream_t st, bool* done) {
+// to the other path), too many runs share the device, or the stream is being
+// captured (a run that replays a graph is refused there, and stays refused)
+cudaError_t resident_run(sw_plan* pl, int it0, int nsteps, cudaStream_t st, OnChipRun& run, bool* done) {
   *done = false;
+  pl->res_last = 0;
   CaptureTolerant others;
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) {
+  if (cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone ||
+      plan_words(pl) != cudaSuccess) {
     cudaGetLastError();
     return cudaSuccess;
   }
-  const size_t words = 2 * (size_t)pl->res_tx * pl->res_tz * pl->res_words;
-  if (plan_words(pl) != cudaSuccess) {
+  if (!pl->res_done && (cudaGetDevice(&pl->res_device) != cudaSuccess ||
+                        cudaEventCreateWithFlags(&pl->res_done, cudaEventDisableTiming) != cudaSuccess)) {
     cudaGetLastError();
     return cudaSuccess;
   }
+  const ResTiles t = shared_tiles(pl, run.begin(pl, st));
+  if (t.tx == 0) return cudaSuccess;
+  const size_t words = 2 * (size_t)t.tx * t.tz * t.words;
   if (pl->inbox_words < words) {
     if (pl->d_inbox) cudaFree(pl->d_inbox);
     pl->d_inbox = nullptr;
@@ -907,14 +1020,15 @@ cudaError_t resident_run(sw_plan* pl, int it0, int nsteps, cudaStream_t st, bool
     }
     pl->inbox_words = words;
   }
-  const cudaError_t e = pl->dtype == SW_F32 ? resident_run_t<float>(pl, pl->p2f, it0, nsteps, st)
-                                            : resident_run_t<double>(pl, pl->p2d, it0, nsteps, st);
+  cudaError_t e = pl->dtype == SW_F32 ? resident_run_t<float>(pl, pl->p2f, t, it0, nsteps, st)
+                                      : resident_run_t<double>(pl, pl->p2d, t, it0, nsteps, st);
   if (launch_refused(e)) {
     cudaGetLastError();
-    pl->res_tx = 0;
+    pl->res = ResTiles();
     return cudaSuccess;
   }
   *done = true;
+  pl->res_last = t.tx * t.tz;
   return e;
 }
 
@@ -1118,8 +1232,8 @@ int sw_plan_info(sw_plan* pl, int32_t* info) {
   }
   info[4] = pl->staged ? pl->sa.chunk_len : 0;
   info[5] = pl->fused ? 1 : 0;
-  info[6] = pl->dim == 2 ? pl->res_tx * pl->res_tz : (pl->fused ? pl->fused_grid : 0);
-  info[7] = pl->fused ? pl->fx.chunk_len : 0;
+  info[6] = pl->dim == 2 ? pl->res.tx * pl->res.tz : (pl->fused ? pl->fused_grid : 0);
+  info[7] = pl->dim == 2 ? pl->res_last : (pl->fused ? pl->fx.chunk_len : 0);
   info[8] = pl->staged ? pl->sa.exact : 1;
   return SW_OK;
 }
@@ -1189,6 +1303,10 @@ int sw_plan_destroy(sw_plan* pl) {
   if (pl->fused_buf) cudaFree(pl->fused_buf);
   if (pl->d_err) cudaFree(pl->d_err);
   if (pl->d_bar) cudaFree(pl->d_bar);
+  if (pl->res_done) {
+    on_chip_forget(pl);
+    cudaEventDestroy(pl->res_done);
+  }
   if (pl->d_inbox) cudaFree(pl->d_inbox);
   if (pl->pitch_buf) cudaFree(pl->pitch_buf);
   delete pl;
@@ -1232,9 +1350,10 @@ int sw_run(sw_plan* pl, int32_t it0, int32_t nsteps, int32_t use_graph, void* st
     if (e != cudaSuccess) return cuda_fail(e, "sw_run");
     return SW_OK;
   }
-  if (pl->path == 0 && pl->res_tx > 0 && nsteps >= SW_RES_STEPS) {
+  OnChipRun run;
+  if (pl->path == 0 && pl->res.tx > 0 && nsteps >= SW_RES_STEPS) {
     bool done;
-    e = resident_run(pl, it0, nsteps, st, &done);
+    e = resident_run(pl, it0, nsteps, st, run, &done);
     if (e != cudaSuccess) return cuda_fail(e, "sw_run: on-chip loop");
     if (done) return SW_OK;
   }

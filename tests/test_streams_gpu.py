@@ -178,3 +178,48 @@ def test_first_run_beside_a_capture(cuda, case):
     assert x.unique().tolist() == [4.0]
     assert to_np(getattr(w, f)).tobytes() == to_np(getattr(ref, f)).tobytes()
     assert to_np(w.data).tobytes() == to_np(ref.data).tobytes()
+
+
+@pytest.mark.parametrize("shape,fits", [((121, 90), 4), ((200, 200), 1), ((400, 400), 1), ((700, 400), 1)])
+def test_runs_in_flight_share_the_device(cuda, shape, fits):
+    """Runs that meet others in flight on other streams take their share of the
+    SMs (or, too large for it, are replayed, or wait for the whole device), the
+    first of the next burst too; alone again a solver takes its own tiles.  Same
+    bits throughout."""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    n, nt = 6, 60
+    ref = _solvers(1, 0, shape, nt)[0]
+    ref.run(nt)
+    want = _state(ref, ref._plans[0], F2)
+    ws = [product2d(case2d(shape=shape, nt=nt, nrec=5, seed=0, MT="explosive", src_scale=1e5)) for _ in range(n)]
+    plans = [w._plan(0) for w in ws]
+    own = plans[0].info()["on_chip_tiles"]
+
+    def alone():
+        for _ in range(8):  # one stream: each run behind the last, not beside it
+            ws[-1].run(4)
+        assert plans[-1].info()["last_run_tiles"] == own
+
+    alone()
+    streams = [torch.cuda.Stream() for _ in range(n)]
+    for burst in range(2):
+        torch.cuda.synchronize()
+        for q, (w, s) in enumerate(zip(ws, streams)):
+            with torch.cuda.stream(s):
+                torch.cuda._sleep(200_000_000)  # its run is in flight for the others
+                w.reset()
+                w.run(nt)
+            last = plans[q].info()["last_run_tiles"]
+            met = q + 1 if burst == 0 else n
+            if met <= fits or shape == (700, 400):  # that grid runs in turn, on the whole device
+                assert last == own
+            else:
+                assert last <= sms // met
+                assert last > 0 or shape == (400, 400)
+        for w, p, s in zip(ws, plans, streams):
+            with torch.cuda.stream(s):
+                got = _state(w, p, F2)
+            for k in want:
+                assert got[k].tobytes() == want[k].tobytes(), k
+    alone()
+    torch.cuda.synchronize()
