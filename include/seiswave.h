@@ -190,8 +190,13 @@ SW_API int sw_check_division(float divisor, int32_t mode, uint64_t* mismatches, 
 /* Block until the stream is idle and report a device-side failure recorded
  * by the plan's kernels since the previous status read (SW_ERR_TIMEOUT: a
  * bounded wait for TMA data, for a tile's rims in the 2D on-chip run or for a
- * grid barrier of the 2D persistent run gave up); a failure is reported once and then cleared, so a caller may retry.  No reference counterpart (the reference has no error
- * path); it is the status read the drivers' loops can add after run(). */
+ * grid barrier of the 2D persistent run gave up); a failure is reported once
+ * and then cleared, so a caller may retry.  After a 2D on-chip run that gave up
+ * the fields and memory variables are those from before the run (its tiles
+ * agree before any writes back), the traces of its steps are undefined; after
+ * the other timeouts all are undefined.  No reference counterpart (the
+ * reference has no error path); it is the status read the drivers' loops can
+ * add after run(). */
 SW_API int sw_plan_status(sw_plan* plan, void* stream);
 
 /* Describe the plan's execution path: info[0] current path of sw_step/sw_run
@@ -233,6 +238,11 @@ SW_API int sw_plan_set_path(sw_plan* plan, int32_t path, int32_t chunk_len);
  * and the later runs replay the launches.  All choices give the same bits.
  * No reference counterpart. */
 SW_API int sw_plan_set_on_chip(sw_plan* plan, int32_t blocks);
+
+/* Failure injection for tests, no reference counterpart: in the next on-chip
+ * run of a 2D plan, tile `tile` (of sw_plan_info's count) behaves as if its
+ * neighbours' rims of the last step had not come. */
+SW_API int sw_plan_stop_on_chip(sw_plan* plan, int32_t tile);
 
 /* Free-surface mode: when on != 0 every step first applies the reference's
  * free-surface hook AEA, as a driver loop `AEA(); update_SSG_VS(i)` does

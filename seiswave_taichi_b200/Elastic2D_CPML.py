@@ -364,6 +364,12 @@ class ElasticWAVE:
         from .adjoint import ForwardOp2D
         return ForwardOp2D.apply(vp, vs, rho, self, int(checkpoint_every), scheme)
 
+    def check_status(self) -> None:
+        """Wait for the steps enqueued so far and raise SeisWaveError if a
+        bounded device wait of theirs gave up."""
+        for plan in self._plans.values():
+            plan.status(self._stream())
+
     def check_finite(self) -> int:
         return self._plan(N.SW2D_SSG_VS).check_finite(self._stream())
 

@@ -416,6 +416,12 @@ class Elastic3DBase:
         cache_store(key, best)
         return best
 
+    def check_status(self) -> None:
+        """Wait for the steps enqueued so far and raise SeisWaveError if a
+        bounded device wait of theirs gave up."""
+        if self._plan is not None:
+            self._plan.status(self._stream())
+
     def check_finite(self) -> int:
         """Number of non-finite wavefield values (0 when the state is finite)."""
         return (self._plan or self._build_plan()).check_finite(self._stream())

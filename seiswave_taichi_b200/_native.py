@@ -36,6 +36,7 @@ EXPORTS = (
     "sw_mlp_backward", "sw2d_abc_adjoint", "sw3d_snapshot_elems", "sw3d_record", "sw3d_adjoint_run",
     "sw3d_abc_correct", "sw3d_abc_features", "sw3d_abc_adjoint", "sw3d_mlp_grad", "sw3d_mlp_forward",
     "sw3d_mlp_backward", "sw_segy_decode", "sw_plan_set_free_surface", "sw_plan_set_on_chip",
+    "sw_plan_stop_on_chip",
 )
 
 SW_ABC_DEPTH = 6
@@ -160,6 +161,7 @@ def load() -> C.CDLL:
         "sw_segy_decode": (C.c_int, [vp, C.c_int64, C.c_int32, C.c_int32, vp, vp, vp]),
         "sw_plan_set_free_surface": (C.c_int, [vp, C.c_int32]),
         "sw_plan_set_on_chip": (C.c_int, [vp, C.c_int32]),
+        "sw_plan_stop_on_chip": (C.c_int, [vp, C.c_int32]),
         "sw2d_record": (C.c_int, [vp, C.c_int32, C.c_int32, vp, vp]),
         "sw2d_adjoint_run": (C.c_int, [vp, C.POINTER(Adjoint2D), C.c_int32, C.c_int32, vp, vp]),
         "sw2d_batch_create": (C.c_int, [C.POINTER(Desc2D), C.c_int32, C.POINTER(vp)]),
@@ -339,6 +341,10 @@ class Plan:
     def set_on_chip(self, blocks: int) -> None:
         """2D: the SMs the on-chip loop of run may take (-1 all, 0 off)."""
         check(load().sw_plan_set_on_chip(self._h, int(blocks)))
+
+    def stop_on_chip(self, tile: int) -> None:
+        """2D, for tests: a tile gives up in the last step of the next on-chip run."""
+        check(load().sw_plan_stop_on_chip(self._h, int(tile)))
 
     def set_exact(self, exact: bool) -> None:
         """Numeric mode of the staged path (the other paths are always exact)."""

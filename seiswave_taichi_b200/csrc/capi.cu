@@ -217,6 +217,7 @@ struct sw_plan {
   int res_most = -1, res_share = 1, res_last = 0;
   size_t inbox_words = 0;
   uint64_t* d_inbox = nullptr;
+  int res_stop_tile = -1;  // sw_plan_stop_on_chip
   // its run in flight (on_chip_runs; the last three under that lock)
   cudaEvent_t res_done = nullptr;
   int res_device = -1;
@@ -887,6 +888,8 @@ cudaError_t resident_run_t(sw_plan* pl, const sw::P2<T>& p, const ResTiles& t, i
   r.smem = t.smem;
   r.inbox = pl->d_inbox;
   r.err = pl->d_err;
+  r.stop_tile = pl->res_stop_tile;
+  pl->res_stop_tile = -1;
   return sw::sw2r_run<T>(r, pl->scheme, pl->order, it0, nsteps, pl->aea ? 1 : 0, st);
 }
 
@@ -1009,7 +1012,7 @@ cudaError_t resident_run(sw_plan* pl, int it0, int nsteps, cudaStream_t st, OnCh
   }
   const ResTiles t = shared_tiles(pl, run.begin(pl, st));
   if (t.tx == 0) return cudaSuccess;
-  const size_t words = 2 * (size_t)t.tx * t.tz * t.words;
+  const size_t words = sw::res2_inbox_words(t.tx, t.tz, t.words);
   if (pl->inbox_words < words) {
     if (pl->d_inbox) cudaFree(pl->d_inbox);
     pl->d_inbox = nullptr;
@@ -1273,6 +1276,14 @@ int sw_plan_set_on_chip(sw_plan* pl, int32_t blocks) {
   if (pl->dim != 2) return fail(SW_ERR_UNSUPPORTED, "the on-chip loop is for 2D plans");
   if (blocks < -1) return fail(SW_ERR_ARG, "blocks must be -1 (all), 0 (off) or the SMs to take at most");
   setup_resident(pl, blocks);
+  return SW_OK;
+}
+
+int sw_plan_stop_on_chip(sw_plan* pl, int32_t tile) {
+  if (!pl) return fail(SW_ERR_ARG, "null plan");
+  if (pl->dim != 2) return fail(SW_ERR_UNSUPPORTED, "the on-chip loop is for 2D plans");
+  if (tile < 0 || tile >= pl->res.tx * pl->res.tz) return fail(SW_ERR_ARG, "no such tile");
+  pl->res_stop_tile = tile;
   return SW_OK;
 }
 

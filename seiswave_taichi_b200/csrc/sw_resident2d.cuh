@@ -17,7 +17,8 @@ namespace sw {
 // One launch: the shot and its tx x tz tiles, one per block; tile (a, b) covers
 // the rows between the cuts a and a+1 (res2_cut_x) and the columns between the
 // cuts b and b+1 (res2_cut_z).  A tile's rim buffers (one per phase, `stride`
-// 8-byte words each) start at word 2*tile*stride of the inbox.
+// 8-byte words each) start at word 2*tile*stride of the inbox; the tiles'
+// agreement at the end of the run takes the word behind them.
 template <typename T>
 struct Res2 {
   P2<T> shot;
@@ -26,7 +27,10 @@ struct Res2 {
   size_t smem;
   uint64_t* inbox;
   int* err;
+  int stop_tile;  // this tile behaves as if its last step's rims had not come (-1: none)
 };
+
+inline size_t res2_inbox_words(int tx, int tz, int stride) { return 2 * (size_t)tx * tz * stride + 1; }
 
 // first column of tile t of tz: equal widths
 __host__ __device__ __forceinline__ int res2_cut_z(int nz, int t, int tz) { return (int)((long long)t * nz / tz); }

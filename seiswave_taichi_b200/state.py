@@ -103,7 +103,8 @@ def read(path, arrays: dict, config: dict) -> dict:
 
 def run_checked(solver, nt, it0: int, every: int, **run_kw) -> None:
     """solver.run() over steps it0 .. it0+nt-1 in segments of `every` steps,
-    scanning the wavefields for NaN/Inf after each segment."""
+    reading the plans' status (a bounded device wait that gave up raises
+    SeisWaveError) and scanning the wavefields for NaN/Inf after each segment."""
     if every < 1:
         raise ValueError("every must be >= 1")
     it = int(it0)
@@ -112,6 +113,9 @@ def run_checked(solver, nt, it0: int, every: int, **run_kw) -> None:
         n = min(int(every), end - it)
         solver.run(n, it0=it, **run_kw)
         it += n
+        status = getattr(solver, "check_status", None)
+        if status is not None:
+            status()
         bad = solver.check_finite()
         if bad:
             raise NonFiniteError(bad, it - 1)
