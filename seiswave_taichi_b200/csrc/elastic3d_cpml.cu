@@ -54,12 +54,15 @@ __device__ __forceinline__ void cpml3c(const P3<T>& p, int comp, int s, int i, i
   d = div_v(d, cf[2 * n]) + psi;
 }
 
-template <typename T, int N, bool TENSOR>
+// LONG: the launch's first plane is x0 (each_slice), else N.  (As an argument of
+// one kernel for both it cost the float kernels, which are at their register
+// limit, 1 to 4% at 200^3.)
+template <typename T, int N, bool TENSOR, bool LONG>
 __global__ void __launch_bounds__(T3Z * T3Y, SW_C3_MINB)
-k3_velocity(const __grid_constant__ P3<T> p, int it, int force_here) {
+k3_velocity(const __grid_constant__ P3<T> p, int it, int force_here, int x0) {
   const int k = blockIdx.x * T3Z + threadIdx.x;
   const int j = blockIdx.y * T3Y + threadIdx.y;
-  const int i = blockIdx.z + N;
+  const int i = blockIdx.z + (LONG ? x0 : N);
   const int nx = p.nx, ny = p.ny, nz = p.nz;
   if (j < N || j >= ny - N || k < N || k >= nz - N) return;
   const long long sx = (long long)ny * nz, sy = nz;
@@ -121,9 +124,9 @@ k3_velocity(const __grid_constant__ P3<T> p, int it, int force_here) {
   }
 }
 
-template <typename T, int N>
+template <typename T, int N, bool LONG>
 __global__ void __launch_bounds__(T3Z * T3Y, SW_C3_MINB)
-k3_stress(const __grid_constant__ P3<T> p, int it, int inject_next) {
+k3_stress(const __grid_constant__ P3<T> p, int it, int inject_next, int x0) {
   {
     const long long b = blockIdx.x + (long long)gridDim.x * (blockIdx.y + (long long)gridDim.y * blockIdx.z);
     const long long n = (long long)gridDim.x * gridDim.y * gridDim.z * (T3Z * T3Y);
@@ -132,7 +135,7 @@ k3_stress(const __grid_constant__ P3<T> p, int it, int inject_next) {
   }
   const int k = blockIdx.x * T3Z + threadIdx.x;
   const int j = blockIdx.y * T3Y + threadIdx.y;
-  const int i = blockIdx.z + N;
+  const int i = blockIdx.z + (LONG ? x0 : N);
   const int nx = p.nx, ny = p.ny, nz = p.nz;
   if (j < N || j >= ny - N || k < N || k >= nz - N) return;
   const long long sx = (long long)ny * nz, sy = nz;
@@ -257,20 +260,35 @@ __global__ void k3_gather(const __grid_constant__ P3<T> p, int it) {
 // ---------------------------------------------------------------------------
 // host-side launchers
 // ---------------------------------------------------------------------------
-template <typename T, int N>
-static dim3 cell_grid(const P3<T>& p) {
-  return dim3((p.nz + T3Z - 1) / T3Z, (p.ny + T3Y - 1) / T3Y, p.nx - 2 * N);
+// One x plane per blockIdx.z; the planes N .. nx-N-1 in launches of at most
+// SW_GRID_Z planes, the limit of a grid's z extent.  The planes of a pass do not
+// read what it writes.
+template <typename T, int N, typename F>
+static void each_slice(const P3<T>& p, F launch) {
+  for (int x0 = N; x0 < p.nx - N; x0 += SW_GRID_Z) {
+    const int planes = x0 + SW_GRID_Z < p.nx - N ? SW_GRID_Z : p.nx - N - x0;
+    launch(dim3((p.nz + T3Z - 1) / T3Z, (p.ny + T3Y - 1) / T3Y, planes), x0);
+  }
 }
 
 template <typename T, int N>
 static void launch3_velocity(const P3<T>& p, int it, bool tensor, bool force_here, cudaStream_t st) {
-  if (tensor) k3_velocity<T, N, true><<<cell_grid<T, N>(p), dim3(T3Z, T3Y), 0, st>>>(p, it, 0);
-  else k3_velocity<T, N, false><<<cell_grid<T, N>(p), dim3(T3Z, T3Y), 0, st>>>(p, it, force_here ? 1 : 0);
+  each_slice<T, N>(p, [&](dim3 grid, int x0) {
+    const bool slices = p.nx - 2 * N > SW_GRID_Z;
+    auto kern = tensor ? (slices ? k3_velocity<T, N, true, true> : k3_velocity<T, N, true, false>)
+                       : (slices ? k3_velocity<T, N, false, true> : k3_velocity<T, N, false, false>);
+    kern<<<grid, dim3(T3Z, T3Y), 0, st>>>(p, it, !tensor && force_here ? 1 : 0, x0);
+  });
 }
 
 template <typename T, int N>
 static void launch3_stress(const P3<T>& p, int it, bool inject_next, cudaStream_t st) {
-  k3_stress<T, N><<<cell_grid<T, N>(p), dim3(T3Z, T3Y), 0, st>>>(p, it, inject_next ? 1 : 0);
+  P3<T> q = p;
+  each_slice<T, N>(p, [&](dim3 grid, int x0) {
+    auto kern = p.nx - 2 * N > SW_GRID_Z ? k3_stress<T, N, true> : k3_stress<T, N, false>;
+    kern<<<grid, dim3(T3Z, T3Y), 0, st>>>(q, it, inject_next ? 1 : 0, x0);
+    q.nrec = 0;  // recorded by the first launch
+  });
 }
 
 #define SW_ORDER_SWITCH(order, CALL)            \

@@ -58,12 +58,14 @@ __device__ __forceinline__ void split_quotients(T (&x)[K], const Damp<T> (&a)[K]
   }
   cell_quotients<K>(x, d, y, ok);
 }
-template <typename T, int N>
+// LONG: the launch's first plane is x0, else 0 (an argument of one kernel for
+// both costs the float kernels up to 5%)
+template <typename T, int N, bool LONG>
 __global__ void __launch_bounds__(TSZ * TSY, SW_KS_MINB)
-ks_velocity(const __grid_constant__ P3<T> p, int it, int src_here) {
+ks_velocity(const __grid_constant__ P3<T> p, int it, int src_here, int x0) {
   const int k = blockIdx.x * TSZ + threadIdx.x;
   const int j = blockIdx.y * TSY + threadIdx.y;
-  const int i = blockIdx.z;
+  const int i = blockIdx.z + (LONG ? x0 : 0);
   const int nx = p.nx, ny = p.ny, nz = p.nz;
   if (j >= ny || k >= nz) return;
   const long long sx = (long long)ny * nz, sy = nz;
@@ -158,9 +160,9 @@ ks_velocity(const __grid_constant__ P3<T> p, int it, int src_here) {
   }
 }
 
-template <typename T, int N>
+template <typename T, int N, bool LONG>
 __global__ void __launch_bounds__(TSZ * TSY, SW_KS_MINB)
-ks_stress(const __grid_constant__ P3<T> p, int it) {
+ks_stress(const __grid_constant__ P3<T> p, int it, int x0) {
   {
     const long long b = blockIdx.x + (long long)gridDim.x * (blockIdx.y + (long long)gridDim.y * blockIdx.z);
     const long long r = b * (TSZ * TSY) + threadIdx.y * TSZ + threadIdx.x;
@@ -168,7 +170,7 @@ ks_stress(const __grid_constant__ P3<T> p, int it) {
   }
   const int k = blockIdx.x * TSZ + threadIdx.x;
   const int j = blockIdx.y * TSY + threadIdx.y;
-  const int i = blockIdx.z;
+  const int i = blockIdx.z + (LONG ? x0 : 0);
   const int nx = p.nx, ny = p.ny, nz = p.nz;
   if (j >= ny || k >= nz) return;
   const long long sx = (long long)ny * nz, sy = nz;
@@ -281,11 +283,21 @@ ks_stress(const __grid_constant__ P3<T> p, int it) {
 template <typename T, int N>
 static cudaError_t launch_spml(const P3<T>& p, int it, bool gather_in_stress, cudaStream_t st) {
   dim3 block(TSZ, TSY);
-  dim3 grid((p.nz + TSZ - 1) / TSZ, (p.ny + TSY - 1) / TSY, p.nx);
-  ks_velocity<T, N><<<grid, block, 0, st>>>(p, it, p.src_kind != SW_SRC_NONE ? 1 : 0);
+  // launches of at most SW_GRID_Z planes, the limit of a grid's z extent
+  auto grid = [&](int x0) {
+    return dim3((p.nz + TSZ - 1) / TSZ, (p.ny + TSY - 1) / TSY, x0 + SW_GRID_Z < p.nx ? SW_GRID_Z : p.nx - x0);
+  };
+  const bool slices = p.nx > SW_GRID_Z;
+  auto velocity = slices ? ks_velocity<T, N, true> : ks_velocity<T, N, false>;
+  auto stress = slices ? ks_stress<T, N, true> : ks_stress<T, N, false>;
+  for (int x0 = 0; x0 < p.nx; x0 += SW_GRID_Z)
+    velocity<<<grid(x0), block, 0, st>>>(p, it, p.src_kind != SW_SRC_NONE ? 1 : 0, x0);
   P3<T> q = p;
   if (!gather_in_stress) q.nrec = 0;
-  ks_stress<T, N><<<grid, block, 0, st>>>(q, it);
+  for (int x0 = 0; x0 < p.nx; x0 += SW_GRID_Z) {
+    stress<<<grid(x0), block, 0, st>>>(q, it, x0);
+    q.nrec = 0;  // recorded by the first launch
+  }
   return cudaGetLastError();
 }
 

@@ -16,6 +16,8 @@
 
 namespace sw {
 
+constexpr int SW_GRID_Z = 65535;  // most blocks along a grid's z
+
 // One-time setup per device (kernel attributes such as the dynamic
 // shared-memory opt-in are per device): runs f() once for each device the
 // calling threads launch on, under a lock; a failed f() is retried next time.
