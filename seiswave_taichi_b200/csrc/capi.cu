@@ -428,8 +428,10 @@ cudaError_t enqueue3(sw_plan* pl, const sw::P3<T>& p, int it, bool first, bool l
         return e;
       }
     }
-    e = sw::sw3_spml_step<T>(q, pl->order, it, pl->gather_in_stress, st);
-    if (e == cudaSuccess && !pl->gather_in_stress) e = sw::sw3_gather<T>(p, it, st);
+    // the per-cell stress kernel records one receiver per thread
+    const bool gather = pl->gather_in_stress && p.nrec <= (long long)std::min(p.nx, sw::SW_GRID_Z) * p.ny * p.nz;
+    e = sw::sw3_spml_step<T>(q, pl->order, it, gather, st);
+    if (e == cudaSuccess && !gather) e = sw::sw3_gather<T>(p, it, st);
     return e;
   }
   const bool tensor = pl->scheme == SW3D_CPML_TENSOR;

@@ -1,9 +1,11 @@
 """Sources and receivers of the per-cell 3D kernels.  A point force near a
 grid's last z block against the staged passes, at every order and shape
-(Elastic3D_SSG_CPML adds 5 to the source's indices, so the case takes them off),
-and a source outside the cells that the passes update against the CPU oracle."""
+(Elastic3D_SSG_CPML adds 5 to the source's indices, so the case takes them off);
+a source outside the cells that the passes update against the CPU oracle; and
+more receivers than the split-PML stress kernel has threads."""
 import numpy as np
 import pytest
+import torch
 
 from cases import case3d, oracle3d, product3d, to_np
 
@@ -50,3 +52,19 @@ def test_source_outside_the_updated_cells(cuda, scheme, N, shape, npml):
         o.run(0, 40)
         for f in F3:
             assert to_np(getattr(w, f)).tobytes() == getattr(o, f).tobytes(), (cell, f)
+
+
+def test_more_receivers_than_threads(cuda):
+    c = case3d(shape=(11, 11, 11), N=1, scheme="SPML", nt=20, npml=3)
+    c["isx"], c["isy"], c["isz"], c["rsx"], c["rsy"], c["rsz"] = 5, 5, 5, 6, 5, 5
+    one, many = product3d(c), product3d(c)
+    n = 20000
+    lin = np.full(n, int(many._rec_lin[0]), np.int64)
+    many._receivers = lambda: (0, lin)
+    many.data = torch.zeros((20, n), dtype=torch.float32, device="cuda")
+    for w in (one, many):
+        w._build_plan().set_path("two_pass")
+        w.run(20)
+    want = to_np(one.data).reshape(20)
+    assert np.abs(want).max() > 0
+    assert (to_np(many.data) == want[:, None]).all()
