@@ -1,0 +1,24 @@
+"""The defaults of 3D plans: the planes per work unit of the staged passes on
+flat grids, where all units are alike and a few large ones beat many small."""
+import numpy as np
+import pytest
+
+from cases import case3d, product3d
+
+pytestmark = pytest.mark.gpu
+
+
+def _plan(shape, N=2, scheme="TENSOR", **kw):
+    w = product3d(case3d(shape=shape, N=N, scheme=scheme, nt=4, hetero=False), **kw)
+    return w, w._build_plan()
+
+
+@pytest.mark.parametrize("N", [1, 2])
+def test_flat_grids_take_large_units(cuda, N):
+    for shape in ((300, 300, 40), (250, 200, 72)):
+        w, p = _plan(shape, N)
+        assert p.info()["path"] == "staged"
+        # 252 and 268 us per step with 2 planes, 220 and 253 with these (order 2)
+        assert p.info()["staged_chunk"] >= 10, shape
+    w, p = _plan((100, 100, 100), N)
+    assert p.info()["staged_chunk"] == 2
