@@ -207,7 +207,7 @@ struct sw_plan {
   // two-pass, 2: fused single pass, 3: 2D persistent (one cooperative launch
   // per run)
   int path = 0;
-  bool path_chosen = false;  // by sw_plan_set_path
+  bool path_chosen = false, chunk_chosen = false;  // by sw_plan_set_path
   unsigned int* d_bar = nullptr;  // 2D persistent path: grid-barrier arrival and generation words
   bool aea = false;               // free-surface hook before every step (sw_plan_set_free_surface)
   // 2D on-chip loop (sw_run of path 0): tiles, the SMs they may take (-1 all),
@@ -640,14 +640,16 @@ int staged_chunk_rule(const sw_plan* pl, int tiles_y, int tiles_z) {
     cudaGetLastError();
     return 8;
   }
-  const double slots = std::min(gv, gs);
   const bool alike = tiles_z <= 2;
   int best = 8;
   double cost = 1e300;
   for (int len = 2; len <= 25; ++len) {
-    const double w = (double)tiles_y * tiles_z * ((p.nx + len - 1) / len) / slots, unit = len + 0.4;
-    const double c = w <= 1 ? (alike ? unit : 1.7 * unit)
-                            : (alike ? 0.5 * (w + std::ceil(w)) * unit : (w + 0.7) * unit);
+    const double units = (double)tiles_y * tiles_z * ((p.nx + len - 1) / len), unit = len + 0.4;
+    double c = 0;
+    for (const int slots : {gv, gs}) {
+      const double w = units / slots;
+      c += w <= 1 ? (alike ? unit : 1.7 * unit) : (alike ? 0.5 * (w + std::ceil(w)) * unit : (w + 0.7) * unit);
+    }
     if (c < cost) {
       cost = c;
       best = len;
@@ -1265,7 +1267,10 @@ int sw_plan_set_path(sw_plan* pl, int32_t path, int32_t chunk_len) {
   pl->path = path;
   pl->path_chosen = true;
   if (pl->staged && path >= 1 && pl->sa.chunks == 0) staged_chunks(pl, 0);  // the fused path ends odd runs staged
-  if (chunk_len > 0 && path == 1) staged_chunks(pl, chunk_len);
+  if (chunk_len > 0 && path == 1) {
+    staged_chunks(pl, chunk_len);
+    pl->chunk_chosen = true;
+  }
   if (chunk_len > 0 && path == 2) {
     sw::FusedConfig fc;
     sw::sw3_fused_config(pl->fused_N, &fc);
@@ -1304,10 +1309,13 @@ int sw_plan_set_free_surface(sw_plan* pl, int32_t on) {
 
 int sw_plan_set_exact(sw_plan* pl, int32_t exact) {
   if (!pl) return fail(SW_ERR_ARG, "null plan");
+  const int was = pl->sa.exact;
   pl->sa.exact = exact ? 1 : 0;
-  if (pl->dim == 3 && !pl->path_chosen) {
-    pl->path = default_path3(pl);
-    if (pl->path == 1 && pl->sa.chunks == 0) staged_chunks(pl, 0);
+  if (pl->dim == 3 && pl->staged) {
+    if (!pl->path_chosen) pl->path = default_path3(pl);
+    // the modes' kernels differ in how many CTAs an SM holds
+    if ((pl->sa.chunks == 0 && pl->path == 1) || (pl->sa.chunks > 0 && was != pl->sa.exact && !pl->chunk_chosen))
+      staged_chunks(pl, 0);
   }
   if (pl->gexec) { cudaGraphExecDestroy(pl->gexec); pl->gexec = nullptr; pl->g_it0 = pl->g_n = -1; }
   return SW_OK;

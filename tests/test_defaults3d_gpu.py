@@ -1,5 +1,6 @@
 """The defaults of 3D plans: the planes per work unit of the staged passes on
-flat grids, where all units are alike and a few large ones beat many small."""
+flat grids, where all units are alike and a few large ones beat many small, and
+chosen again when the numeric mode changes unless the caller has chosen them."""
 import numpy as np
 import pytest
 
@@ -22,3 +23,18 @@ def test_flat_grids_take_large_units(cuda, N):
         assert p.info()["staged_chunk"] >= 10, shape
     w, p = _plan((100, 100, 100), N)
     assert p.info()["staged_chunk"] == 2
+
+
+def test_units_follow_the_numeric_mode(cuda):
+    shape = (300, 300, 40)  # exact: two CTAs per SM, fast: three
+    exact = _plan(shape)[1].info()["staged_chunk"]
+    w, p = _plan(shape, exact=False)
+    fast = p.info()["staged_chunk"]
+    assert fast != exact  # 200 us per step with 7 planes, 211 with the exact kernels' 20
+    p.set_exact(True)
+    assert p.info()["staged_chunk"] == exact
+    p.set_exact(False)
+    assert p.info()["staged_chunk"] == fast
+    p.set_path("staged", 12)
+    p.set_exact(True)
+    assert p.info()["staged_chunk"] == 12
