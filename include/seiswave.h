@@ -200,8 +200,9 @@ SW_API int sw_check_division(float divisor, int32_t mode, uint64_t* mismatches, 
 SW_API int sw_plan_status(sw_plan* plan, void* stream);
 
 /* Describe the plan's execution path: info[0] current path of sw_step/sw_run
- * (0 per-cell two-pass kernels, the default of 3D float64 plans, of split
- * PML and of orders 3 and 4 in exact numerics; 2D: sw_step and sw_run without a graph
+ * (0 per-cell two-pass kernels, the default of 3D float64 plans and, where the
+ * staged tiles fit the grid worse, of split PML and of orders 3 and 4 in exact
+ * numerics; 2D: sw_step and sw_run without a graph
  * make two launches per step, sw_run with one keeps runs of at least 4 steps of
  * orders up to 4 that record a velocity on the chip where their tiles fit --
  * one cooperative launch, neighbouring tiles exchange their rims -- and

@@ -671,16 +671,30 @@ void staged_chunks(sw_plan* pl, int len) {
   a.chunks = (p.nx + len - 1) / len;
 }
 
-// The path of a 3D plan that its caller has not chosen: the staged kernels in
-// the fast numeric mode (only they have it) and for CPML of orders 1 and 2; the
-// per-cell kernels for split PML and orders 3 and 4, whose staged tiles leave
-// too few warps on an SM (us per step at 200^3, staged / per cell: order 2 412
-// / 573, order 3 683 / 615, order 4 736 / 636; split PML order 2 738 / 622,
-// order 4 1229 / 718).
+// The path of a 3D plan that its caller has not chosen: the staged kernels for
+// CPML in the fast numeric mode (only they have it) and at orders 1 and 2; at
+// orders 3 and 4 and for split PML, whose staged tiles leave fewer warps on an
+// SM, the per-cell kernels, except on grids of 2 million cells and more where
+// the staged tiles are the better fit.  Us per step, staged / per cell:
+//   order 3     32-wide tiles 128^3 146 / 150, 160^3 249 / 275, 300 x 300 x 64
+//               379 / 450 (96^3 68 / 66); 40-wide 200^3 670 / 586, flat 300 x 300
+//               x 40 369 / 423 (100 x 100 x 40 59 / 55)
+//   order 4     160^3 343 / 279, 200^3 724 / 600, flat 300 x 300 x 40 399 / 432
+//   split PML   order 1 40-wide 200^3 574 / 591, 250 x 200 x 72 387 / 433, 32-wide
+//               160^3 315 / 271; order 2 200^3 669 / 600, 250 x 200 x 72 500 / 436,
+//               flat 300 x 300 x 40 436 / 542; orders 3, 4 flat 554 / 562, 764 / 630
+// Flat: more of the per-cell kernels' 32-wide z blocks lie idle, by 1.5 times,
+// than of the staged tiles.
 int default_path3(const sw_plan* pl) {
   if (!pl->staged) return 0;
-  if (pl->scheme == SW3D_SPML) return 0;
-  return pl->sa.exact == 0 || pl->order <= 2 ? 1 : 0;
+  const bool spml = pl->scheme == SW3D_SPML;
+  if (!spml && (pl->sa.exact == 0 || pl->order <= 2)) return 1;
+  if (pl->ncell < 2000000) return 0;
+  const int nz = pl->p3f.nz, tz = pl->staged_tz;
+  const bool wide = tz == 40;
+  const bool flat = 2 * ((nz + 31) / 32 * 32) >= 3 * ((nz + tz - 1) / tz * tz);
+  if (spml) return pl->order == 1 ? wide : (pl->order == 2 ? flat : 0);
+  return pl->order == 3 ? !wide || flat : (pl->order == 4 ? flat : 0);
 }
 
 void setup_staged(sw_plan* pl) {
