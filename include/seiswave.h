@@ -208,7 +208,9 @@ SW_API int sw_plan_status(sw_plan* plan, void* stream);
  * one cooperative launch, neighbouring tiles exchange their rims -- and
  * replays the launches otherwise; 3D float CPML of orders 1 and 2: a run of at
  * least 6 steps of a large grid whose rows are no multiple of 16 bytes steps
- * pitched copies of the state with the kernels of path 1 and copies them back;
+ * pitched copies of the state with the kernels of path 1 and copies them back,
+ * where the copies take at most a quarter of the free memory and path 0 has not
+ * been chosen by sw_plan_set_path;
  * 1 TMA-staged
  * two-pass kernels, 2 fused single-pass kernel, 3 2D persistent: sw_run is
  * one cooperative launch for all its steps, the phases separated by a

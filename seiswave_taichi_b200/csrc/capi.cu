@@ -740,11 +740,15 @@ void setup_staged(sw_plan* pl) {
   if (pl->path == 1 || pl->pitch_ok) staged_chunks(pl, 0);  // else when the path is chosen
 }
 
-// The pitched copies of a plan: true when they exist.  They are allocated by
-// the first run that wants them; without memory, or while the stream is being
-// captured, the two-pass kernels run instead.
+// The pitched copies of a plan: true when a run may use them.  They double the
+// plan's memory, so they are taken only where they leave three quarters of the
+// free memory to the caller's program, and not once the caller has chosen the
+// two-pass kernels.  They are allocated by the first run that wants them and
+// kept to the plan's end; otherwise, and while the stream is being captured, the
+// two-pass kernels run.
 bool pitch_ready(sw_plan* pl, int nsteps, cudaStream_t st) {
-  if (pl->dim != 3 || !pl->pitch_ok || pl->path != 0 || pl->aea || nsteps < SW_PITCH_STEPS) return false;
+  if (pl->dim != 3 || !pl->pitch_ok || pl->path != 0 || pl->path_chosen || pl->aea || nsteps < SW_PITCH_STEPS)
+    return false;
   if (pl->pitch_buf) return true;
   CaptureTolerant others;
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
@@ -757,6 +761,11 @@ bool pitch_ready(sw_plan* pl, int nsteps, cudaStream_t st) {
   const size_t cells = (size_t)p.nx * p.ny * pz;
   const size_t m0 = (size_t)p.sn[0] * p.ny * pz, m1 = (size_t)p.nx * p.sn[1] * pz;
   const size_t total = 12 * cells + 6 * (m0 + m1);
+  size_t room = 0, all = 0;
+  if (cudaMemGetInfo(&room, &all) != cudaSuccess || 4 * total * sizeof(float) > room) {
+    cudaGetLastError();
+    return false;
+  }
   float* b = nullptr;
   if (cudaMalloc(&b, total * sizeof(float)) != cudaSuccess) {
     cudaGetLastError();
@@ -1058,10 +1067,9 @@ cudaError_t resident_run(sw_plan* pl, int it0, int nsteps, cudaStream_t st, OnCh
   return e;
 }
 
-cudaError_t enqueue_sequence(sw_plan* pl, int it0, int nsteps, cudaStream_t st) {
+cudaError_t enqueue_sequence(sw_plan* pl, int it0, int nsteps, bool pitched, cudaStream_t st) {
   if (pl->fused && pl->path == 2 && nsteps >= 2 && !pl->aea) return enqueue_fused_run(pl, it0, nsteps, st);
-  if (pl->pitch_buf && pl->path == 0 && !pl->aea && nsteps >= SW_PITCH_STEPS)
-    return enqueue_pitched_run(pl, it0, nsteps, st);
+  if (pitched) return enqueue_pitched_run(pl, it0, nsteps, st);
   for (int s = 0; s < nsteps; ++s) {
     cudaError_t e = enqueue_step(pl, it0 + s, s == 0, s == nsteps - 1, false, 0.0, st);
     if (e != cudaSuccess) return e;
@@ -1386,7 +1394,7 @@ int sw_run(sw_plan* pl, int32_t it0, int32_t nsteps, int32_t use_graph, void* st
   }
   const bool pitched = pitch_ready(pl, nsteps, st);
   if (!use_graph) {
-    e = enqueue_sequence(pl, it0, nsteps, st);
+    e = enqueue_sequence(pl, it0, nsteps, pitched, st);
     if (e != cudaSuccess) return cuda_fail(e, "sw_run");
     return SW_OK;
   }
@@ -1405,7 +1413,7 @@ int sw_run(sw_plan* pl, int32_t it0, int32_t nsteps, int32_t use_graph, void* st
     }
     e = cudaStreamBeginCapture(pl->cap_stream, cudaStreamCaptureModeThreadLocal);
     if (e != cudaSuccess) return cuda_fail(e, "sw_run: begin capture");
-    cudaError_t le = enqueue_sequence(pl, it0, nsteps, pl->cap_stream);
+    cudaError_t le = enqueue_sequence(pl, it0, nsteps, pitched, pl->cap_stream);
     cudaGraph_t g = nullptr;
     e = cudaStreamEndCapture(pl->cap_stream, &g);
     if (le != cudaSuccess) { if (g) cudaGraphDestroy(g); return cuda_fail(le, "sw_run: capture"); }
