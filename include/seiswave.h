@@ -168,9 +168,11 @@ SW_API int sw2d_plan_create(const sw2d_desc* desc, sw_plan** plan);
  * Elastic3D_SSG_SPML.py:8-138 and their SetADEPML3D. */
 SW_API int sw3d_plan_create(const sw3d_desc* desc, sw_plan** plan);
 
-/* Accepted for 3D plans and without effect: the kernels of path 0 give each
- * cell its own thread and stream no x planes (path 1 and 2 take their planes
- * per work unit through sw_plan_set_path). */
+/* The x planes per work unit of a 3D plan's runs on pitched copies (path 0 of a
+ * plan without path 1, see sw_plan_info).  Accepted for the other 3D plans and
+ * without effect: the kernels of path 0 give each cell its own thread and stream
+ * no x planes (path 1 and 2 take their planes per work unit through
+ * sw_plan_set_path). */
 SW_API int sw_plan_set_tile(sw_plan* plan, int32_t x_chunk);
 
 /* No reference counterpart (a self-check of this library's exact division).
@@ -216,7 +218,8 @@ SW_API int sw_plan_status(sw_plan* plan, void* stream);
  * one cooperative launch for all its steps, the phases separated by a
  * bounded grid barrier; opt-in, as path 0 is faster on B200 at every grid
  * size measured; sw_step keeps the two launches), [1] constant-divisor fast path verified, [2] staged
- * path available, [3] its grid, [4] its x-chunk length, [5] fused path set
+ * path available, [3] its grid, [4] its x-chunk length (without path 1: that of
+ * runs on pitched copies, 0 where there are none), [5] fused path set
  * up, [6] its grid (2D: the tiles of the on-chip loop, 0 where sw_run replays
  * the launches), [7] its x-chunk length (2D: the tiles of the last such run, 0
  * if it was replayed), [8] exact numerics (see

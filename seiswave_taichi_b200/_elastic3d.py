@@ -357,31 +357,41 @@ class Elastic3DBase:
     # -- autotuner (no reference counterpart) ------------------------------------
     AUTOTUNE_CHUNKS = (2, 3, 4, 6, 8, 12, 16, 25, 50)
 
+    AUTOTUNE_REV = 2  # of the work order that the cached choices were timed with
+    PITCHED_STEPS = 6  # the shortest run on pitched copies
+
     def autotune(self, steps: int = 6, force: bool = False) -> int:
         """Choose the x planes per work unit of the plan's current path (the
-        staged or fused chunk; the per-cell kernels have none) by timing
+        staged or fused chunk, or that of runs on pitched copies) by timing
         `steps` steps of each candidate on this solver's own grid, with its
         state replaced by random values for the trials and restored
         afterwards (results do not depend on the choice).  The winner is
         cached per (GPU, solver class, order, dtype, numeric mode, path, log2
         shape bucket) in the batch autotuner's JSON file
-        (SEISWAVE_AUTOTUNE_CACHE).  Returns the chosen chunk length."""
+        (SEISWAVE_AUTOTUNE_CACHE).  Returns the chosen chunk length, or 0,
+        without trials, where the path has no work units (the per-cell
+        kernels)."""
         import math
         from .batch import cache_load, cache_store
         plan = self._plan or self._build_plan()
         info = plan.info()
         path_name = info["path"]
+        pitched = path_name == "two_pass" and not info["staged"] and info["staged_chunk"] > 0
+        if pitched:
+            path_name, steps = "pitched", max(int(steps), self.PITCHED_STEPS)
+        if path_name == "two_pass" or (pitched and self.nt <= steps):
+            return 0
         nx, ny, nz = self.gridsize
         dev = torch.cuda.get_device_name(self._dev).replace(" ", "_")
         bucket = "-".join(str(round(math.log2(max(n, 1)))) for n in (nx, ny, nz))
-        key = (f"3d|{dev}|{type(self).__module__}|{self.star}|{self._dt_torch}|{int(info['exact'])}|"
-               f"{path_name}|{bucket}")
+        key = (f"3d.{self.AUTOTUNE_REV}|{dev}|{type(self).__module__}|{self.star}|{self._dt_torch}|"
+               f"{int(info['exact'])}|{path_name}|{bucket}")
 
         def apply(chunk):
-            if path_name in ("staged", "fused"):
-                plan.set_path(path_name, int(chunk))
-            else:
+            if pitched:
                 plan.set_tile(int(chunk))
+            else:
+                plan.set_path(path_name, int(chunk))
 
         v = cache_load().get(key)
         if not force and isinstance(v, int) and v in self.AUTOTUNE_CHUNKS and v <= nx:
@@ -400,7 +410,7 @@ class Elastic3DBase:
         best, best_ms = None, float("inf")
         for chunk in [c for c in self.AUTOTUNE_CHUNKS if c <= nx]:
             apply(chunk)
-            self.run(1, 0, use_graph=False)
+            self.run(steps if pitched else 1, 0, use_graph=False)
             e0 = torch.cuda.Event(enable_timing=True)
             e1 = torch.cuda.Event(enable_timing=True)
             e0.record(st)

@@ -740,6 +740,11 @@ void setup_staged(sw_plan* pl) {
   if (pl->path == 1 || pl->pitch_ok) staged_chunks(pl, 0);  // else when the path is chosen
 }
 
+// whether runs of a plan may step pitched copies
+bool pitched_runs(const sw_plan* pl) {
+  return pl->dim == 3 && pl->pitch_ok && pl->path == 0 && !pl->path_chosen && !pl->aea;
+}
+
 // The pitched copies of a plan: true when a run may use them.  They double the
 // plan's memory, so they are taken only where they leave three quarters of the
 // free memory to the caller's program, and not once the caller has chosen the
@@ -747,8 +752,7 @@ void setup_staged(sw_plan* pl) {
 // kept to the plan's end; otherwise, and while the stream is being captured, the
 // two-pass kernels run.
 bool pitch_ready(sw_plan* pl, int nsteps, cudaStream_t st) {
-  if (pl->dim != 3 || !pl->pitch_ok || pl->path != 0 || pl->path_chosen || pl->aea || nsteps < SW_PITCH_STEPS)
-    return false;
+  if (!pitched_runs(pl) || nsteps < SW_PITCH_STEPS) return false;
   if (pl->pitch_buf) return true;
   CaptureTolerant others;
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
@@ -1205,7 +1209,12 @@ int sw_plan_set_tile(sw_plan* pl, int32_t x_chunk) {
   if (!pl) return fail(SW_ERR_ARG, "null plan");
   if (pl->dim != 3) return fail(SW_ERR_UNSUPPORTED, "tile choice applies to 3D plans");
   if (x_chunk < 1) return fail(SW_ERR_ARG, "x_chunk must be >= 1");
-  return SW_OK;  // the per-cell kernels stream no planes
+  // the per-cell kernels stream no planes; pitched runs have the staged kernels' units
+  if (pitched_runs(pl)) {
+    staged_chunks(pl, x_chunk);
+    if (pl->gexec) { cudaGraphExecDestroy(pl->gexec); pl->gexec = nullptr; pl->g_it0 = pl->g_n = -1; }
+  }
+  return SW_OK;
 }
 
 int sw_check_division(float divisor, int32_t mode, uint64_t* mismatches, void* stream) {
@@ -1264,7 +1273,7 @@ int sw_plan_info(sw_plan* pl, int32_t* info) {
       info[3] = gv;
     cudaGetLastError();
   }
-  info[4] = pl->staged ? pl->sa.chunk_len : 0;
+  info[4] = pl->staged || pitched_runs(pl) ? pl->sa.chunk_len : 0;
   info[5] = pl->fused ? 1 : 0;
   info[6] = pl->dim == 2 ? pl->res.tx * pl->res.tz : (pl->fused ? pl->fused_grid : 0);
   info[7] = pl->dim == 2 ? pl->res_last : (pl->fused ? pl->fx.chunk_len : 0);
