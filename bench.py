@@ -327,6 +327,23 @@ def run_reference(args, rank, world):
     return 0
 
 
+def run_kernels(cfg, info, nt: int):
+    """This library's kernels of one run of nt steps by a plan with this info,
+    and how many launches that is: velocity + stress kernel per time step, plus
+    a moment-tensor source's injection before the first step (receivers and
+    next-step sources ride inside the stress kernel); 2D: one launch for a run
+    that stayed on the chip."""
+    if len(cfg["shape"]) == 2:
+        if info["last_run_tiles"]:
+            return "k2r_run", 1
+        return "k2_velocity + k2_stress", 2 * nt
+    if cfg.get("scheme") == "SPML":
+        name = {"staged": "k3s_velocity + k3s_stress", "two_pass": "ks_velocity + ks_stress"}[info["path"]]
+        return name, 2 * nt
+    name = {"staged": "k3s_velocity + k3s_stress", "two_pass": "k3_velocity + k3_stress", "fused": "k3_fused"}
+    return name[info["path"]], (nt if info["path"] == "fused" else 2 * nt) + 1
+
+
 def max_over_ranks(ms: float, dist, device="cuda") -> float:
     """The slowest rank's device time: every rank takes part, in the same
     order, and gets the maximum (a no-op on one process)."""
@@ -450,7 +467,8 @@ def run_batch(args, rank, world, local):
             "shots_per_s": world * len(waves) * args.steps / (ms * 1e-3),
             "sequential": {"value": whole_job_value(world, cells, nt, 1, seq_ms), "unit": "Gcell-updates/s",
                            "shots_per_s": world * len(waves) / (seq_ms * 1e-3),
-                           "what": "the same shots one after the other, each from its own cached CUDA graph"},
+                           "what": "the same shots one after the other, each run one on-chip launch or its own "
+                                   "cached CUDA graph"},
             "fwi_step": {"ms": fwi_ms, "checkpoint_every": 100,
                          "what": "batched forward with checkpoints + 64 per-shot adjoints + gradient chain, "
                                  "observed traces from pinned host memory, gradients back to the host"},
@@ -792,14 +810,9 @@ def main(argv=None):
     if rank == 0 and world == 1 and not args.no_cpu_baseline:
         cpu = cpu_baseline(cfg)
 
-    # per run: velocity + stress kernel per time step, plus the first step's
-    # moment-tensor injection (receivers and next-step sources ride inside the
-    # stress kernel); w.reset() zeroes the state with torch fills
-    # (2D: the whole run is one on-chip launch)
-    launches_per_run = 2 * nt + 1 if three_d else 1
-    info = w._plan.info() if three_d else {"path": "two_pass", "run": "on-chip loop"}
-    kname = {"staged": "k3s_velocity + k3s_stress", "two_pass": "k3_velocity + k3_stress",
-             "fused": "k3_fused"}.get(info["path"], info["path"]) if three_d else "k2r_run"
+    # w.reset() zeroes the state with torch fills, which are not counted
+    info = (w._plan if three_d else next(iter(w._plans.values()))).info()
+    kname, launches_per_run = run_kernels(cfg, info, nt)
     if rank == 0:
         line = {
             "metric": "Gcell-updates/s", "value": value, "unit": "Gcell-updates/s", "n_gpus": world,
