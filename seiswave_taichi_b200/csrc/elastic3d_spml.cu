@@ -12,11 +12,14 @@
 
 namespace sw {
 
-// Resident blocks per SM the float kernels are compiled for: one thread per
-// cell waits on its loads (us per step with 4, 5, 6, 8 blocks: 200^3 order 2
+// Resident blocks per SM the kernels are compiled for: one thread per cell
+// waits on its loads (us per step with 4, 5, 6, 8 blocks: float 200^3 order 2
 // 874, 780, 729, 622, order 4 897, 830, 812, 718; 100^3 order 4 107, 106, 107,
-// 102)
-#define SW_KS_MINB (sizeof(T) == 4 ? 8 : 1)
+// 102).  Double with the compiler's own count, 2, 3, 4, 5: 160 x 150 x 101 order
+// 2 569, 569, 466, 392, 355, order 8 935, 524, 423, 377, 360 (its own 139
+// registers left one block on an SM); 60 x 60 x 61 order 3 43, 43, 38, 38, 38,
+// order 8 62, 39, 40, 33, 37.
+#define SW_KS_MINB (sizeof(T) == 4 ? 8 : 5)
 constexpr int TSZ = 32;
 constexpr int TSY = 8;
 
