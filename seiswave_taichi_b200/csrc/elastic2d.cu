@@ -27,6 +27,13 @@ namespace sw {
 // (full occupancy made them slower: 12.6 against 13.3 Gcell/s at 400^2), and
 // so do the double ones.
 #define SW_BATCH_MINB (sizeof(T) == 4 ? 2048 / (BX * BZ) : 1)
+// Resident blocks per SM where the compiler's own register count lies just above
+// a step of the residency (float VS: velocity 50 registers at order 1 and 77 at
+// order 6, stress 86 at order 8): us per step at 2000 x 900 52.8 -> 51.1, 83.5 ->
+// 80.3, 104.9 -> 99.6.  0: its own count.  Order 2 (50 -> 48, one block more) gains
+// 1.3% there and loses 3% in single steps of 400^2, and keeps its count.
+#define SW_VEL2_MINB (sizeof(T) == 4 && SCHEME == SW2D_SSG_VS ? (N == 1 ? 10 : N == 6 ? 7 : 0) : 0)
+#define SW_STR2_MINB (sizeof(T) == 4 && SCHEME == SW2D_SSG_VS && N == 8 ? 6 : 0)
 constexpr int T2Z = 32;
 constexpr int T2X = 4;
 
@@ -334,7 +341,7 @@ __device__ __forceinline__ void str2_cell(const P2<T>& p, int i, int j, int it, 
 }
 
 template <typename T, int N, int SCHEME>
-__global__ void __launch_bounds__(T2Z * T2X)
+__global__ void __launch_bounds__(T2Z * T2X, SW_VEL2_MINB)
 k2_velocity(const __grid_constant__ P2<T> p, int it, T amp, int src_here) {
   const int j = blockIdx.x * T2Z + threadIdx.x;
   const int i = blockIdx.y * T2X + threadIdx.y;
@@ -343,7 +350,7 @@ k2_velocity(const __grid_constant__ P2<T> p, int it, T amp, int src_here) {
 }
 
 template <typename T, int N, int SCHEME>
-__global__ void __launch_bounds__(T2Z * T2X)
+__global__ void __launch_bounds__(T2Z * T2X, SW_STR2_MINB)
 k2_stress(const __grid_constant__ P2<T> p, int it, int inject_next) {
   // receivers of the velocity fields (final for this step, not written here)
   {
