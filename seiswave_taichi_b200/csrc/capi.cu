@@ -2,9 +2,9 @@
 //
 // A plan validates a descriptor once (shapes, orders, slab extents, source and
 // receiver cells) and freezes the kernel parameter blocks; sw_step / sw_run
-// then only enqueue kernels.  sw_run replays a cached CUDA graph of the whole
-// step sequence so the per-step launch cost of the reference's Python loop
-// (test2d_homegenous.py:55-56) disappears.
+// then only enqueue kernels.  sw_run keeps a 2D loop on the chip in one launch or
+// replays a cached CUDA graph of the whole step sequence, so the per-step launch
+// cost of the reference's Python loop (test2d_homegenous.py:55-56) disappears.
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
@@ -628,7 +628,12 @@ int units_grid(int units, int per_sm) {
 // and CTAs work in rounds, which the x ends and L2 blur by half.  The cheapest
 // of 2 .. 25 planes by this rule is within 0.7% of the best measured on average
 // over 52 grids, orders and modes, 3.8% at worst (0.25 N planes of fill and 1.7
-// units for every grid, as before: 4% and 16%).  Us per step, planes per unit:
+// units of the busier pass for every grid: 4% and 16%).  At orders 2 and 4 with
+// three or more tiles along z that older form is kept: on 22 such grids and modes
+// it is level at order 2 and 1.3% faster at order 4 (240 x 180 x 160 order 4 fast
+// 492 with its 8 planes, 502 with 6), at orders 1 and 3 it is 1.6% slower on
+// average (200^3 order 1 418 with its 2 planes, 396 with 5).  Us per step, planes
+// per unit:
 // 300 x 300 x 40 order 2 252 with 2, 235 with 4, 254 with 6, 218 with 10, 254 with
 // 12, 224 with 20 (285 units); 200^3 order 2 436, 411, 421, 443 with 2, 4, 8, 12;
 // 100^3 114, 134, 176 with 2, 4, 6.
@@ -640,7 +645,7 @@ int staged_chunk_rule(const sw_plan* pl, int tiles_y, int tiles_z) {
     cudaGetLastError();
     return 8;
   }
-  const bool alike = tiles_z <= 2;
+  const bool alike = tiles_z <= 2, tail = !alike && pl->staged_N % 2 == 0;
   int best = 8;
   double cost = 1e300;
   for (int len = 2; len <= 25; ++len) {
@@ -649,6 +654,10 @@ int staged_chunk_rule(const sw_plan* pl, int tiles_y, int tiles_z) {
     for (const int slots : {gv, gs}) {
       const double w = units / slots;
       c += w <= 1 ? (alike ? unit : 1.7 * unit) : (alike ? 0.5 * (w + std::ceil(w)) * unit : (w + 0.7) * unit);
+    }
+    if (tail) {
+      const double w = units / std::min(gv, gs);
+      c = ((w <= 1 ? 0 : w) + 1.7) * (len + 0.25 * pl->staged_N);
     }
     if (c < cost) {
       cost = c;
