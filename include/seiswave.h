@@ -10,8 +10,9 @@
  *
  * Ownership: every array is allocated by the caller (PyTorch in the Python
  * package) and borrowed by the plan; nothing here frees caller memory.  A plan
- * owns only its small internal scratch (step counters, CUDA graphs), released
- * by sw_plan_destroy.  Device arrays are C-contiguous, last index fastest:
+ * owns only its internal scratch (step counters, rim buffers, CUDA graphs; the
+ * fused path's second buffer set and the pitched copies of sw_plan_info's path 0
+ * are as large as the caller's state), released by sw_plan_destroy.  Device arrays are C-contiguous, last index fastest:
  * (nx, nz) in 2D, (nx, ny, nz) in 3D.
  *
  * Errors: every call returns SW_OK (0) or a negative SW_ERR_* code; the
@@ -291,7 +292,8 @@ SW_API int sw_step_amp(sw_plan* plan, int32_t it, double amplitude, void* stream
 
 /* Steps it0 .. it0+nsteps-1 back to back, the reference driver loop
  * `for i in range(nt): obj.update_*(i)` (e.g. test2d_homegenous.py:55-56),
- * replayed from a cached CUDA graph when use_graph != 0. */
+ * when use_graph != 0 as one launch that stays on the chip (2D, sw_plan_info) or
+ * replayed from a cached CUDA graph. */
 SW_API int sw_run(sw_plan* plan, int32_t it0, int32_t nsteps, int32_t use_graph, void* stream);
 
 /* ---- batches of 2D shots (no reference counterpart) -------------------------

@@ -341,9 +341,14 @@ class Elastic3DBase:
         return self
 
     def run(self, nt=None, it0: int = 0, use_graph: bool = True, free_surface=None):
-        """Steps it0 .. it0+nt-1 in one enqueue (CUDA graph), the drivers'
-        `for i in range(nt): test.update_SSG(i)` loop; free_surface=True/False
-        sets the free-surface mode first (set_free_surface)."""
+        """Steps it0 .. it0+nt-1, the drivers' `for i in range(nt):
+        test.update_SSG(i)` loop, in one enqueue: a cached CUDA graph of two
+        launches per step, without use_graph the launches themselves.  Large
+        float32 grids of orders 1 and 2 whose rows are no multiple of 16 bytes
+        step pitched copies of the state that the plan keeps, memory permitting
+        (the plan's set_path("two_pass") leaves them out).
+        free_surface=True/False sets the free-surface mode first
+        (set_free_surface)."""
         if free_surface is not None:
             self.set_free_surface(free_surface)
         nt = self.nt - it0 if nt is None else int(nt)

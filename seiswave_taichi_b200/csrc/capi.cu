@@ -157,8 +157,9 @@ __global__ void k_count_nonfinite(const T* a, long long n, unsigned long long* o
 
 }  // namespace
 
-// fewest steps of a run that pay for the pitched copies' way in and out
-// (about as much traffic as 1.2 steps)
+// fewest steps of a run that pay for the pitched copies' way in and out (about
+// as much traffic as 1.2 steps) once they exist: 6 steps, per cell / pitched, 200 x
+// 190 x 201 1.05, 300 x 300 x 41 1.07, 180 x 180 x 181 0.99
 #define SW_PITCH_STEPS 6
 
 // tiles of the 2D on-chip loop (tx = 0: none fit)
@@ -744,8 +745,14 @@ void setup_staged(sw_plan* pl) {
   for (int q = 0; q < 9; ++q) direct = direct && aligned(p.f[q], 16);
   direct = direct && aligned(p.rho, 16) && aligned(p.lam, 16) && aligned(p.mu, 16);
   // Rows that are no multiple of 16 bytes: a run steps pitched copies where the
-  // staged kernels are the faster path by more than the way in and out (us per
-  // step, per cell -> pitched: 200 x 190 x 201 order 2 560 -> 422)
+  // staged kernels are the faster path by more than the way in and out.  Time of
+  // a run of 100 steps, per cell / pitched (orders 1 and 2 differ by 3%): 116 x 116
+  // x 113 0.91, 130 x 130 x 131 1.04, 150 x 150 x 151 1.10, 165^3 1.15, 180 x 180 x
+  // 181 1.18, 200 x 190 x 201 1.28, 400 x 400 x 201 1.45; 300 x 300 x 37 1.5, x 41
+  // 1.2, x 33 0.9 (the per-cell blocks beyond z = 32 have no cell to update); 600 x
+  // 600 x 33 1.10.  12 steps, again and with the copies' allocation: 150 x 150 x 151
+  // 1.03, 0.83; 200 x 190 x 201 1.17, 1.04.  Below 3 million cells the two are
+  // level within 10%: the bound is kept from slower per-cell kernels.
   pl->pitch_ok = p.nz % 4 != 0 && pl->gather_in_stress && pl->scheme != SW3D_SPML && pl->order <= 2 &&
                  (long long)p.nx * p.ny * p.nz >= 1500000LL;
   if (!direct && !pl->pitch_ok) return;

@@ -23,12 +23,12 @@
 // are enough.  Tags count phases from 1; the inbox is zeroed before every
 // launch, on its stream.
 //
-// Measured on B200 (us per step from rest, two launches per step from a graph
-// -> on the chip): 60 x 64 9.9 -> 4.7, 200^2 10.2 -> 4.5, 400^2 11.7 -> 6.2,
-// 700 x 400 15.0 -> 9.6, 1000 x 420 18.8 -> 12.6; float64 100^2 10.9 -> 4.2.
+// Measured on B200 (us per step of 300, order 2, two launches per step from a
+// graph -> on the chip): 60 x 64 8.6 -> 3.9, 200^2 9.2 -> 4.1, 400^2 10.9 -> 5.3,
+// 700 x 400 14.8 -> 7.9, 1000 x 420 18.9 -> 9.9; float64 121 x 90 11.5 -> 4.1.
 // What is left: two exchanges of about 1.2 us, instruction issue (about 190
 // warp instructions per 32 cells and phase, more in the slabs and where
-// numerators are below 2^-100).  640 threads: 94 registers and no spills, 20
+// numerators are below 2^-100).  640 threads: 96 registers and no spills, 20
 // warps; 512, 768 and 1024 threads measured 7-16% slower at 400^2.
 //
 // Every cell runs the expressions of vel2_cell / str2_cell (elastic2d.cu) in

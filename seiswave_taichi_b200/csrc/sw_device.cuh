@@ -472,8 +472,9 @@ __device__ __forceinline__ void cell_quotients(double (&x)[K], const double (&d)
 }
 
 // quotients of a component's derivatives by the spacings of axes A, B, C as one
-// range-tested group (div_c's bits): at 128 x 120 x 112 in double
-// 444 -> 410 us per step
+// range-tested group (div_c's bits), against one by one: us per step of the
+// per-cell CPML kernels at 128 x 120 x 112 in double 313 -> 232, at 200^3 in float
+// order 3 652 -> 617, order 4 678 -> 640
 template <typename T, int A, int B, int C>
 __device__ __forceinline__ void spacings(const P3<T>& p, T& a, T& b, T& c) {
   const T h[3] = {p.dx, p.dy, p.dz};

@@ -1,6 +1,6 @@
 // sw_tma.cuh -- TMA (cp.async.bulk.tensor) and mbarrier helpers, inline PTX
-// for sm_100a.  Every wait is bounded: after SW_WAIT_LIMIT polls the caller
-// gets `false` back, records an error word and leaves without hanging.
+// for sm_100a.  Every wait is bounded: after SW_WAIT_NS the caller gets
+// `false` back, records an error word and leaves without hanging.
 #pragma once
 
 #include <cstdint>
